@@ -159,7 +159,8 @@ int prec_gpu_mul_device(const uint64_t *d_a, size_t an, const uint64_t *d_b, siz
 /* Diagnostic form of prec_gpu_mul_device: records a CUDA event on `stream`
  * before the first and after every kernel of the product, synchronises,
  * and writes each kernel's device time (ms) to stage_ms[0 .. *nstages)
- * (at most 8).  Kernel names: prec_gpu_stage_name(path, i) with the path of
+ * (at most 8).  It always takes the NTT band's kernels, also where
+ * prec_gpu_mul_device forms a short product directly.  Kernel names: prec_gpu_stage_name(path, i) with the path of
  * prec_gpu_stats_t.  Replaces: the wall-clock phase timers of the
  * reference's benches (test/bench_ntt.cpp:25-58, pi/pi_chudnovsky.cpp:183-188). */
 int prec_gpu_mul_device_profile(const uint64_t *d_a, size_t an, const uint64_t *d_b, size_t bn,

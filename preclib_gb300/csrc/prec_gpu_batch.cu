@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "../../include/prec_gpu.h"
+#include "mul_direct.cuh"
 #include "prec_gpu_internal.h"
 
 using namespace precgpu;
@@ -39,13 +40,14 @@ struct Chunk {
 
 struct Cls {
     int k = 0;
+    int direct = -1;              // class of the direct form (mul_direct.cuh), or -1
     int square = 0;               // every product of the class is a square
     Plan pl;                      // class-wide plan (k, set, k1, k2, rows, crt)
     std::vector<int> items;       // indices into the batch's products
     size_t ws_per = 0;            // workspace bytes per product (four-step)
     int per_chunk = 0;            // products per chunk
     std::vector<Chunk> chunks;
-    SmallDesc* d_small = nullptr; // device descriptors (single-CTA classes)
+    SmallDesc* d_small = nullptr; // device descriptors (direct and single-CTA classes)
     ProdPtrs* d_ptrs = nullptr;   // device descriptors (four-step classes)
     uint8_t* ws = nullptr;        // workspace of one chunk
     bool persistent = false;      // one persistent kernel per chunk (ntt_class.cu)
@@ -125,7 +127,9 @@ static void batch_enqueue(prec_gpu_batch* b, cudaStream_t origin, bool branch) {
     for (Cls& c : b->classes) {
         cudaStream_t st = branch ? c.stream : origin;
         if (branch && !rec) cudaStreamWaitEvent(st, b->fork, 0);
-        if (c.pl.path == 0) {
+        if (c.direct >= 0) {
+            launch_direct_batch(c.d_small, (int)c.items.size(), c.direct, st);
+        } else if (c.pl.path == 0) {
             ntt_launch_small(c.d_small, nullptr, (int)c.items.size(), c.k, ctx_field(0), c.pl.crt, st);
         } else {
             ProdArgs args{};
@@ -175,9 +179,11 @@ static int batch_build(const prec_gpu_product_t* items, size_t count, bool onesh
     b->oneshot = ost;
     b->items.assign(items, items + count);
     b->err = ctx_device_err();
-    // classes by key (64-bit digits << 8 | k << 1 | square): a dense table,
-    // not a map lookup per product (a binary-splitting level has ~10^6 of them)
-    std::vector<int> cls_of(1 << 9, -1);
+    // classes by key (64-bit digits << 8 | k << 1 | square, or the direct
+    // form's class past those): a dense table, not a map lookup per product
+    // (a binary-splitting level has ~10^6 of them)
+    constexpr int kDirectKey = 1 << 9;
+    std::vector<int> cls_of(kDirectKey + kDirectClasses, -1);
     std::vector<Cls> found;
     const bool wide = wide_digits();
     for (size_t i = 0; i < count; ++i) {
@@ -188,6 +194,17 @@ static int batch_build(const prec_gpu_product_t* items, size_t count, bool onesh
         }
         if (p.an == 0 || p.bn == 0) {
             b->zero_items.push_back((int)i);
+            continue;
+        }
+        const int direct = direct_class(p.an, p.bn);
+        if (direct >= 0) {
+            int& ci = cls_of[kDirectKey + direct];
+            if (ci < 0) {
+                ci = (int)found.size();
+                found.emplace_back();
+                found[ci].direct = direct;
+            }
+            found[ci].items.push_back((int)i);
             continue;
         }
         // the transform length and digit width pick the class; the class

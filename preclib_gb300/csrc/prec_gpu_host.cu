@@ -25,6 +25,7 @@
 
 #include "../../include/prec_gpu.h"
 #include "fft_kernels.cuh"
+#include "mul_direct.cuh"
 #include "ntt_kernels.cuh"
 #include "prec_gpu_internal.h"
 
@@ -298,11 +299,14 @@ struct Lane {
     double* h_maxdist = nullptr;
     FftArgs* fft_args = nullptr;  // the FP64 band product's arguments, read by its kernels
     cudaEvent_t last_done = nullptr, ev0 = nullptr, ev1 = nullptr;
+    unsigned long long last_stream = 0;  // id of the stream last_done was recorded on (ids are never reused)
+    bool has_last = false;
     cudaEvent_t ev_a = nullptr, ev_b = nullptr;  // each operand on the device
     cudaEvent_t stage_ev[kMaxStages + 1] = {};
     cudaEvent_t chunk_done[kCrtMaxChunks] = {};
     cudaEvent_t copy_done = nullptr;
     uint32_t* chunk_words = nullptr;  // 2 * kCrtMaxChunks words
+    uint32_t* direct_counter = nullptr;  // finished CTAs of a direct product (zero between products)
     PrimeStreams prime_streams = {};
     std::map<GraphKey, GraphEntry> graphs;  // single-product graphs by plan shape
 };
@@ -518,6 +522,7 @@ static int init_locked(Ctx& c, int device) {
     CK(cudaMallocHost(&c.h_err, kStatBytes));
     CK((cudaError_t)ntt_configure_kernels());
     CK((cudaError_t)fft_configure_kernels());
+    CK((cudaError_t)configure_direct());
     CK(cudaMalloc(&c.fft_tw, fft_table_bytes()));
     fft_build_table(c.fft_tw, nullptr);
     CK(cudaGetLastError());
@@ -547,6 +552,7 @@ static void lane_destroy(Lane& L) {
     cudaFreeHost(L.h_err);
     cudaFree(L.fft_args);
     cudaFree(L.chunk_words);
+    cudaFree(L.direct_counter);
     for (cudaEvent_t e : {L.last_done, L.ev0, L.ev1, L.ev_a, L.ev_b, L.copy_done})
         if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : L.stage_ev)
@@ -570,6 +576,8 @@ static int lane_create(Lane& L) {
     for (int i = 0; i < kCrtMaxChunks; ++i) CK(cudaEventCreateWithFlags(&L.chunk_done[i], cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&L.copy_done, cudaEventDisableTiming));
     CK(cudaMalloc(&L.chunk_words, 2 * kCrtMaxChunks * sizeof(uint32_t)));
+    CK(cudaMalloc(&L.direct_counter, sizeof(uint32_t)));
+    CK(cudaMemset(L.direct_counter, 0, sizeof(uint32_t)));
     CK(cudaEventCreateWithFlags(&L.last_done, cudaEventDisableTiming));
     CK(cudaEventCreate(&L.ev0));
     CK(cudaEventCreate(&L.ev1));
@@ -675,6 +683,27 @@ static int grow(void** buf, size_t* cap, size_t bytes, bool slack) {
         want = bytes;
     }
     *cap = want;
+    return 0;
+}
+
+// Work on `st` starts after the lane's previous product.  On the previous
+// product's own stream the stream's order says so already: no event wait.
+// Streams are told apart by their id, which, unlike the handle, no later
+// stream gets again; a stream being captured always gets the wait.
+static int lane_begin(Lane& L, cudaStream_t st) {
+    unsigned long long id = 0;
+    CK(cudaStreamGetId(st, &id));
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cap));
+    if (!L.has_last || id != L.last_stream || cap != cudaStreamCaptureStatusNone)
+        CK(cudaStreamWaitEvent(st, L.last_done, 0));
+    return 0;
+}
+
+static int lane_end(Lane& L, cudaStream_t st) {
+    CK(cudaStreamGetId(st, &L.last_stream));
+    CK(cudaEventRecord(L.last_done, st));
+    L.has_last = true;
     return 0;
 }
 
@@ -1008,7 +1037,7 @@ static int host_mul(const uint64_t* a, size_t an, const uint64_t* b, size_t bn, 
     uint64_t* d_out = L.io + la_pad + lb_pad;
     cudaStream_t st = L.stream;
     NvtxRange range("prec_gpu_mul %zux%zu %s", la, lb, use_fft ? "fft" : (blocked ? "blocked" : "ntt"));
-    CK(cudaStreamWaitEvent(st, L.last_done, 0));
+    if ((r = lane_begin(L, st))) return r;
     // the per-prime chains start on a's forward columns while b is copied
     CK(cudaMemcpyAsync(d_a, a, la * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
     CK(cudaEventRecord(L.ev_a, st));
@@ -1078,7 +1107,7 @@ static int host_mul(const uint64_t* a, size_t an, const uint64_t* b, size_t bn, 
     const bool fft_failed = use_fft && (*L.h_err & kDevErrFftRound);
     if (copied) CK(cudaStreamWaitEvent(st, L.copy_done, 0));
     else if (!fft_failed) CK(cudaMemcpyAsync(out, d_out, lout * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-    CK(cudaEventRecord(L.last_done, st));
+    if ((r = lane_end(L, st))) return r;
     {
         NvtxRange wait("wait for product and result copy");
         CK(cudaStreamSynchronize(st));
@@ -1167,16 +1196,24 @@ int prec_gpu_mul_device(const uint64_t* d_a, size_t an, const uint64_t* d_b, siz
     const uint64_t B = block_limbs();
     if (an > B || bn > B) {
         if ((r = prepare_blocked(L, an, bn, B, pl))) return r;
-        CK(cudaStreamWaitEvent(st, L.last_done, 0));
+        if ((r = lane_begin(L, st))) return r;
         if ((r = enqueue_blocked(c, L, d_a, an, d_b, bn, d_out, st, B, c.d_err))) return r;
-        CK(cudaEventRecord(L.last_done, st));
+        if ((r = lane_end(L, st))) return r;
+        return 0;
+    }
+    if (direct_single(an, bn)) {
+        if ((r = ensure_ws(L, direct_scratch_bytes(an, bn)))) return r;
+        if ((r = lane_begin(L, st))) return r;
+        launch_direct_single(d_a, an, d_b, bn, d_out, L.ws, L.direct_counter, st);
+        CK(cudaGetLastError());
+        if ((r = lane_end(L, st))) return r;
         return 0;
     }
     if ((r = plan_for(2 * (uint64_t)an, 2 * (uint64_t)bn, an + bn, pl, wide_digits()))) return r;
     if ((r = ensure_ws(L, pl.work_bytes))) return r;
-    CK(cudaStreamWaitEvent(st, L.last_done, 0));
+    if ((r = lane_begin(L, st))) return r;
     if ((r = enqueue_ntt(c, L, d_a, an, d_b, bn, d_out, pl, st, c.d_err))) return r;
-    CK(cudaEventRecord(L.last_done, st));
+    if ((r = lane_end(L, st))) return r;
     return 0;
 }
 
@@ -1193,9 +1230,9 @@ int prec_gpu_mul_device_profile(const uint64_t* d_a, size_t an, const uint64_t* 
     Plan pl;
     if ((r = plan_for(2 * (uint64_t)an, 2 * (uint64_t)bn, an + bn, pl, wide_digits()))) return r;
     if ((r = ensure_ws(L, pl.work_bytes))) return r;
-    CK(cudaStreamWaitEvent(st, L.last_done, 0));
+    if ((r = lane_begin(L, st))) return r;
     if ((r = enqueue_ntt(c, L, d_a, an, d_b, bn, d_out, pl, st, c.d_err, L.stage_ev))) return r;
-    CK(cudaEventRecord(L.last_done, st));
+    if ((r = lane_end(L, st))) return r;
     CK(cudaStreamSynchronize(st));
     const int n = kStageCount[pl.path];
     for (int i = 0; i < n; ++i) CK(cudaEventElapsedTime(&stage_ms[i], L.stage_ev[i], L.stage_ev[i + 1]));
