@@ -19,7 +19,7 @@
 // limbs 5.2 T/s (there the flushes and the carry stage show).  44643 products of
 // 58 .. 66 limbs: kernels 0.98 -> 0.14 ms against the single-CTA transform.
 // A single product is bound by latency instead: launch, two trips to L2 and
-// the carries of the last CTA; 1024 x 1000 limbs 28.7 -> 10.2 us.
+// the carries of the last CTA; 1024 x 1000 limbs 28.7 -> 8.1 us.
 #include "mul_direct.cuh"
 
 #include "ntt_engine.cuh"
@@ -107,6 +107,8 @@ __global__ void __launch_bounds__(DirectGeom<R, G>::THREADS) k_direct(const Smal
     constexpr int S = Blk<R>::S;
     extern __shared__ __align__(16) uint32_t dsm[];
     __shared__ BlockCarryShared sh;
+    pdl_enter();
+    pdl_next();
     const int sub = threadIdx.x / G;
     const int item = blockIdx.x * D::PER_CTA + sub;
     const bool live = item < count;  // a group past the end runs an empty product
@@ -223,7 +225,7 @@ void launch_direct_batch(const SmallDesc* d_descs, int count, int cls, cudaStrea
 #define X(C, R, G)                                                                                              \
     if (cls == C) {                                                                                             \
         using D = DirectGeom<R, G>;                                                                             \
-        launch_kernel(k_direct<R, G>, (count + D::PER_CTA - 1) / D::PER_CTA, D::THREADS, D::SMEM, st, d_descs, count); \
+        launch_pdl(false, k_direct<R, G>, (count + D::PER_CTA - 1) / D::PER_CTA, D::THREADS, D::SMEM, st, d_descs, count); \
         count_launches(1);                                                                                      \
     }
     PREC_DIRECT(X)
@@ -262,6 +264,10 @@ __global__ void __launch_bounds__(kGridThreads) k_direct_grid(DirectArgs f) {
     // partial sums: slot s < SL of a column block holds slice s's sums, slot
     // SL the low part of the slice that crosses from block c to block c + na
     uint32_t* part = sb + (f.nb + 1) * S;
+    pdl_enter();
+    pdl_next();
+    f.a = after_entry(f.a);
+    f.b = after_entry(f.b);
     constexpr int PS = 3 * R + 1;  // words per slot (odd: no bank conflicts across slots)
 #pragma unroll 4
     for (int i = threadIdx.x; i < f.na * (R / 2); i += kGridThreads) Blk<R>::put(sa + S, i, i < f.la ? __ldg(&f.a[i]) : 0ull);
@@ -395,9 +401,9 @@ static size_t grid_smem(int cb, int na, int nb) {
            sizeof(uint32_t);
 }
 
-// Direct up to 2^22 limb pairs: measured 8.2 us at 64 x 64 limbs (transform
-// 12.3), 10.3 at 1024 x 1000 (26.7), 16.4 at 2048 x 2048 (22.5), 24.6 at
-// 3072 x 3072 (22.6).  4096 limbs are what one CTA's shared memory takes.
+// Direct up to 2^22 limb pairs: measured 5.9 us at 64 x 64 limbs (transform
+// 12.6), 8.1 at 1024 x 1000 (28.7), 14.9 at 2048 x 2048 and 16.4 at
+// 4096 x 1000 (19.2).  4096 limbs are what one CTA's shared memory takes.
 bool direct_single(uint64_t la, uint64_t lb) {
     const uint64_t hi = la > lb ? la : lb;
     return hi <= kDirectGridMax && la * lb <= 1ull << 22;
@@ -426,7 +432,7 @@ void launch_direct_single(const uint64_t* a, uint64_t la, const uint64_t* b, uin
     while (cb < 8 && (f.na + cb - 1) / cb > device_sm_count()) cb *= 2;
 #define X(C)                                                                                           \
     if (cb == C) {                                                                                     \
-        launch_kernel(k_direct_grid<C>, (f.na + C - 1) / C, kGridThreads, grid_smem(C, f.na, f.nb), st, f); \
+        launch_pdl(false, k_direct_grid<C>, (f.na + C - 1) / C, kGridThreads, grid_smem(C, f.na, f.nb), st, f); \
         count_launches(1);                                                                             \
     }
     PREC_DIRECT_GRID(X)

@@ -6,17 +6,18 @@
 namespace precgpu {
 
 template <int SET>
-__global__ void __launch_bounds__(kCarryThreads) k_crt_carry(ProdArgs args, const ProdPtrs* __restrict__ batch) {
+__global__ void __launch_bounds__(kCarryThreads, set_wide(SET) ? 6 : 5) k_crt_carry(ProdArgs args, const ProdPtrs* __restrict__ batch) {
+    pdl_enter();
     crt_carry_tile<SET>(args, batch, GridIdx{});
 }
 
 void launch_crt_carry(int set, const ProdArgs& a, cudaStream_t st, const ProdPtrs* batch, int count, int max_nblk,
                       int nblk_launch) {
     const dim3 grid(batch ? max_nblk : (nblk_launch > 0 ? nblk_launch : a.nblk), 1, count);
-    if (set == 0) launch_kernel(k_crt_carry<0>, grid, kCarryThreads, 0, st, a, batch);
-    else if (set == 1) launch_kernel(k_crt_carry<1>, grid, kCarryThreads, 0, st, a, batch);
-    else if (set == kWideSet) launch_kernel(k_crt_carry<kWideSet>, grid, kCarryThreads, 0, st, a, batch);
-    else launch_kernel(k_crt_carry<kWideSetL>, grid, kCarryThreads, 0, st, a, batch);
+    if (set == 0) launch_pdl(a.chain != 0, k_crt_carry<0>, grid, kCarryThreads, 0, st, a, batch);
+    else if (set == 1) launch_pdl(a.chain != 0, k_crt_carry<1>, grid, kCarryThreads, 0, st, a, batch);
+    else if (set == kWideSet) launch_pdl(a.chain != 0, k_crt_carry<kWideSet>, grid, kCarryThreads, 0, st, a, batch);
+    else launch_pdl(a.chain != 0, k_crt_carry<kWideSetL>, grid, kCarryThreads, 0, st, a, batch);
     count_launches(1);
 }
 
@@ -49,6 +50,7 @@ void ntt_launch_4step(int set, const ProdArgs& args, cudaStream_t st, cudaEvent_
         for (int p = 0; p < kSetPrimes[set]; ++p) {
             cudaStream_t s = ps->s[p];
             ProdArgs a = args;
+            a.chain = 1;
             a.prime0 = p;
             if (staged) {
                 cudaStreamWaitEvent(s, a_ready, 0);
@@ -67,8 +69,10 @@ void ntt_launch_4step(int set, const ProdArgs& args, cudaStream_t st, cudaEvent_
             cudaEventRecord(ps->join[p], s);
             cudaStreamWaitEvent(st, ps->join[p], 0);
         }
-        if (chunks) launch_crt_chunks(set, args, st, *chunks);
-        else launch_crt_carry(set, args, st);
+        ProdArgs a = args;
+        a.chain = 1;
+        if (chunks) launch_crt_chunks(set, a, st, *chunks);
+        else launch_crt_carry(set, a, st);
         return;
     }
     if (ev) cudaEventRecord(ev[0], st);

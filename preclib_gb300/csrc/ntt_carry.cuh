@@ -107,7 +107,7 @@ struct WideEdge {
 // of warp 0 recomputing the block's edge after their own four kept the
 // other warps waiting at the barrier: 3.9 stalled warps per issue).
 template <bool LAZY>
-__device__ __forceinline__ void wide_sums(const ProdPtrs& PP, const ProdArgs& args, int64_t m0, u128 (&T)[kCarryLimbs],
+__device__ __forceinline__ void wide_sums(const uint32_t* __restrict__ work, const ProdArgs& args, int64_t m0, u128 (&T)[kCarryLimbs],
                                           uint64_t& prev_hi, WideEdge* s_edge) {
     static_assert(kCarryLimbs >= 4 && kCarryLimbs % 4 == 0, "limbs per thread: whole 16-byte loads");
     constexpr int L = kCarryLimbs;
@@ -120,7 +120,7 @@ __device__ __forceinline__ void wide_sums(const ProdPtrs& PP, const ProdArgs& ar
             uint4 r[5];
 #pragma unroll
             for (int j = 0; j < 5; ++j)
-                r[j] = __ldg(reinterpret_cast<const uint4*>(PP.work + (uint64_t)(2 * j) * N + m0) + h);
+                r[j] = __ldg(reinterpret_cast<const uint4*>(work + (uint64_t)(2 * j) * N + m0) + h);
             uint32_t y[5];
 #pragma unroll
             for (int j = 0; j < 5; ++j) y[j] = r[j].x;
@@ -137,7 +137,7 @@ __device__ __forceinline__ void wide_sums(const ProdPtrs& PP, const ProdArgs& ar
         }
     } else {
 #pragma unroll
-        for (int k = 0; k < L; ++k) c[k] = coef5<LAZY>(PP.work, N, m0 + k, args);
+        for (int k = 0; k < L; ++k) c[k] = coef5<LAZY>(work, N, m0 + k, args);
     }
     const u128 s_last = limb_sum(c[L - 1], c[L - 2].w1, c[L - 3].w2);
     const uint32_t hi_last = (uint32_t)(s_last >> 64);
@@ -174,6 +174,7 @@ __device__ __forceinline__ void crt_carry_tile(const ProdArgs& args, const ProdP
     __shared__ uint32_t s_last;
     __shared__ WideEdge s_edge[kCarryThreads / 32];
     const ProdPtrs PP = select_product_at(args, batch, ix.z());
+    const uint32_t* __restrict__ work = after_entry(PP.work);
     const uint32_t bid = args.crt_blk0 + ix.x();  // chunked CRT: blocks from crt_blk0
     if ((int)bid >= PP.nblk) return;  // batch: a shorter product of the class
     const uint64_t N = 1ull << args.k;
@@ -186,11 +187,11 @@ __device__ __forceinline__ void crt_carry_tile(const ProdArgs& args, const ProdP
     u128 T[kCarryLimbs];
     uint64_t prev_hi = 0;
     if constexpr (set_wide(SET)) {
-        wide_sums<SET == kWideSet>(PP, args, m0, T, prev_hi, s_edge);
+        wide_sums<SET == kWideSet>(work, args, m0, T, prev_hi, s_edge);
     } else {
-        const uint32_t* __restrict__ r0 = PP.work;
-        const uint32_t* __restrict__ r1 = PP.work + 2 * N;
-        const uint32_t* __restrict__ r2 = PP.work + 4 * N;
+        const uint32_t* __restrict__ r0 = work;
+        const uint32_t* __restrict__ r1 = work + 2 * N;
+        const uint32_t* __restrict__ r2 = work + 4 * N;
         const uint64_t i0 = 2 * (uint64_t)m0;
         if (i0 + 2 * kCarryLimbs <= N) {
             uint32_t y[3][2 * kCarryLimbs];

@@ -73,6 +73,7 @@ __device__ __forceinline__ void col_top_upper_zero(uint32_t* sm, const uint2* __
 template <int SET, int M, int C, int MR, int K2 = 0>
 __global__ void __launch_bounds__(256, cols_minb(M, MR)) k_fwd_cols(ProdArgs args, const ProdPtrs* __restrict__ batch) {
     extern __shared__ uint32_t sm[];
+    pdl_enter();
 #define PREC_K2 K2
 #define PREC_TILE_X blockIdx.x
 #define PREC_TILE_Y blockIdx.y
@@ -101,6 +102,7 @@ __global__ void __launch_bounds__(256, 3) k_fwd_cols_pipe(ProdArgs args, const P
     static_assert(set_wide(SET), "64-bit digits: whole limbs staged");
     static_assert(K2 > 0, "a constant row length");
     extern __shared__ uint32_t sm[];
+    pdl_enter();
     constexpr int NP = sch_np(M, MR);
     constexpr int TW = C * astride_for(M);  // words per tile buffer
     const ProdPtrs P = select_product(args, batch);
@@ -112,7 +114,6 @@ __global__ void __launch_bounds__(256, 3) k_fwd_cols_pipe(ProdArgs args, const P
     constexpr uint32_t N2 = 1u << K2;
     constexpr int KK = M + K2;  // log2 of the transform length
     constexpr int nbx = (int)(N2 / C);
-    if (args.publish && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *args.publish = P;
     const uint64_t nl = operand ? P.lb : P.la;
     if (nl > (1ull << (KK - 1))) {  // the plan puts both operands in the lower half
         if (threadIdx.x == 0) atomicOr(args.err, kDevErrPlan);
@@ -190,6 +191,7 @@ __device__ __forceinline__ void fwd_cols_tile(const ProdArgs& args, const ProdPt
 template <int SET, int M, int C, int MR, int K2 = 0>
 __global__ void __launch_bounds__(256, cols_minb(M, MR)) k_inv_cols(ProdArgs args, const ProdPtrs* __restrict__ batch) {
     extern __shared__ uint32_t sm[];
+    pdl_enter();
 #define PREC_K2 K2
 #define PREC_TILE_X blockIdx.x
 #define PREC_TILE_Y blockIdx.y

@@ -17,12 +17,12 @@ bool launch_fwd_cols_k2(int set, const ProdArgs& a, int cg, int mr, dim3 grid, s
     if (one_prime && !batch && !a.operand_only && set == kWideSet && a.k1 == 10 && a.k2 == 11 && cg == 8 &&
         mr == 6) {
         const dim3 pg((grid.x + kFwdPipeTiles - 1) / kFwdPipeTiles, grid.y, grid.z);
-        launch_kernel(k_fwd_cols_pipe<kWideSet, 10, 8, 6, 11>, pg, 256, 2 * smem, st, a, batch);
+        launch_pdl(a.chain != 0, k_fwd_cols_pipe<kWideSet, 10, 8, 6, 11>, pg, 256, 2 * smem, st, a, batch);
         return true;
     }
 #define X(S, MM, CC, RR, KK)                                                                   \
     if (set == S && a.k1 == MM && cg == CC && mr == RR && a.k2 == KK) {                         \
-        launch_kernel(k_fwd_cols<S, MM, CC, RR, KK>, grid, 32 * CC, smem, st, a, batch);        \
+        launch_pdl(a.chain != 0, k_fwd_cols<S, MM, CC, RR, KK>, grid, 32 * CC, smem, st, a, batch);        \
         return true;                                                                            \
     }
     PREC_COLS_FWD_K2_CONFIGS(X)

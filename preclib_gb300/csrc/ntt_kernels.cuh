@@ -66,13 +66,13 @@ struct ProdArgs {
     int prime0;         // first prime of this launch of the transform kernels (grid.y covers the rest)
     int cg;             // columns per column-pass CTA (0: default)
     int cmr;            // column pass radix cap, 4 or 6 (0: default)
+    int chain;          // per-prime chains (host side: how the kernels are launched)
     int operand_only;   // forward columns of one operand: 1 = a, 2 = b (0: both)
     int rmr;            // row pass radix cap, 4 or 6 (0: default)
     int crt_chunk;      // CRT in limb chunks (chunk_words set): this launch's chunk
     int crt_blk0;       //   its first carry block
     int crt_last;       //   whether it is the last chunk
     uint32_t* chunk_words;  // per chunk: [2c] finished blocks, [2c+1] carry into chunk c (nullptr: one launch)
-    ProdPtrs* publish;      // forward columns store the product's ProdPtrs here for the later kernels (or nullptr)
     CrtConst crt;       // sets 0 and 1
     Crt5Const crt5;     // set 2
     FieldArgs f;
@@ -93,6 +93,21 @@ struct ProdPtrs {
 };
 
 #ifdef __CUDACC__
+// Programmatic dependent launch (launch_pdl): a kernel may start while the
+// one before it in its stream still runs.  pdl_enter, at the top of every
+// kernel so launched, waits for that kernel's end (its writes are then
+// visible).  pdl_next lets the next kernel start once every CTA got there;
+// only the direct products use it: CTAs of a large product's next pass that
+// wait on an SM keep running passes off it (1M x 1M 162 -> 173 us).
+__device__ __forceinline__ void pdl_enter() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// p, for loads that must not move above pdl_enter: read-only loads count as
+// independent of every store, but not of the pointer they use
+template <class T>
+__device__ __forceinline__ T* after_entry(T* p) {
+    asm volatile("" : "+l"(p));
+    return p;
+}
 // the product this CTA works on: the launch's own arguments, or entry
 // blockIdx.z of a batch's descriptor array (a separate value, so the kernel
 // parameter block is never written and stays in the constant bank)
@@ -215,6 +230,33 @@ inline void launch_kernel(void (*k)(P...), dim3 grid, dim3 block, size_t smem, c
     } else {
         k<<<grid, block, smem, st>>>(std::forward<A>(args)...);
     }
+}
+
+// launch_kernel for a kernel that begins with pdl_enter: launched in a
+// stream, it starts without waiting for the end of the stream's previous
+// kernel to reach the launch queue.  GB300 starts a dependent kernel on a
+// 2.05 us tick otherwise: four dependent kernels of 2 us each took 16.4 us
+// back to back, 14.3 as one graph, 10.8 this way.
+// (chain: a kernel of a per-prime chain, launched plainly -- beside four other
+// chains there is nothing to gain, and it measured slower: square of 300007
+// limbs 61.4 -> 62.9 us)
+template <class... P, class... A>
+inline void launch_pdl(bool chain, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    if (chain || thread_recorder()) {
+        launch_kernel(k, grid, block, smem, st, std::forward<A>(args)...);
+        return;
+    }
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, static_cast<P>(std::forward<A>(args))...);
 }
 
 // Kernel launches issued by the library (process-wide, prec_gpu_launch_count);

@@ -22,6 +22,7 @@ namespace precgpu {
 template <int SET, int M, bool SQ, int MR>
 __global__ void __launch_bounds__(256, MR == 6 ? 2 : PREC_ROWS_MINB) k_rows(ProdArgs args, const ProdPtrs* __restrict__ batch) {
     extern __shared__ uint32_t sm[];
+    pdl_enter();
     rows_tile<SET, M, SQ, MR>(args, batch, GridIdx{}, sm);
 }
 
@@ -59,7 +60,7 @@ void launch_rows(int set, const ProdArgs& a, cudaStream_t st, const ProdPtrs* ba
     const int mr = row_radix_cap(m, a.rmr);
 #define X(S, MM, SQ, RR)                                                                  \
     if (set == S && m == MM && (a.square != 0) == SQ && mr == RR) {                       \
-        launch_kernel(k_rows<S, MM, SQ, RR>, grid, threads, smem, st, a, batch);                 \
+        launch_pdl(a.chain != 0, k_rows<S, MM, SQ, RR>, grid, threads, smem, st, a, batch);                 \
         count_launches(1);                                                              \
         return;                                                                         \
     }

@@ -35,7 +35,7 @@ __device__ __forceinline__ void rows_tile(const ProdArgs& args, const ProdPtrs* 
     const uint2* __restrict__ twf = args.f.tf[prime];
     const uint2* __restrict__ twi = args.f.ti[prime];
     const int rows = args.rows;
-    uint32_t* __restrict__ A = P.work + ((uint64_t)(prime * 2) << args.k);
+    uint32_t* __restrict__ A = after_entry(P.work) + ((uint64_t)(prime * 2) << args.k);
     const uint32_t* __restrict__ B = A + (1ull << args.k);
     const uint32_t row0 = ix.x() * rows;
     constexpr int NA = SQ ? 1 : 2;  // a square transforms its one operand only

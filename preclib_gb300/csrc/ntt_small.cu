@@ -25,7 +25,10 @@ __global__ void __launch_bounds__(256) k_small(const SmallDesc* __restrict__ des
     __shared__ BlockCarryShared sh;
     constexpr int NP = sch_np(M);
     constexpr int AS = astride_for(M);
-    const SmallDesc d = descs ? descs[blockIdx.x] : single;
+    pdl_enter();
+    SmallDesc d = descs ? descs[blockIdx.x] : single;
+    d.a = after_entry(d.a);
+    d.b = after_entry(d.b);
     const uint32_t* __restrict__ da = reinterpret_cast<const uint32_t*>(d.a);
     const uint32_t* __restrict__ db = reinterpret_cast<const uint32_t*>(d.b);
     const uint64_t nda = 2 * d.la, ndb = 2 * d.lb;
@@ -165,7 +168,7 @@ void ntt_launch_small(const SmallDesc* d_descs, const SmallDesc* single, int cou
     const size_t smem = ntt_small_smem_bytes(k);
 #define X(MM) \
     if (k == MM) {                                                     \
-        launch_kernel(k_small<MM>, count, threads, smem, st, d_descs, one, f, crt); \
+        launch_pdl(false, k_small<MM>, count, threads, smem, st, d_descs, one, f, crt); \
         count_launches(1);                                             \
     }
     PREC_SMALL(X)

@@ -8,8 +8,8 @@
 //     prime and direction serves every transform length);
 //   * per calling thread, a lane (Lane): a stream for the host-pointer
 //     entry points, a workspace and staging buffers that grow to the
-//     largest product the thread has made, and its graphs, so
-//     products from different threads overlap on the device.
+//     largest product the thread has made, so products from
+//     different threads overlap on the device.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -245,35 +245,9 @@ int plan_for(uint64_t da, uint64_t db, uint64_t lout, Plan& pl, bool wide) {
     return 0;
 }
 
-// A single four-step product up to 2^kGraphMaxLog2 points runs as one CUDA
-// graph replay: its kernels are the batch form's with a one-entry
-// descriptor array, built once per plan shape; each call uploads the
-// descriptor (operands, output, workspace, sizes) and launches the graph.
-// Below 2^19 points the four kernels take only a few microseconds each,
-// so launching them one by one left the GPU waiting on the host.
-constexpr int kGraphMaxLog2 = 18;
-
-struct GraphKey {
-    int set, k, k1, cg, cmr, rmr, rows, square;
-    bool operator<(const GraphKey& o) const {
-        const int a[8] = {set, k, k1, cg, cmr, rmr, rows, square};
-        const int b[8] = {o.set, o.k, o.k1, o.cg, o.cmr, o.rmr, o.rows, o.square};
-        return std::lexicographical_compare(a, a + 8, b, b + 8);
-    }
-};
-
-struct GraphEntry {
-    cudaGraphExec_t exec = nullptr;
-    ProdPtrs* d_desc = nullptr;  // the one-entry descriptor array the later kernels read
-    uint64_t launches = 0;       // kernels per replay
-    cudaGraphNode_t first = nullptr;  // the forward column node: the product's arguments by value
-    cudaKernelNodeParams params{};
-    cudaGraph_t graph = nullptr;  // kept: a node's parameters are set through its graph's node handle
-};
-
 // One calling thread's resources (a "lane"): its streams, the per-product
 // workspace and staging buffers, the status block a host product reads
-// back, events, per-prime streams and single-product graphs.
+// back, events and per-prime streams.
 // Products on different lanes run concurrently on the GPU; a lane runs one
 // product at a time (mu).  A thread takes a lane on its first call and
 // keeps it; past kMaxLanes threads, threads share lanes round-robin.  (The
@@ -308,7 +282,6 @@ struct Lane {
     uint32_t* chunk_words = nullptr;  // 2 * kCrtMaxChunks words
     uint32_t* direct_counter = nullptr;  // finished CTAs of a direct product (zero between products)
     PrimeStreams prime_streams = {};
-    std::map<GraphKey, GraphEntry> graphs;  // single-product graphs by plan shape
 };
 
 struct Ctx {
@@ -539,12 +512,6 @@ static int init_locked(Ctx& c, int device) {
 
 static void lane_destroy(Lane& L) {
     if (L.stream) cudaStreamSynchronize(L.stream);
-    for (auto& kv : L.graphs) {
-        cudaGraphExecDestroy(kv.second.exec);
-        cudaGraphDestroy(kv.second.graph);
-        cudaFree(kv.second.d_desc);
-    }
-    L.graphs.clear();
     cudaFree(L.ws);
     cudaFree(L.io);
     cudaFree(L.blk);
@@ -726,74 +693,6 @@ static int ensure_io(Lane& L, size_t limbs) {
 // Enqueues one NTT-band product on device pointers.
 // A square (d_a == d_b, la == lb) transforms its one operand only on the
 // four-step path; the single-CTA path reads the operand twice.
-// One four-step product as a replay of its shape's graph (built on first
-// use).  The forward column kernel takes the product by value -- a replay
-// sets that node's parameters -- and stores its descriptor for the row,
-// inverse column and carry kernels, which run in batch form on it.  (An
-// upload of the descriptor by a copy in the stream measured 8-10 us slower
-// per product when the caller's operands were page-locked.)
-static int enqueue_graph(Lane& L, const ProdArgs& args, const Plan& pl, cudaStream_t st) {
-    const GraphKey key{pl.set, pl.k, pl.k1, pl.cg, pl.cmr, pl.rmr, pl.rows, args.square};
-    auto it = L.graphs.find(key);
-    if (it == L.graphs.end()) {
-        GraphEntry e;
-        CK(cudaMalloc(&e.d_desc, sizeof(ProdPtrs)));
-        ProdArgs first = args;
-        first.publish = e.d_desc;
-        ProdArgs cls = args;  // class-wide fields; the product's own come from the descriptor
-        cls.a = cls.b = nullptr;
-        cls.out = nullptr;
-        cls.work = cls.scratch = nullptr;
-        const uint64_t lout_max = set_wide(pl.set) ? (1ull << pl.k) + 1 : (1ull << pl.k) / 2 + 1;
-        const uint64_t bl = (uint64_t)crt_block_limbs(pl.set);
-        const int max_nblk = (int)((lout_max + bl - 1) / bl);
-        // the four launches as a chain of kernel nodes (explicit
-        // construction: no stream capture)
-        GraphRecorder rec;
-        cudaError_t err = cudaGraphCreate(&rec.graph, 0);
-        if (err != cudaSuccess) {
-            cudaFree(e.d_desc);
-            return cuda_code(err);
-        }
-        const uint64_t before = launches_this_thread();
-        t_recorder = &rec;
-        launch_fwd_cols(pl.set, first, L.cap);
-        launch_rows(pl.set, cls, L.cap, e.d_desc, 1);
-        launch_inv_cols(pl.set, cls, L.cap, e.d_desc, 1);
-        launch_crt_carry(pl.set, cls, L.cap, e.d_desc, 1, max_nblk);
-        t_recorder = nullptr;
-        e.launches = launches_this_thread() - before;  // recorded, counted at every replay
-        uncount_launches(e.launches);
-        cudaGraph_t g = rec.graph;
-        err = rec.err;
-        // the forward column node: the first recorded
-        cudaGraphNode_t root = rec.first;
-        if (err == cudaSuccess && root) err = cudaGraphKernelNodeGetParams(root, &e.params);
-        if (err == cudaSuccess && !root) err = cudaErrorInvalidValue;
-        e.first = root;
-        if (err == cudaSuccess) err = cudaGraphInstantiate(&e.exec, g, 0);
-        if (err != cudaSuccess) {
-            if (g) cudaGraphDestroy(g);
-            cudaFree(e.d_desc);
-            return cuda_code(err);
-        }
-        e.graph = g;
-        it = L.graphs.emplace(key, e).first;
-    }
-    GraphEntry& e = it->second;
-    ProdArgs first = args;
-    first.publish = e.d_desc;
-    const ProdPtrs* no_batch = nullptr;
-    void* params[2] = {&first, &no_batch};
-    cudaKernelNodeParams kp = e.params;
-    kp.kernelParams = params;
-    kp.extra = nullptr;
-    CK(cudaGraphExecKernelNodeSetParams(e.exec, e.first, &kp));
-    CK(cudaGraphLaunch(e.exec, st));
-    count_launches(e.launches);
-    return 0;
-}
-
 // Device error bits go to `err` (the lane's status block for host
 // products, the library-wide word otherwise).
 static int enqueue_ntt(Ctx& c, Lane& L, const uint64_t* d_a, uint64_t la, const uint64_t* d_b, uint64_t lb,
@@ -837,12 +736,6 @@ static int enqueue_ntt(Ctx& c, Lane& L, const uint64_t* d_a, uint64_t la, const 
         args.crt5 = pl.crt5;
         args.f = c.field[pl.set];
         const bool split = c.split_primes && pl.split;
-        // (a caller capturing `st` into its own graph gets plain launches: the
-        // descriptor upload reads host memory that is gone at its replay)
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (!split && !ev && pl.k <= kGraphMaxLog2 && cudaStreamIsCapturing(st, &cap) == cudaSuccess &&
-            cap == cudaStreamCaptureStatusNone)
-            return enqueue_graph(L, args, pl, st);
         ntt_launch_4step(pl.set, args, st, ev, split ? &L.prime_streams : nullptr, a_ready, b_ready,
                          split ? chunks : nullptr);
     }
@@ -1038,11 +931,12 @@ static int host_mul(const uint64_t* a, size_t an, const uint64_t* b, size_t bn, 
     cudaStream_t st = L.stream;
     NvtxRange range("prec_gpu_mul %zux%zu %s", la, lb, use_fft ? "fft" : (blocked ? "blocked" : "ntt"));
     if ((r = lane_begin(L, st))) return r;
-    // the per-prime chains start on a's forward columns while b is copied
+    // per-prime chains start on a's forward columns while b is copied
+    const bool chains = !use_fft && !blocked && pl.path == 1 && c.split_primes && pl.split;
     CK(cudaMemcpyAsync(d_a, a, la * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-    CK(cudaEventRecord(L.ev_a, st));
+    if (chains) CK(cudaEventRecord(L.ev_a, st));
     if (!square) CK(cudaMemcpyAsync(d_b, b, lb * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-    CK(cudaEventRecord(L.ev_b, st));
+    if (chains) CK(cudaEventRecord(L.ev_b, st));
     CK(cudaEventRecord(L.ev0, st));
     bool copied = false;  // the result went out chunk by chunk
     nvtxRangePushA("enqueue product");
@@ -1073,7 +967,7 @@ static int host_mul(const uint64_t* a, size_t an, const uint64_t* b, size_t bn, 
         // a large product's CRT runs in limb chunks; each chunk's limbs copy
         // out on the copy stream while the next chunks run
         CrtChunks ch{};
-        const bool chunked = pl.path == 1 && c.split_primes && pl.split && pl.nblk >= 2 * kCrtMaxChunks;
+        const bool chunked = chains && pl.nblk >= 2 * kCrtMaxChunks;
         if (chunked) {
             const int per = (pl.nblk + kCrtMaxChunks - 1) / kCrtMaxChunks;
             ch.count = (pl.nblk + per - 1) / per;  // every chunk nonempty
@@ -1082,7 +976,8 @@ static int host_mul(const uint64_t* a, size_t an, const uint64_t* b, size_t bn, 
             for (int i = 0; i < ch.count; ++i) ch.done[i] = L.chunk_done[i];
             CK(cudaMemsetAsync(L.chunk_words, 0, 2 * kCrtMaxChunks * sizeof(uint32_t), st));
         }
-        if ((r = enqueue_ntt(c, L, d_a, la, d_b, lb, d_out, pl, st, L.d_err, nullptr, L.ev_a, L.ev_b, chunked ? &ch : nullptr)))
+        if ((r = enqueue_ntt(c, L, d_a, la, d_b, lb, d_out, pl, st, L.d_err, nullptr, chains ? L.ev_a : nullptr,
+                             chains ? L.ev_b : nullptr, chunked ? &ch : nullptr)))
             return r;
         if (chunked) {
             const uint64_t bl = (uint64_t)crt_block_limbs(pl.set);
