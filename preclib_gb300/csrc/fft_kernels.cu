@@ -344,6 +344,7 @@ __global__ void __launch_bounds__(kFftCarryThreads) k_fft_carry(const FftArgs* _
     __shared__ uint32_t s_bmap[kFftCarryThreads];
     __shared__ uint32_t s_last;
     const double dist = *f.maxdist;
+    if (f.host_dist && blockIdx.x == 0 && threadIdx.x == 0) *f.host_dist = dist;
     if (!(dist <= 0.25)) {  // also NaN / inf: nothing is written
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(f.err, kDevErrFftRound);
         return;
@@ -452,6 +453,19 @@ __global__ void __launch_bounds__(kFftCarryThreads) k_fft_carry(const FftArgs* _
     // a product fits La+Lb limbs: everything above must be zero
     for (int64_t m = Lout + threadIdx.x; m < L; m += blockDim.x)
         if (__ldcg(&high[m - Lout]) != 0) atomicOr(f.err, kDevErrCarry);
+}
+
+__global__ void __launch_bounds__(256) k_stage(ulonglong2* dst, const ulonglong2* __restrict__ src, uint64_t n2) {
+    pdl_enter();
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n2) dst[i] = src[i];
+}
+
+void launch_stage(uint64_t* dst, const uint64_t* src, uint64_t n, cudaStream_t st) {
+    const uint64_t n2 = (n + 1) / 2;
+    launch_pdl(false, k_stage, (unsigned)((n2 + 255) / 256), 256, 0, st, reinterpret_cast<ulonglong2*>(dst),
+               reinterpret_cast<const ulonglong2*>(src), n2);
+    count_launches(1);
 }
 
 // e^(2 pi i e / 2^16) for e < 2^15

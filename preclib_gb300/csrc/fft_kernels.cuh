@@ -19,6 +19,7 @@ struct FftArgs {
     double2* work;        // N complex values
     long long* coef;      // N rounded coefficients
     double* maxdist;      // max |x - round(x)| of this product
+    double* host_dist;    // page-locked copy of it for the host, or nullptr
     int* err;
     const double2* tw;    // e^(2 pi i e / 2^16), e < 2^15
     uint64_t la, lb, lout;
@@ -29,6 +30,10 @@ struct FftArgs {
 };
 
 constexpr int fpad_host(int i) { return i + (i >> 4); }
+
+// dst[0 .. n) = src[0 .. n) limbs, both on 16-byte boundaries; src may be
+// page-locked host memory
+void launch_stage(uint64_t* dst, const uint64_t* src, uint64_t n, cudaStream_t st);
 
 size_t fft_table_bytes();
 void fft_build_table(double2* tw, cudaStream_t st);
