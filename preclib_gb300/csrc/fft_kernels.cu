@@ -3,609 +3,524 @@
 // Replaces preclib's mul_fft (src/mul_fft.cpp:340-394) with the same method
 // -- both operands packed as the real and imaginary parts of one complex
 // FP64 FFT (fft_load_digits, 234-246), the two spectra separated and
-// multiplied (fft_pair_convolution, 248-305), one inverse FFT, rounding to
-// the nearest integer (307-309, 364-376) and a signed carry back to limbs
+// multiplied (fft_pair_convolution, 248-305), the inverse FFT, rounding to
+// the nearest integer (307-309, 364-376) and a carry back to limbs
 // (fft_from_digits, 311-338) -- laid out for many SMs:
 //
 //  digits   balanced b-bit digits (|d| <= 2^(b-1)), b chosen per transform
 //           length from a worst-case error bound (host side); every digit
 //           is computed on its own: d_i = raw_i - 2^b t_i + t_{i-1} with
 //           t_j = [raw_j >= 2^(b-1)], so no carry chain is needed.
-//  twiddles one table of e^(2 pi i e / 2^16), e < 2^15, from sincospi()
-//           (the reference builds per-stage tables by a recurrence,
-//           mul_fft.cpp:57-76).
+//  twiddles two tables from sincospi() (the reference builds per-stage tables
+//           by a recurrence, mul_fft.cpp:57-76): e^(2 pi i e / 2^16) in
+//           natural order for the inverse, e^(-pi i 0.b0b1b2..) by the bits
+//           of the block index for the forward transform.
 //  four-step N = N1 * N2:
-//    k_fft_fwd_cols  digits -> column DIF over i1 -> twiddle w^-(i2 k1)
-//    k_fft_rows      rows k1 and N1-k1 together: row DIF, separation and
-//                    product (P_-k = conj P_k), row DIT, twiddle w^(i2 k1)
-//    k_fft_inv_cols  column DIT -> x/N -> nearest integer, max distance
-//    k_fft_carry     limbs from the signed coefficients (blocks, then the
-//                    last block joins their carries); writes nothing when
+//    k_fft_digits    limbs (device or page-locked host memory) -> digits
+//    k_fft_fwd_cols  columns: the top log2 N1 levels of the transform
+//    k_fft_rows      rows k1 and N1-k1 together: the other levels, product
+//                    (P_-k = conj P_k), fold to half length, inverse levels
+//    k_fft_inv_cols  columns of the inverse -> x scale -> nearest integer,
+//                    max distance
+//    k_fft_carry     limbs from the signed coefficients; writes nothing when
 //                    the max distance exceeds 0.25.
+//
+// What bounds it: FP64 issue.  GB300 takes one FP64 warp instruction per 64
+// cycles on each SM quarter (measured; 19 cycles per SM with all four
+// busy), whatever the kind and at no extra latency.  So the transform is
+// arranged for few FP64 instructions and for four warps per SM, and integer
+// work, shared memory and barriers come free beside it:
+//   * a butterfly (x + wy, x - wy) is 8 fused operations, two chained fma per
+//     part (x - wy = 2x - (x + wy) would make it 6, 1.5 us less at 3000 x 3000
+//     limbs, but its mean rounding distance came out 7% above the earlier
+//     kernels'; this form's is 2% below);
+//   * forward: block q of a level splits x^2m - r^2 into x^m -+ r, one twiddle
+//     per block, natural to bit-reversed order: the four-step twiddles are
+//     part of the rows' own twiddles and cost nothing;
+//   * inverse: stage b pairs i and i + 2^b with w^(i mod 2^b), over the whole
+//     index: again no separate twiddles;
+//   * product: 4 i P_k = F_k^2 - conj(F_-k)^2, 7 operations;
+//   * the inverse output is real: P is folded to Z_k = E_k + i O_k of half
+//     length, whose inverse has the even coefficients as real and the odd
+//     ones as imaginary parts.
+// Per call: 256 x 193 limbs 45.5 -> 32.0 us, 3000 x 3000 59.5 -> 42.1,
+// 6144 x 6144 80.4 -> 53.5 (kernels alone 34 -> 20, 46 -> 29, 63 -> 35).
 #include <cuda_runtime.h>
 
-#include <map>
-#include <mutex>
-#include <tuple>
-#include <vector>
+#include <cooperative_groups.h>
 
 #include "fft_kernels.cuh"
-#include "ntt_kernels.cuh"
+#include "ntt_engine.cuh"
 
 namespace precgpu {
 
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-    return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
-}
-__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 conj2(double2 a) { return make_double2(a.x, -a.y); }
-
-// w_N^e = e^(2 pi i e / N) for 0 <= e < N, N = 2^k <= 2^16
-__device__ __forceinline__ double2 root(const double2* __restrict__ tw, uint32_t e, int k) {
-    const uint32_t half = 1u << (k - 1);
-    const double2 w = __ldg(&tw[(e & (half - 1)) << (kFftMaxLog2 - k)]);
-    return (e & half) ? make_double2(-w.x, -w.y) : w;
-}
-
-__device__ __forceinline__ int fpad(int i) { return i + (i >> 4); }  // 16-byte elements, 1 spare per 16
-
-// raw b-bit digit i of an n-limb operand (zero past its top)
-__device__ __forceinline__ uint32_t raw_digit(const uint64_t* __restrict__ a, uint64_t n, int b, uint64_t i) {
-    const uint64_t bit = (uint64_t)b * i;
-    const uint64_t limb = bit >> 6;
-    const int sh = (int)(bit & 63);
-    uint64_t v = limb < n ? __ldg(&a[limb]) >> sh : 0;
-    if (sh + b > 64 && limb + 1 < n) v |= __ldg(&a[limb + 1]) << (64 - sh);
+// raw b-bit digit starting at bit `bit` of the limbs s (one past them readable)
+__device__ __forceinline__ uint32_t raw_digit(const uint64_t* s, uint32_t bit, int b) {
+    const uint32_t l = bit >> 6, sh = bit & 63;
+    uint64_t v = s[l] >> sh;
+    if (sh + b > 64) v |= s[l + 1] << (64 - sh);
     return (uint32_t)(v & ((1ull << b) - 1));
 }
 
-// balanced digit i (|d| <= 2^(b-1)) of an operand with `nd` digits
-__device__ __forceinline__ double bal_digit(const uint64_t* __restrict__ a, uint64_t n, int b, uint64_t i, uint64_t nd) {
-    if (i >= nd) return 0.0;
-    const uint32_t half = 1u << (b - 1);
-    const uint32_t r = raw_digit(a, n, b, i);
-    const int t_in = i > 0 && raw_digit(a, n, b, i - 1) >= half ? 1 : 0;
-    const int t_out = r >= half ? 1 : 0;
-    return (double)((int64_t)r - ((int64_t)t_out << b) + t_in);
+// an exact double from an integer |d| < 2^31
+__device__ __forceinline__ double small_double(int d) {
+    return __hiloint2double(0x43300000, d ^ (int)0x80000000) - __hiloint2double(0x43300000, (int)0x80000000);
 }
 
-// One register pass: stages over bits lo .. lo+RB-1 of `narr` arrays of 2^m
-// points in shared memory (array stride `as`, element i at fpad(i)); item u
-// holds elements base + (q << lo), q < 2^RB.  DIF (forward, sign -1,
-// natural -> bit-reversed) runs the pass's stages from its top bit down, DIT
-// (inverse, sign +1, bit-reversed -> natural) from its bottom bit up; the
-// stage at bit b pairs i and i + 2^b with twiddle w_(2^(b+1))^(i mod 2^b).
-template <bool DIT, int RB>
-__device__ __forceinline__ void fft_pass(double2* s, int as, int narr, int m, int lo, const double2* __restrict__ tw) {
-    const int lgper = m - RB;
-    const uint32_t lomask = (1u << lo) - 1;
-    for (int w = threadIdx.x; w < (narr << lgper); w += blockDim.x) {
-        const int a = w >> lgper;
-        const uint32_t u = w & ((1u << lgper) - 1);
-        const uint32_t base = ((u >> lo) << (lo + RB)) | (u & lomask);
-        const uint32_t ulo = u & lomask;
-        double2* row = s + a * as;
-        double2 x[1 << RB];
-#pragma unroll
-        for (int q = 0; q < (1 << RB); ++q) x[q] = row[fpad((int)(base + ((uint32_t)q << lo)))];
-#pragma unroll
-        for (int t = 0; t < RB; ++t) {
-            const int bb = DIT ? t : RB - 1 - t;
-            const int h = 1 << bb;
-#pragma unroll
-            for (int q = 0; q < (1 << RB); ++q) {
-                if (q & h) continue;
-                const uint32_t j = ulo | ((uint32_t)(q & (h - 1)) << lo);
-                const double2 X = x[q], Y = x[q + h];
-                double2 r = make_double2(1.0, 0.0);
-                if (j) {
-                    r = root(tw, j << (m - 1 - (lo + bb)), m);
-                    if (!DIT) r.y = -r.y;
-                }
-                if (DIT) {
-                    const double2 tt = j ? cmul(Y, r) : Y;
-                    x[q] = cadd(X, tt);
-                    x[q + h] = csub(X, tt);
-                } else {
-                    x[q] = cadd(X, Y);
-                    const double2 d = csub(X, Y);
-                    x[q + h] = j ? cmul(d, r) : d;
-                }
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < (1 << RB); ++q) row[fpad((int)(base + ((uint32_t)q << lo)))] = x[q];
+constexpr int kDigitThreads = 256;
+constexpr int kDigitLimbs = kDigitThreads * 30 / 64 + 4;  // limbs 257 digits of up to 30 bits touch, and one more
+
+// digits of both operands: element i = (a_i, b_i); starts the distance at 0
+__global__ void __launch_bounds__(kDigitThreads) k_fft_digits(FftArgs f) {
+    __shared__ uint64_t s[2][kDigitLimbs];
+    pdl_enter();
+    const uint64_t i0 = (uint64_t)blockIdx.x * kDigitThreads;
+    // from digit i0 - 1 (its top bit decides digit i0's carry)
+    const uint64_t first = i0 ? i0 - 1 : 0;
+    const uint64_t l0 = first * f.b >> 6;
+    const uint64_t* __restrict__ pa = after_entry(f.a);
+    const uint64_t* __restrict__ pb = after_entry(f.bp);
+    const int nl = (int)(((i0 + kDigitThreads) * f.b + 63) / 64 - l0) + 1;
+    for (int t = threadIdx.x; t < nl; t += kDigitThreads) {
+        s[0][t] = l0 + t < f.la ? __ldg(&pa[l0 + t]) : 0;
+        s[1][t] = l0 + t < f.lb ? __ldg(&pb[l0 + t]) : 0;
     }
-}
-
-template <bool DIT>
-__device__ __forceinline__ void fft_pass_rb(int rb, double2* s, int as, int narr, int m, int lo,
-                                            const double2* __restrict__ tw) {
-    if (rb == 3) fft_pass<DIT, 3>(s, as, narr, m, lo, tw);
-    else if (rb == 2) fft_pass<DIT, 2>(s, as, narr, m, lo, tw);
-    else fft_pass<DIT, 1>(s, as, narr, m, lo, tw);
-}
-
-// the whole 2^m-point transform of `narr` arrays in passes of up to radix
-// 2^PREC_FFT_MAX_RB, one barrier per pass; DIF from the top bits, DIT from the
-// bottom bits.  Radix 2 is the default: at 2^15 points radix-4 and radix-8
-// passes measured 10% and 30% slower (more registers per thread, the same
-// FP64 work, and these kernels are bound by the FP64 pipe and by latency).
-#ifndef PREC_FFT_MAX_RB
-#define PREC_FFT_MAX_RB 1
-#endif
-constexpr int kFftMaxRb = PREC_FFT_MAX_RB;
-
-template <bool DIT>
-__device__ void fft_stages(double2* s, int as, int narr, int m, const double2* __restrict__ tw) {
-    if (!DIT) {
-        for (int top = m; top > 0;) {
-            const int rb = top < kFftMaxRb ? top : kFftMaxRb;
-            fft_pass_rb<false>(rb, s, as, narr, m, top - rb, tw);
-            __syncthreads();
-            top -= rb;
-        }
-    } else {
-        for (int lo = 0; lo < m;) {
-            const int rb = m - lo < kFftMaxRb ? m - lo : kFftMaxRb;
-            fft_pass_rb<true>(rb, s, as, narr, m, lo, tw);
-            __syncthreads();
-            lo += rb;
-        }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *f.maxdist = 0.0;
+    __syncthreads();
+    const uint64_t i = i0 + threadIdx.x;
+    const uint32_t half = 1u << (f.b - 1);
+    const uint32_t bit = (uint32_t)(i * f.b - (l0 << 6));
+    double v[2];
+#pragma unroll
+    for (int o = 0; o < 2; ++o) {
+        const uint32_t r = raw_digit(s[o], bit, f.b);
+        const int t_in = i > 0 && raw_digit(s[o], bit - f.b, f.b) >= half ? 1 : 0;
+        const int d = (int)r - (r >= half ? 1 << f.b : 0) + t_in;
+        v[o] = small_double(i < (o ? f.db : f.da) ? d : 0);
     }
+    if (i < f.ncoef) f.work[i] = make_double2(v[0], v[1]);
+}
+
+// (x, y) -> (x + wy, x - wy)
+__device__ __forceinline__ void butterfly(double2& x, double2& y, double2 w) {
+    const double re = fma(w.x, y.x, fma(-w.y, y.y, x.x));
+    const double im = fma(w.x, y.y, fma(w.y, y.x, x.y));
+    y = make_double2(fma(-w.x, y.x, fma(w.y, y.y, x.x)), fma(-w.x, y.y, fma(-w.y, y.x, x.y)));
+    x = make_double2(re, im);
+}
+// w = 1, and w = -i
+__device__ __forceinline__ void butterfly1(double2& x, double2& y) {
+    const double2 t = x;
+    x = make_double2(t.x + y.x, t.y + y.y);
+    y = make_double2(t.x - y.x, t.y - y.y);
+}
+__device__ __forceinline__ void butterfly_mi(double2& x, double2& y) {
+    const double2 t = x;
+    x = make_double2(t.x + y.y, t.y - y.x);
+    y = make_double2(t.x - y.y, t.y + y.x);
+}
+
+// One column of 2^M points: N1/2 threads, one butterfly each per level; C
+// columns per CTA (one, once a column fills a warp).
+template <int M>
+struct ColGeom {
+    static constexpr int HALF = 1 << (M - 1);
+    static constexpr int THREADS = HALF < 32 ? 32 : HALF;
+    static constexpr int C = THREADS / HALF;
+};
+
+// forward columns: levels 0 .. M-1; grid N2 / C
+template <int M>
+__global__ void __launch_bounds__(ColGeom<M>::THREADS) k_fft_fwd_cols(FftArgs f) {
+    using G = ColGeom<M>;
+    constexpr int H = G::HALF, N1 = 2 * H;
+    __shared__ double2 s[G::C][N1];
+    const int col = threadIdx.x / H, j = threadIdx.x % H;
+    const uint32_t N2 = 1u << f.k2;
+    const uint32_t c = blockIdx.x * G::C + col;
+    double2 w[M];
+#pragma unroll
+    for (int l = 2; l < M; ++l) w[l] = __ldg(&f.twr[j >> (M - 1 - l)]);
+    pdl_enter();
+    const double2* __restrict__ src = after_entry(f.work);
+    const uint64_t nd = f.da > f.db ? f.da : f.db;
+    const bool upper = nd > f.ncoef / 2;  // else the upper half is zero: level 0 copies
+    const uint64_t i = (uint64_t)j * N2 + c;
+    double2 x = make_double2(0.0, 0.0), y = x;
+    if (i < nd) x = src[i];
+    if (upper && i + f.ncoef / 2 < nd) y = src[i + f.ncoef / 2];
+    if (upper) butterfly1(x, y);
+    else y = x;
+    int pos = j;
+#pragma unroll
+    for (int l = 1; l < M; ++l) {
+        s[col][pos] = x;
+        s[col][pos + (H >> (l - 1))] = y;
+        __syncthreads();
+        const int h = H >> l;
+        const int q = j / h;
+        pos = q * 2 * h + j % h;
+        x = s[col][pos];
+        y = s[col][pos + h];
+        if (l == 1) {
+            if (q) butterfly_mi(x, y);
+            else butterfly1(x, y);
+        } else {
+            butterfly(x, y, w[l]);
+        }
+        if (l + 1 < M) __syncthreads();
+    }
+    f.work[(uint64_t)pos * N2 + c] = x;
+    f.work[(uint64_t)(pos + 1) * N2 + c] = y;
 }
 
 __device__ __forceinline__ uint32_t bitrev(uint32_t x, int bits) { return bits ? __brev(x) >> (32 - bits) : 0u; }
 
-// forward column pass: grid N2/C CTAs, C adjacent columns each
-template <int C>
-__global__ void __launch_bounds__(256) k_fft_fwd_cols(FftArgs f, FftArgs* publish) {
-    extern __shared__ double2 fsm[];
-    // the product's arguments for the three kernels after this one
-    if (blockIdx.x == 0 && threadIdx.x == 0) *publish = f;
-    const int N1 = 1 << f.k1;
-    const uint32_t N2 = 1u << f.k2;
-    const int as = fpad(N1) + 1;
-    const uint32_t c0 = blockIdx.x * C;
-    // the product's max distance starts at 0 (the previous product's readers
-    // are earlier in stream order)
-    if (blockIdx.x == 0 && threadIdx.x == 0) *f.maxdist = 0.0;
-    for (int w = threadIdx.x; w < C * N1; w += blockDim.x) {
-        const int col = w % C, i1 = w / C;
-        const uint64_t i = (uint64_t)i1 * N2 + c0 + col;
-        fsm[col * as + fpad(i1)] = make_double2(bal_digit(f.a, f.la, f.b, i, f.da), bal_digit(f.bp, f.lb, f.b, i, f.db));
-    }
-    __syncthreads();
-    fft_stages<false>(fsm, as, C, f.k1, f.tw);
-    for (int w = threadIdx.x; w < C * N1; w += blockDim.x) {
-        const int col = w % C, s = w / C;
-        const uint32_t k1 = bitrev((uint32_t)s, f.k1);
-        const uint32_t i2 = c0 + col;
-        double2 r = root(f.tw, (i2 * k1) & ((1u << f.k) - 1), f.k);
-        r.y = -r.y;
-        f.work[(uint64_t)s * N2 + i2] = cmul(fsm[col * as + fpad(s)], r);
-    }
-}
-
 // row pass: CTA r handles frequency rows k1 = r and N1 - r (one row when
-// they coincide); grid N1/2 + 1
-__global__ void __launch_bounds__(256) k_fft_rows(const FftArgs* __restrict__ fa) {
-    const FftArgs f = *fa;
-    extern __shared__ double2 fsm[];
-    const int N1 = 1 << f.k1, N2 = 1 << f.k2;
-    const int as = fpad(N2) + 1;
-    const uint32_t ka = blockIdx.x, kb = (N1 - blockIdx.x) & (N1 - 1);
-    const int nrow = ka == kb ? 1 : 2;
-    const uint32_t sa = bitrev(ka, f.k1), sb = bitrev(kb, f.k1);
-    double2* rowp[2] = {f.work + (uint64_t)sa * N2, f.work + (uint64_t)sb * N2};
-    for (int w = threadIdx.x; w < nrow * N2; w += blockDim.x) {
-        const int r = w / N2, t = w % N2;
-        fsm[r * as + fpad(t)] = rowp[r][t];
-    }
-    __syncthreads();
-    fft_stages<false>(fsm, as, nrow, f.k2, f.tw);
-    // separation of the packed spectra and product; slot t holds k2 = bitrev(t)
-    double2 prod[8];  // at most 2 * N2 / blockDim = 8 elements per thread
-    int cnt = 0;
-    for (int w = threadIdx.x; w < nrow * N2; w += blockDim.x, ++cnt) {
-        const int r = w / N2, t = w % N2;
-        const uint32_t k1 = r ? kb : ka;
-        const uint32_t k2 = bitrev((uint32_t)t, f.k2);
-        const uint32_t pk2 = (N2 - k2 - (k1 != 0 ? 1u : 0u)) & (N2 - 1);
-        const int pr = (nrow == 1) ? 0 : 1 - r;  // the partner row
-        const double2 F = fsm[r * as + fpad(t)];
-        const double2 G = conj2(fsm[pr * as + fpad(bitrev(pk2, f.k2))]);  // conj(F_-k)
-        const double2 A = make_double2(0.5 * (F.x + G.x), 0.5 * (F.y + G.y));
-        // B = (F - conj F_-k) / 2i
-        const double2 D = csub(F, G);
-        const double2 B = make_double2(0.5 * D.y, -0.5 * D.x);
-        prod[cnt] = cmul(A, B);
-    }
-    __syncthreads();
-    cnt = 0;
-    for (int w = threadIdx.x; w < nrow * N2; w += blockDim.x, ++cnt) {
-        const int r = w / N2, t = w % N2;
-        fsm[r * as + fpad(t)] = prod[cnt];
-    }
-    __syncthreads();
-    fft_stages<true>(fsm, as, nrow, f.k2, f.tw);
-    for (int w = threadIdx.x; w < nrow * N2; w += blockDim.x) {
-        const int r = w / N2, i2 = w % N2;
-        const uint32_t k1 = r ? kb : ka;
-        const double2 rt = root(f.tw, (i2 * k1) & ((1u << f.k) - 1), f.k);
-        rowp[r][i2] = cmul(fsm[r * as + fpad(i2)], rt);
-    }
-}
-
-// inverse column pass, scaling, rounding; grid N2/C
-template <int C>
-__global__ void __launch_bounds__(256) k_fft_inv_cols(const FftArgs* __restrict__ fa) {
-    const FftArgs f = *fa;
-    extern __shared__ double2 fsm[];
-    __shared__ double s_max[8];
+// they coincide); grid N1/2 + 1, N2 threads (2^M = N2)
+template <int M>
+__global__ void __launch_bounds__(M < 5 ? 32 : 1 << M) k_fft_rows(FftArgs f) {
+    constexpr int N2 = 1 << M, H = N2 / 2, Q = N2 / 4;
+    __shared__ double2 s[2][N2];
     const int N1 = 1 << f.k1;
-    const uint32_t N2 = 1u << f.k2;
-    const int as = fpad(N1) + 1;
-    const uint32_t c0 = blockIdx.x * C;
-    for (int w = threadIdx.x; w < C * N1; w += blockDim.x) {
-        const int col = w % C, s = w / C;
-        fsm[col * as + fpad(s)] = f.work[(uint64_t)s * N2 + c0 + col];
-    }
-    __syncthreads();
-    // block 0 alone reads the first element; the carry kernel's counter
-    // lives there and starts at 0
-    if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long*>(f.work) = 0ull;
-    fft_stages<true>(fsm, as, C, f.k1, f.tw);
-    const double inv_n = 1.0 / (double)(1u << f.k);
-    double dmax = 0.0;
-    for (int w = threadIdx.x; w < C * N1; w += blockDim.x) {
-        const int col = w % C, i1 = w / C;
-        const double v = fsm[col * as + fpad(i1)].x * inv_n;
-        const double r = rint(v);
-        double d = fabs(v - r);
-        if (!isfinite(v)) d = INFINITY;
-        dmax = fmax(dmax, d);
-        f.coef[(uint64_t)i1 * N2 + c0 + col] = (long long)r;
-    }
-    for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
-    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = dmax;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int i = 1; i < (int)(blockDim.x >> 5); ++i) dmax = fmax(dmax, s_max[i]);
-        // non-negative doubles order like their bit patterns
-        atomicMax(reinterpret_cast<unsigned long long*>(f.maxdist), (unsigned long long)__double_as_longlong(dmax));
-    }
-}
-
-// signed carry: one CTA of 1024 threads, limbs of the product from the
-// rounded coefficients c_i (value sum c_i 2^(b i)).  A limb's sum
-// S_m = sum of c_i 2^(b i - 64 m) over the coefficients starting in it is a
-// signed 128-bit value; v_m = lo64(S_m) + hi(S_{m-1}) = u_m + g_m 2^64 with
-// g_m in {-1, 0, 1}, and the carry chain c_{m+1} = g_m + floor((u_m + c_m)
-// / 2^64) stays in {-1, 0, 1}.  Each thread composes the chain of its limbs
-// into a map {-1,0,1} -> {-1,0,1}; the block scans the maps.
-typedef __int128 i128;
-
-__device__ __forceinline__ i128 limb_sum_s(const long long* __restrict__ c, uint64_t ncoef, int b, int64_t m) {
-    if (m < 0) return 0;
-    const uint64_t lo_bit = (uint64_t)m * 64;
-    uint64_t i = (lo_bit + b - 1) / b;
-    i128 s = 0;
-    for (; i < ncoef && (uint64_t)b * i < lo_bit + 64; ++i)
-        s += (i128)((unsigned __int128)(i128)c[i] << ((uint64_t)b * i - lo_bit));  // two's complement shift
-    return s;
-}
-
-__device__ __forceinline__ int chain_step(uint64_t u, int g, int cin, uint64_t* out_limb) {
-    const uint64_t r = u + (uint64_t)(int64_t)cin;
-    if (out_limb) *out_limb = r;
-    int fl = 0;
-    if (cin < 0 && u == 0) fl = -1;
-    if (cin > 0 && u == ~0ull) fl = 1;
-    return g + fl;
-}
-
-// Carry maps {-1,0,1} -> {-1,0,1} packed as three 2-bit fields (value + 1).
-constexpr uint32_t kMapIdentity = 0u | (1u << 2) | (2u << 4);
-__device__ __forceinline__ int map_apply(uint32_t m, int x) { return (int)((m >> (2 * (x + 1))) & 3u) - 1; }
-// g after f
-__device__ __forceinline__ uint32_t map_compose(uint32_t g, uint32_t f) {
-    uint32_t r = 0;
+    const uint32_t ka = blockIdx.x, kb = (N1 - blockIdx.x) & (N1 - 1);
+    const bool one = ka == kb;
+    const uint32_t sl[2] = {bitrev(ka, f.k1), bitrev(kb, f.k1)};
+    const int r = threadIdx.x / H & 1, j = threadIdx.x % H;
+    const bool on = threadIdx.x < N2 && !(one && r);
+    const uint32_t slot = r ? sl[1] : sl[0];
+    double2 w[M];
 #pragma unroll
-    for (int x = -1; x <= 1; ++x) r |= (uint32_t)(map_apply(g, map_apply(f, x)) + 1) << (2 * (x + 1));
-    return r;
+    for (int l = 0; l < M; ++l) w[l] = __ldg(&f.twr[(slot << l) + (j >> (M - 1 - l))]);
+    const uint32_t k1 = r ? kb : ka;
+    // fold twiddle i e^(2 pi i k / N) of this thread's frequency pair k, k + N/2
+    const double2 e = __ldg(&f.tw[(k1 + ((uint32_t)bitrev(j, M - 1) << f.k1)) << (kFftMaxLog2 - f.k)]);
+    pdl_enter();
+    const double2* __restrict__ src = after_entry(f.work) + (uint64_t)slot * N2;
+    double2 x, y;
+    if (on) {
+        x = src[j];
+        y = src[j + H];
+    }
+    int pos = j;
+#pragma unroll
+    for (int l = 0; l < M; ++l) {
+        const int h = H >> l;
+        if (l) {
+            __syncthreads();
+            pos = (j / h) * 2 * h + j % h;
+            if (on) {
+                x = s[r][pos];
+                y = s[r][pos + h];
+            }
+            __syncthreads();
+        }
+        if (on) {
+            butterfly(x, y, w[l]);
+            s[r][pos] = x;
+            s[r][pos + h] = y;
+        }
+    }
+    __syncthreads();
+    // product and fold: slots 2j, 2j + 1 hold k and k + N/2; the partner of
+    // slot t (frequency -k) is slot N2-1-t of the other row, in row 0 the
+    // slot of the negated index
+    double2 z;
+    if (on) {
+        const int pr = one ? 0 : 1 - r;
+        int p0 = N2 - 1 - 2 * j, p1 = p0 - 1;
+        if (k1 == 0) {
+            p0 = bitrev((N2 - bitrev(2 * j, M)) & (N2 - 1), M);
+            p1 = bitrev((N2 - bitrev(2 * j + 1, M)) & (N2 - 1), M);
+        }
+        const double2 F0 = s[r][2 * j], F1 = s[r][2 * j + 1], G0 = s[pr][p0], G1 = s[pr][p1];
+        // 4 P = (2 m, t)
+        const double m0 = fma(F0.x, F0.y, G0.x * G0.y);
+        const double t0 = fma(F0.y, F0.y, fma(-F0.x, F0.x, fma(-G0.y, G0.y, G0.x * G0.x)));
+        const double m1 = fma(F1.x, F1.y, G1.x * G1.y);
+        const double t1 = fma(F1.y, F1.y, fma(-F1.x, F1.x, fma(-G1.y, G1.y, G1.x * G1.x)));
+        const double a1 = m0 + m1, a2 = m0 - m1, b1 = t0 + t1, b2 = t0 - t1;
+        // 8 Z = (2 a1 + i b1) + u (2 a2 + i b2), u = i e
+        const double ur = -e.y, ui = e.x;
+        z = make_double2(fma(2.0, a1, fma(2.0 * ur, a2, -ui * b2)), fma(ur, b2, fma(2.0 * ui, a2, b1)));
+    }
+    __syncthreads();
+    // inverse levels over N2/2 points in bit-reversed order; real and
+    // imaginary parts by different threads (four busy warps at N2 = 128)
+    double* sd = reinterpret_cast<double*>(&s[0][0]);
+    auto at = [&](int row, int part, int i) -> double& { return sd[(row * 2 + part) * H + i]; };
+    if (on) {
+        at(r, 0, j) = z.x;
+        at(r, 1, j) = z.y;
+    }
+    const int part = threadIdx.x / H & 1;
+    const int ir = (threadIdx.x % H) / Q, ij = threadIdx.x % Q;
+    const bool ion = threadIdx.x < N2 && !(one && ir);
+#pragma unroll
+    for (int b = 0; b < M - 1; ++b) {
+        const int h = 1 << b;
+        const int p = (ij >> b) * 2 * h + (ij & (h - 1));
+        double2 wt = make_double2(1.0, 0.0);
+        if (b) wt = __ldg(&f.tw[(uint32_t)(ij & (h - 1)) << (kFftMaxLog2 - 1 - b)]);
+        __syncthreads();
+        double o0 = 0.0, o1 = 0.0;
+        if (ion) {
+            const double xs = at(ir, part, p), ys = at(ir, part, p + h);
+            if (b == 0) {
+                o0 = xs + ys;
+                o1 = xs - ys;
+            } else {
+                const double yo = at(ir, 1 - part, p + h);
+                o0 = fma(wt.x, ys, fma(part ? wt.y : -wt.y, yo, xs));
+                o1 = fma(-wt.x, ys, fma(part ? -wt.y : wt.y, yo, xs));
+            }
+        }
+        __syncthreads();
+        if (ion) {
+            at(ir, part, p) = o0;
+            at(ir, part, p + h) = o1;
+        }
+    }
+    __syncthreads();
+    if (on) f.work[(uint64_t)slot * N2 + j] = make_double2(at(r, 0, j), at(r, 1, j));
 }
 
-#ifndef PREC_FFT_CARRY_THREADS
-#define PREC_FFT_CARRY_THREADS 256
-#endif
-#ifndef PREC_FFT_CARRY_LIMBS
-#define PREC_FFT_CARRY_LIMBS 2
-#endif
-constexpr int kFftCarryThreads = PREC_FFT_CARRY_THREADS;
-constexpr int kFftCarryLimbs = PREC_FFT_CARRY_LIMBS;  // limbs per thread
-constexpr int kFftCarryBlockLimbs = kFftCarryThreads * kFftCarryLimbs;
+// 1.5 * 2^52: adding it rounds |v| < 2^51 to the nearest integer (ties to
+// even, as rint) and leaves that integer in the low bits
+__device__ __forceinline__ double round_magic() { return 6755399441055744.0; }
 
-// Phase 1 (every block): the block's limbs from the signed coefficient sums,
-// the carry chain inside the block resolved with a block carry-in of 0
-// (maps composed by warp shuffles and a block scan), limbs written -- below
-// La+Lb to the output, above it to scratch -- and the block's composed map
-// published.  Phase 2 (the last block to finish, fence + atomic counter):
-// loads the block maps into shared memory (one load per thread, all in
-// flight at once), composes them in order, adds each nonzero block carry-in
-// into its block (+1 ripples through all-ones limbs, -1 through zero limbs;
-// rare), and checks that every limb past La+Lb and the final carry are zero.
-// scratch (the transform buffer, free by now): [0] counter, [1 .. nblk]
-// block maps, then the limbs from La+Lb up.
-__global__ void __launch_bounds__(kFftCarryThreads) k_fft_carry(const FftArgs* __restrict__ fa) {
-    const FftArgs f = *fa;
-    __shared__ uint32_t s_wmap[kFftCarryThreads / 32];
-    __shared__ uint32_t s_bmap[kFftCarryThreads];
-    __shared__ uint32_t s_last;
+// inverse columns (half length: N2/2 columns of N1 points), scaling,
+// rounding; grid N2 / 2 / C
+template <int M>
+__global__ void __launch_bounds__(ColGeom<M>::THREADS) k_fft_inv_cols(FftArgs f) {
+    using G = ColGeom<M>;
+    constexpr int H = G::HALF, N1 = 2 * H;
+    __shared__ double2 s[G::C][N1];
+    __shared__ unsigned long long s_max[G::THREADS / 32];
+    const int col = threadIdx.x / H, j = threadIdx.x % H;
+    const uint32_t N2 = 1u << f.k2, N2h = N2 / 2;
+    const uint32_t c = blockIdx.x * G::C + col;
+    const bool on = c < N2h;  // (N = 64 has fewer columns than one CTA takes)
+    double2 w[M];
+#pragma unroll
+    for (int b = 0; b < M; ++b)
+        w[b] = __ldg(&f.tw[((uint32_t)(j & ((1 << b) - 1)) * N2h + (on ? c : 0)) << (kFftMaxLog2 - f.k2 - b)]);
+    pdl_enter();
+    const double2* __restrict__ src = after_entry(f.work);
+    double2 x = make_double2(0.0, 0.0), y = x;
+    if (on) {
+        x = src[(uint64_t)(2 * j) * N2 + c];
+        y = src[(uint64_t)(2 * j + 1) * N2 + c];
+    }
+    int pos = 2 * j;
+#pragma unroll
+    for (int b = 0; b < M; ++b) {
+        const int h = 1 << b;
+        if (b) {
+            s[col][pos] = x;
+            s[col][pos + (h >> 1)] = y;
+            __syncthreads();
+            pos = (j >> b) * 2 * h + (j & (h - 1));
+            x = s[col][pos];
+            y = s[col][pos + h];
+            if (b + 1 < M) __syncthreads();
+        }
+        butterfly(x, y, w[b]);
+    }
+    // element i1 = pos, pos + H of column c: coefficients 2n, 2n + 1 of n = i1 N2/2 + c
+    const double scale = __hiloint2double((1023 - f.k - 2) << 20, 0);  // 2^-(k+2)
+    const double magic = round_magic();
+    unsigned long long dmax = 0;
+    auto round1 = [&](double v) -> long long {
+        const double m = fma(v, scale, magic);
+        const double r = m - magic;
+        const double d = fma(v, scale, -r);
+        // |d| by its bits (non-negative doubles order like them; NaN above
+        // all); a value past 2^51 cannot be rounded this way: refused
+        unsigned long long bits = (unsigned long long)__double_as_longlong(d) & 0x7fffffffffffffffull;
+        const unsigned long long big = (unsigned long long)__double_as_longlong(r) & 0x7fffffffffffffffull;
+        if (big >= 0x4320000000000000ull) bits = 0x7ff0000000000000ull;
+        dmax = bits > dmax ? bits : dmax;
+        return __double_as_longlong(m) - __double_as_longlong(magic);
+    };
+    longlong2* coef = reinterpret_cast<longlong2*>(f.coef);
+    const long long x0 = round1(x.x), x1 = round1(x.y), y0 = round1(y.x), y1 = round1(y.y);
+    if (on) {
+        coef[(uint64_t)pos * N2h + c] = make_longlong2(x0, x1);
+        coef[(uint64_t)(pos + H) * N2h + c] = make_longlong2(y0, y1);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long v = __shfl_xor_sync(0xffffffffu, dmax, o);
+        dmax = v > dmax ? v : dmax;
+    }
+    if (G::THREADS > 32) {
+        if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = dmax;
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int i = 1; i < G::THREADS / 32; ++i) dmax = s_max[i] > dmax ? s_max[i] : dmax;
+    }
+    if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned long long*>(f.maxdist), dmax);
+}
+
+// Carry: limbs of the product sum c_i 2^(bi) from the signed coefficients.
+// c_i + 2^62 - 2^(62-b) (for i = 0: c_i + 2^62) is positive and adds up to the
+// same number plus 2^(bN + 62 - b), past every limb of the product, so the
+// carries are 0 or 1: S_m, the sum of the coefficients that start in limb m,
+// gives limb lo64(S_m) + hi64(S_m-1) + carry, as in the NTT band.  The
+// product runs as one cluster of up to 8 CTAs: each puts its carry aggregate
+// into every CTA's shared memory, one cluster barrier, and every limb is
+// written once, final.  (As separate CTAs joined by the last one over the
+// carry maps of signed limbs this kernel took 9 - 11 us.)
+constexpr int kFftCarryThreads = 512;
+constexpr int kFftCarryCluster = 8;
+
+template <int L>
+__global__ void __launch_bounds__(kFftCarryThreads) k_fft_carry(FftArgs f) {
+    namespace cg = cooperative_groups;
+    __shared__ uint32_t s_wg[kFftCarryThreads / 32], s_wp[kFftCarryThreads / 32];
+    __shared__ uint32_t s_blk[kFftCarryCluster];
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t rank = blockIdx.x, ranks = gridDim.x;
+    cluster.barrier_arrive();  // (the other CTAs' shared memory exists once all arrived)
+    pdl_enter();
+    const long long* __restrict__ coef = after_entry(f.coef);
     const double dist = *f.maxdist;
-    if (f.host_dist && blockIdx.x == 0 && threadIdx.x == 0) *f.host_dist = dist;
+    if (f.host_dist && rank == 0 && threadIdx.x == 0) *f.host_dist = dist;
     if (!(dist <= 0.25)) {  // also NaN / inf: nothing is written
-        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(f.err, kDevErrFftRound);
+        if (rank == 0 && threadIdx.x == 0) atomicOr(f.err, kDevErrFftRound);
+        cluster.barrier_wait();
         return;
     }
-    // Balanced digits can place signed contributions past the product's
-    // La+Lb limbs (they cancel a borrow that runs up to them), so the chain
-    // covers every limb a coefficient reaches; those limbs must end as 0.
-    const int64_t Lout = (int64_t)f.lout;
-    const int64_t Lcoef = (int64_t)(((uint64_t)f.b * f.ncoef + 63) / 64) + 2;
-    const int64_t L = Lcoef > Lout ? Lcoef : Lout;
-    const int nblk = (int)((L + kFftCarryBlockLimbs - 1) / kFftCarryBlockLimbs);
-    uint64_t* scr = reinterpret_cast<uint64_t*>(f.work);
-    uint32_t* counter = reinterpret_cast<uint32_t*>(scr);
-    uint64_t* bmap = scr + 1;
-    uint64_t* high = scr + 1 + nblk;  // limbs Lout .. L-1
-    auto limb_ref = [&](int64_t m) -> uint64_t& { return m < Lout ? f.out[m] : high[m - Lout]; };
-
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // a graph launch uses the largest grid of the transform length: blocks
-    // past this product's limbs only take part in the count below
-    const bool idle = (int)blockIdx.x >= nblk;
-    const int64_t m0 = (int64_t)blockIdx.x * kFftCarryBlockLimbs + (int64_t)threadIdx.x * kFftCarryLimbs;
-    uint64_t u[kFftCarryLimbs];
-    int g[kFftCarryLimbs];
-    if (!idle) {
-        i128 prev = limb_sum_s(f.coef, f.ncoef, f.b, m0 - 1);
+    const int b = f.b;
+    const int64_t m0 = ((int64_t)rank * kFftCarryThreads + threadIdx.x) * L;
+    // one limb past the product, checked to be zero, where the coefficients cover it
+    const int64_t lim = (int64_t)f.lout + ((uint64_t)b * f.ncoef >= 64 * (f.lout + 1) ? 1 : 0);
+    u128 T[L + 1];  // S of limbs m0 - 1 .. m0 + L - 1
 #pragma unroll
-        for (int k = 0; k < kFftCarryLimbs; ++k) {
-            const i128 cur = m0 + k < L ? limb_sum_s(f.coef, f.ncoef, f.b, m0 + k) : (i128)0;
-            const i128 v = (i128)(uint64_t)cur + (prev >> 64);
-            u[k] = (uint64_t)v;
-            g[k] = (int)(v >> 64);
-            prev = cur;
-        }
-    }
-    // this thread's chain as a map of its carry-in
-    uint32_t tmap = 0;
+    for (int k = 0; k <= L; ++k) {
+        const int64_t m = m0 + k - 1;
+        T[k] = 0;
+        if (m < 0 || m >= lim) continue;
+        const uint32_t bit = (uint32_t)m * 64;
+        const uint32_t i0 = (bit + b - 1) / b;
+        const uint32_t off = i0 * b - bit;
+        long long c[8];
 #pragma unroll
-    for (int x = -1; x <= 1; ++x) {
-        int c = x;
+        for (int u = 0; u < 8; ++u) c[u] = off + u * b < 64 && i0 + u < f.ncoef ? coef[i0 + u] : 0;
 #pragma unroll
-        for (int k = 0; k < kFftCarryLimbs; ++k)
-            if (m0 + k < L) c = chain_step(u[k], g[k], c, nullptr);
-        tmap |= (uint32_t)((c < -1 ? -1 : (c > 1 ? 1 : c)) + 1) << (2 * (x + 1));
-    }
-    // inclusive scan of the maps over the warp, then over the warps
-    uint32_t inc = tmap;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t o = __shfl_up_sync(0xffffffffu, inc, d);
-        if (lane >= d) inc = map_compose(inc, o);
-    }
-    if (lane == 31) s_wmap[warp] = inc;
-    __syncthreads();
-    uint32_t below = kMapIdentity;  // warps before this one
-    for (int w = 0; w < warp; ++w) below = map_compose(s_wmap[w], below);
-    uint32_t excl = __shfl_up_sync(0xffffffffu, inc, 1);
-    if (lane == 0) excl = kMapIdentity;
-    const int cin = map_apply(map_compose(excl, below), 0);
-    {
-        int c = cin;
-#pragma unroll
-        for (int k = 0; k < kFftCarryLimbs; ++k) {
-            if (m0 + k >= L) break;
-            uint64_t limb;
-            c = chain_step(u[k], g[k], c, &limb);
-            limb_ref(m0 + k) = limb;
-        }
-    }
-    if (threadIdx.x == 0 && !idle) {
-        uint32_t bm = kMapIdentity;
-        for (int w = 0; w < kFftCarryThreads / 32; ++w) bm = map_compose(s_wmap[w], bm);
-        bmap[blockIdx.x] = bm;
-    }
-    // ---- phase 2: the last block resolves the carries between blocks
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        s_last = atomicAdd(counter, 1u) == (uint32_t)gridDim.x - 1 ? 1u : 0u;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    // (one L2 round trip per block map, in the serial loop below, made this
-    // kernel 14 us long at 3000 x 3000 limbs)
-    const bool staged = nblk <= kFftCarryThreads;
-    if (staged && (int)threadIdx.x < nblk) s_bmap[threadIdx.x] = (uint32_t)__ldcg(&bmap[threadIdx.x]);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int c = 0;
-        for (int bk = 0; bk < nblk; ++bk) {
-            if (c != 0) {
-                const int64_t e = (int64_t)(bk + 1) * kFftCarryBlockLimbs < L ? (int64_t)(bk + 1) * kFftCarryBlockLimbs : L;
-                for (int64_t m = (int64_t)bk * kFftCarryBlockLimbs; m < e; ++m) {
-                    uint64_t& x = limb_ref(m);
-                    const uint64_t old = __ldcg(&x);
-                    x = old + (uint64_t)(int64_t)c;
-                    if (c > 0 ? old != ~0ull : old != 0) break;
-                }
+        for (int u = 0; u < 8; ++u) {
+            if (off + u * b < 64 && i0 + u < f.ncoef) {
+                const uint64_t v = (uint64_t)c[u] + (1ull << 62) - (i0 + u ? 1ull << (62 - b) : 0);
+                T[k] += (u128)v << (off + u * b);
             }
-            c = map_apply(staged ? s_bmap[bk] : (uint32_t)__ldcg(&bmap[bk]), c);
         }
-        if (c != 0) atomicOr(f.err, kDevErrCarry);
+    }
+    u128 S[L];
+#pragma unroll
+    for (int k = 0; k < L; ++k) S[k] = T[k + 1];
+    uint64_t v[L];
+    uint32_t gbits;
+    bool G, P;
+    limbs_from_sums<L>(S, (uint64_t)(T[0] >> 64), v, gbits, G, P);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t gm = __ballot_sync(0xffffffffu, G), pm = __ballot_sync(0xffffffffu, P);
+    if (lane == 0) {
+        s_wg[warp] = (uint32_t)(carry_chain(gm, pm, false) >> 32) & 1;
+        s_wp[warp] = pm == 0xffffffffu;
     }
     __syncthreads();
-    // a product fits La+Lb limbs: everything above must be zero
-    for (int64_t m = Lout + threadIdx.x; m < L; m += blockDim.x)
-        if (__ldcg(&high[m - Lout]) != 0) atomicOr(f.err, kDevErrCarry);
+    // warp aggregates as bits; the CTA's own aggregate to every CTA of the cluster
+    constexpr int NW = kFftCarryThreads / 32;
+    const uint32_t bg = __ballot_sync(0xffffffffu, lane < NW && s_wg[lane & (NW - 1)] != 0);
+    const uint32_t bp = __ballot_sync(0xffffffffu, lane < NW && s_wp[lane & (NW - 1)] != 0);
+    cluster.barrier_wait();
+    if (ranks > 1) {
+        if (warp == 0 && lane < (int)ranks) {
+            const uint32_t agg = ((uint32_t)(carry_chain(bg, bp, false) >> NW) & 1) | (bp == (1u << NW) - 1 ? 2u : 0u);
+            *cluster.map_shared_rank(&s_blk[rank], lane) = agg;
+        }
+        cluster.sync();
+    }
+    bool cin = false;
+    for (uint32_t r = 0; r < rank; ++r) cin = (s_blk[r] & 1) || ((s_blk[r] & 2) && cin);
+    const bool wcin = (carry_chain(bg, bp, cin) >> warp) & 1;
+    bool c = (carry_chain(gm, pm, wcin) >> lane) & 1;
+#pragma unroll
+    for (int k = 0; k < L; ++k) {
+        const uint64_t x = v[k] + (c ? 1u : 0u);
+        c = ((gbits >> k) & 1) || (v[k] == ~0ull && c);
+        const int64_t m = m0 + k;
+        if (m < (int64_t)f.lout) f.out[m] = x;
+        else if (m < lim && x != 0) atomicOr(f.err, kDevErrCarry);  // a product fits La+Lb limbs
+    }
 }
 
-__global__ void __launch_bounds__(256) k_stage(ulonglong2* dst, const ulonglong2* __restrict__ src, uint64_t n2) {
-    pdl_enter();
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n2) dst[i] = src[i];
-}
-
-void launch_stage(uint64_t* dst, const uint64_t* src, uint64_t n, cudaStream_t st) {
-    const uint64_t n2 = (n + 1) / 2;
-    launch_pdl(false, k_stage, (unsigned)((n2 + 255) / 256), 256, 0, st, reinterpret_cast<ulonglong2*>(dst),
-               reinterpret_cast<const ulonglong2*>(src), n2);
-    count_launches(1);
-}
-
-// e^(2 pi i e / 2^16) for e < 2^15
+// e^(2 pi i e / 2^16) for e < 2^15, then e^(-pi i 0.b0b1..) for q = ..b1b0 < 2^15
 __global__ void k_fft_table(double2* tw) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e < (1 << (kFftMaxLog2 - 1))) {
         double s, c;
         sincospi((double)e / (double)(1 << (kFftMaxLog2 - 1)), &s, &c);
         tw[e] = make_double2(c, s);
+        const int q = (int)bitrev((uint32_t)e, kFftMaxLog2 - 1);
+        sincospi((double)e / (double)(1 << (kFftMaxLog2 - 1)), &s, &c);
+        tw[(1 << (kFftMaxLog2 - 1)) + q] = make_double2(c, -s);
     }
 }
 
 // ---------------------------------------------------------------------------
 
-#ifndef PREC_FFT_COLS
-#define PREC_FFT_COLS 1
-#endif
-constexpr int kFftCols = PREC_FFT_COLS;  // columns per column-pass CTA
-
-size_t fft_table_bytes() { return (size_t)sizeof(double2) << (kFftMaxLog2 - 1); }
+size_t fft_table_bytes() { return (size_t)sizeof(double2) << kFftMaxLog2; }
 
 void fft_build_table(double2* tw, cudaStream_t st) {
     k_fft_table<<<(1 << (kFftMaxLog2 - 1)) / 256, 256, 0, st>>>(tw);
     count_launches(1);
 }
 
-static size_t cols_smem(int k1) { return (size_t)kFftCols * (fpad_host(1 << k1) + 1) * sizeof(double2); }
-static size_t rows_smem(int k2) { return (size_t)2 * (fpad_host(1 << k2) + 1) * sizeof(double2); }
-
-int fft_configure_kernels() {
-    cudaError_t e = cudaFuncSetAttribute(k_fft_fwd_cols<kFftCols>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)cols_smem(kFftMaxLog2 - kFftMaxLog2 / 2));
-    if (!e) e = cudaFuncSetAttribute(k_fft_inv_cols<kFftCols>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)cols_smem(kFftMaxLog2 - kFftMaxLog2 / 2));
-    if (!e) e = cudaFuncSetAttribute(k_fft_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)rows_smem(kFftMaxLog2 - kFftMaxLog2 / 2));
-    return (int)e;
+template <int L>
+static void launch_carry(const FftArgs& f, cudaStream_t st) {
+    const uint64_t per = (uint64_t)kFftCarryThreads * L;
+    uint64_t n = (f.lout + 1 + per - 1) / per;
+    if (n > kFftCarryCluster) n = kFftCarryCluster;
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)n;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = (unsigned)n;
+    cfg.blockDim = kFftCarryThreads;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    cudaLaunchKernelEx(&cfg, k_fft_carry<L>, f);
 }
 
-static int carry_blocks(uint64_t b, uint64_t ncoef, uint64_t lout) {
-    const int64_t lcoef = (int64_t)((b * ncoef + 63) / 64) + 2;
-    const int64_t L = lcoef > (int64_t)lout ? lcoef : (int64_t)lout;
-    return (int)((L + kFftCarryBlockLimbs - 1) / kFftCarryBlockLimbs);
-}
+#define PREC_FFT_LOG2(X) X(3) X(4) X(5) X(6) X(7) X(8)
 
-// The first kernel takes the product's arguments by value (launch
-// parameters: no copy in the stream) and stores them at d_args, where the
-// other three read them.
-static void launch4(const FftArgs& f, FftArgs* d_args, int nblk, cudaStream_t st, cudaEvent_t* ev) {
-    if (ev) cudaEventRecord(ev[0], st);
-    const int ncol = (1 << f.k2) / kFftCols;
-    launch_kernel(k_fft_fwd_cols<kFftCols>, ncol, 256, cols_smem(f.k1), st, f, d_args);
-    if (ev) cudaEventRecord(ev[1], st);
-    launch_kernel(k_fft_rows, (1 << f.k1) / 2 + 1, 256, rows_smem(f.k2), st, d_args);
-    if (ev) cudaEventRecord(ev[2], st);
-    launch_kernel(k_fft_inv_cols<kFftCols>, ncol, 256, cols_smem(f.k1), st, d_args);
-    if (ev) cudaEventRecord(ev[3], st);
-    launch_kernel(k_fft_carry, nblk, kFftCarryThreads, 0, st, d_args);
-    count_launches(4);
-    if (ev) cudaEventRecord(ev[4], st);
-}
-
-// One graph per (column, row) length and argument buffer (each library
-// lane has its own), its carry grid the length's largest (16-bit digits;
-// the extra blocks idle).  A replay sets the first node's parameters to
-// the product's arguments.  (An upload of the arguments by a copy in the
-// stream measured 8 us slower per product when the caller's operands were
-// page-locked.)  The map is shared by the lanes (g_fft_mu); a graph is
-// only replayed by its own lane, one product at a time.
-struct FftGraph {
-    cudaGraphExec_t exec = nullptr;
-    cudaGraphNode_t first = nullptr;  // k_fft_fwd_cols
-    cudaKernelNodeParams params{};
-    cudaGraph_t graph = nullptr;  // kept: a node's parameters are set through its graph's node handle
-};
-typedef std::tuple<int, int, const FftArgs*> FftGraphKey;
-static std::map<FftGraphKey, FftGraph> g_fft_graphs;
-static std::mutex g_fft_mu;
-
-void fft_release_graphs(const FftArgs* d_args) {
-    std::lock_guard<std::mutex> lk(g_fft_mu);
-    for (auto it = g_fft_graphs.begin(); it != g_fft_graphs.end();) {
-        if (d_args && std::get<2>(it->first) != d_args) {
-            ++it;
-            continue;
-        }
-        cudaGraphExecDestroy(it->second.exec);
-        cudaGraphDestroy(it->second.graph);
-        it = g_fft_graphs.erase(it);
-    }
-}
-
-int fft_launch(const FftArgs& f, FftArgs* d_args, cudaStream_t st, cudaEvent_t* ev, cudaStream_t cap) {
-    cudaError_t e;
-    if (ev || !cap) {
-        launch4(f, d_args, carry_blocks(f.b, f.ncoef, f.lout), st, ev);
-        return (int)cudaGetLastError();
-    }
-    const FftGraphKey key(f.k1, f.k2, d_args);
-    std::map<FftGraphKey, FftGraph>::iterator it;
-    {
-        std::lock_guard<std::mutex> lk(g_fft_mu);
-        it = g_fft_graphs.find(key);
-    }
-    if (it == g_fft_graphs.end()) {
-        // the four launches as a chain of kernel nodes (explicit
-        // construction: no stream capture)
-        GraphRecorder rec;
-        if ((e = cudaGraphCreate(&rec.graph, 0)) != cudaSuccess) return (int)e;
-        const uint64_t before = launches_this_thread();
-        thread_recorder() = &rec;
-        launch4(f, d_args, carry_blocks(16, 1ull << (f.k1 + f.k2), 0), cap, nullptr);
-        thread_recorder() = nullptr;
-        uncount_launches(launches_this_thread() - before);  // recorded: counted at every replay
-        cudaGraph_t g = rec.graph;
-        e = rec.err;
-        FftGraph fg;
-        // the forward column node: the first recorded
-        fg.first = rec.first;
-        if (e == cudaSuccess && fg.first) e = cudaGraphKernelNodeGetParams(fg.first, &fg.params);
-        if (e == cudaSuccess && !fg.first) e = cudaErrorInvalidValue;
-        if (e == cudaSuccess) e = cudaGraphInstantiate(&fg.exec, g, 0);
-        if (e != cudaSuccess) {
-            if (g) cudaGraphDestroy(g);
-            return (int)e;
-        }
-        fg.graph = g;
-        std::lock_guard<std::mutex> lk(g_fft_mu);
-        it = g_fft_graphs.emplace(key, fg).first;
-    }
-    FftGraph& fg = it->second;
-    FftArgs* pub = d_args;
-    void* params[2] = {const_cast<FftArgs*>(&f), &pub};
-    cudaKernelNodeParams kp = fg.params;
-    kp.kernelParams = params;
-    kp.extra = nullptr;
-    if ((e = cudaGraphExecKernelNodeSetParams(fg.exec, fg.first, &kp)) != cudaSuccess) return (int)e;
-    e = cudaGraphLaunch(fg.exec, st);
-    if (e == cudaSuccess) count_launches(4);
-    return (int)e;
+int fft_launch(const FftArgs& f, cudaStream_t st) {
+    const uint64_t nd = f.da > f.db ? f.da : f.db;
+    launch_pdl(false, k_fft_digits, (unsigned)((nd + kDigitThreads - 1) / kDigitThreads), kDigitThreads, 0, st, f);
+#define X(M) \
+    if (f.k1 == M) launch_pdl(false, k_fft_fwd_cols<M>, (1u << f.k2) / ColGeom<M>::C, ColGeom<M>::THREADS, 0, st, f);
+    PREC_FFT_LOG2(X)
+#undef X
+#define X(M) \
+    if (f.k2 == M) launch_pdl(false, k_fft_rows<M>, (1u << f.k1) / 2 + 1, M < 5 ? 32 : 1 << M, 0, st, f);
+    PREC_FFT_LOG2(X)
+#undef X
+#define X(M) \
+    if (f.k1 == M) launch_pdl(false, k_fft_inv_cols<M>, ((1u << f.k2) / 2 + ColGeom<M>::C - 1) / ColGeom<M>::C, ColGeom<M>::THREADS, 0, st, f);
+    PREC_FFT_LOG2(X)
+#undef X
+    // limbs per thread: 8 CTAs of 512 threads cover 4096 limbs of one each
+    const uint64_t one = (uint64_t)kFftCarryThreads * kFftCarryCluster;
+    if (f.lout <= one) launch_carry<1>(f, st);
+    else if (f.lout <= 2 * one) launch_carry<2>(f, st);
+    else launch_carry<3>(f, st);
+    count_launches(5);
+    return (int)cudaGetLastError();
 }
 
 }  // namespace precgpu

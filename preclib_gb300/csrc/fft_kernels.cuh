@@ -13,7 +13,7 @@ constexpr int kFftMaxLog2 = 16;     // largest FP64 transform (6144 x 6144 limbs
 constexpr int kDevErrFftRound = 4;  // device error bit: max distance above 0.25
 
 struct FftArgs {
-    const uint64_t* a;
+    const uint64_t* a;    // operands and result: device or page-locked host memory
     const uint64_t* bp;
     uint64_t* out;
     double2* work;        // N complex values
@@ -22,6 +22,7 @@ struct FftArgs {
     double* host_dist;    // page-locked copy of it for the host, or nullptr
     int* err;
     const double2* tw;    // e^(2 pi i e / 2^16), e < 2^15
+    const double2* twr;   // e^(-pi i 0.b0b1..), q = ..b1b0 < 2^15
     uint64_t la, lb, lout;
     uint64_t da, db;      // balanced digit counts
     uint64_t ncoef;       // N
@@ -29,24 +30,10 @@ struct FftArgs {
     int k, k1, k2;        // log2 N = k1 + k2 (column length 2^k1, row length 2^k2)
 };
 
-constexpr int fpad_host(int i) { return i + (i >> 4); }
-
-// dst[0 .. n) = src[0 .. n) limbs, both on 16-byte boundaries; src may be
-// page-locked host memory
-void launch_stage(uint64_t* dst, const uint64_t* src, uint64_t n, cudaStream_t st);
-
+// both twiddle tables: tw, then twr at tw + 2^15
 size_t fft_table_bytes();
 void fft_build_table(double2* tw, cudaStream_t st);
-int fft_configure_kernels();
-// The product's 4 kernels: the first takes the arguments by value and
-// stores them at `d_args` (device) for the others; one graph replay
-// (built for `cap` once per length and argument buffer), or, with `ev`
-// (or without `cap`), plain launches with an event before the first and
-// after each.  Returns a cudaError_t.  The caller runs one product at a
-// time per argument buffer (its library lane's lock).
-int fft_launch(const FftArgs& f, FftArgs* d_args, cudaStream_t st, cudaEvent_t* ev = nullptr,
-               cudaStream_t cap = nullptr);
-// destroys the cached graphs of one argument buffer (a lane's), or all
-void fft_release_graphs(const FftArgs* d_args = nullptr);
+// The product's 5 kernels on `st`.  Returns a cudaError_t.
+int fft_launch(const FftArgs& f, cudaStream_t st);
 
 }  // namespace precgpu

@@ -201,7 +201,6 @@ constexpr int kColGroup = PREC_COL_GROUP;      // adjacent columns per column-pa
 struct GraphRecorder {
     cudaGraph_t graph = nullptr;
     std::vector<std::pair<cudaStream_t, cudaGraphNode_t>> last;  // per stream handle
-    cudaGraphNode_t first = nullptr;  // the first node recorded
     cudaError_t err = cudaSuccess;
     uint64_t nodes = 0;
     cudaGraphNode_t tail(cudaStream_t st) const;

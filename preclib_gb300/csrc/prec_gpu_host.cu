@@ -257,7 +257,6 @@ constexpr int kMaxLanes = 16;
 struct Lane {
     std::mutex mu;
     cudaStream_t stream = nullptr;  // host-pointer products
-    cudaStream_t cap = nullptr;     // the stream handle this lane's graph nodes are recorded for
     // host products with a chunked CRT: each chunk's limbs copy out on
     // `copy` while the next chunks run
     cudaStream_t copy = nullptr;
@@ -272,7 +271,6 @@ struct Lane {
     int* h_err = nullptr;     // pinned copy of the status
     double* d_maxdist = nullptr;
     double* h_maxdist = nullptr;
-    FftArgs* fft_args = nullptr;  // the FP64 band product's arguments, read by its kernels
     cudaEvent_t last_done = nullptr, ev0 = nullptr, ev1 = nullptr;
     unsigned long long last_stream = 0;  // id of the stream last_done was recorded on (ids are never reused)
     bool has_last = false;
@@ -349,7 +347,6 @@ void GraphRecorder::add_kernel(const void* func, dim3 grid, dim3 block, size_t s
     cudaGraphNode_t dep = tail(st), node = nullptr;
     err = cudaGraphAddKernelNode(&node, graph, dep ? &dep : nullptr, dep ? 1 : 0, &kp);
     if (err != cudaSuccess) return;
-    if (!first) first = node;
     set_tail(st, node);
     ++nodes;
 }
@@ -366,7 +363,6 @@ void GraphRecorder::add_memset(void* dst, size_t bytes, cudaStream_t st) {
     cudaGraphNode_t dep = tail(st), node = nullptr;
     err = cudaGraphAddMemsetNode(&node, graph, dep ? &dep : nullptr, dep ? 1 : 0, &mp);
     if (err != cudaSuccess) return;
-    if (!first) first = node;
     set_tail(st, node);
     ++nodes;
 }
@@ -495,7 +491,6 @@ static int init_locked(Ctx& c, int device) {
     CK(cudaMemset(c.d_err, 0, kStatBytes));
     CK(cudaMallocHost(&c.h_err, kStatBytes));
     CK((cudaError_t)ntt_configure_kernels());
-    CK((cudaError_t)fft_configure_kernels());
     CK((cudaError_t)configure_direct());
     CK(cudaMalloc(&c.fft_tw, fft_table_bytes()));
     fft_build_table(c.fft_tw, nullptr);
@@ -519,7 +514,6 @@ static void lane_destroy(Lane& L) {
     cudaFree(L.blk);
     cudaFree(L.d_err);
     cudaFreeHost(L.h_err);
-    cudaFree(L.fft_args);
     cudaFree(L.chunk_words);
     cudaFree(L.direct_counter);
     for (cudaEvent_t e : {L.last_done, L.ev0, L.ev1, L.ev_a, L.ev_b, L.copy_done})
@@ -533,14 +527,12 @@ static void lane_destroy(Lane& L) {
         if (L.prime_streams.join[p]) cudaEventDestroy(L.prime_streams.join[p]);
     }
     if (L.prime_streams.fork) cudaEventDestroy(L.prime_streams.fork);
-    for (cudaStream_t s : {L.stream, L.cap, L.copy})
+    for (cudaStream_t s : {L.stream, L.copy})
         if (s) cudaStreamDestroy(s);
-    fft_release_graphs(L.fft_args);
 }
 
 static int lane_create(Lane& L) {
     CK(cudaStreamCreateWithFlags(&L.stream, cudaStreamNonBlocking));
-    CK(cudaStreamCreateWithFlags(&L.cap, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&L.copy, cudaStreamNonBlocking));
     for (int i = 0; i < kCrtMaxChunks; ++i) CK(cudaEventCreateWithFlags(&L.chunk_done[i], cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&L.copy_done, cudaEventDisableTiming));
@@ -563,7 +555,6 @@ static int lane_create(Lane& L) {
     CK(cudaMallocHost(&L.h_err, kStatBytes));
     L.d_maxdist = reinterpret_cast<double*>(reinterpret_cast<char*>(L.d_err) + 8);
     L.h_maxdist = reinterpret_cast<double*>(reinterpret_cast<char*>(L.h_err) + 8);
-    CK(cudaMalloc(&L.fft_args, sizeof(FftArgs)));
     return 0;
 }
 
@@ -872,7 +863,7 @@ static bool fft_plan_for(uint64_t la, uint64_t lb, FftPlan& fp) {
         fp.b = b;
         fp.k = k;
         // the longer half along the columns: twice the row-pair CTAs of the
-        // FP64-bound row kernel for odd k
+        // row kernel, which has the most FP64 work, for odd k
         fp.k1 = (k + 1) / 2;
         fp.k2 = k - fp.k1;
         fp.da = da;
@@ -973,15 +964,9 @@ static int host_mul(const uint64_t* a, size_t an, const uint64_t* b, size_t bn, 
     bool copied = false;  // the result went out chunk by chunk
     nvtxRangePushA("enqueue product");
     if (use_fft) {
-        FftArgs f{};  // pageable: the small upload travels in the command stream
-        if (staged) {  // (every limb is read several times: one trip over the link)
-            launch_stage(L.io, d_a, la_pad + lb, st);
-            f.a = L.io;
-            f.bp = square ? L.io : L.io + la_pad;
-        } else {
-            f.a = d_a;
-            f.bp = d_b;
-        }
+        FftArgs f{};
+        f.a = d_a;
+        f.bp = d_b;
         f.out = d_out;
         f.host_dist = staged ? L.h_maxdist : nullptr;
         f.work = reinterpret_cast<double2*>(L.ws);
@@ -989,6 +974,7 @@ static int host_mul(const uint64_t* a, size_t an, const uint64_t* b, size_t bn, 
         f.maxdist = L.d_maxdist;
         f.err = err;
         f.tw = c.fft_tw;
+        f.twr = c.fft_tw + (1 << (kFftMaxLog2 - 1));
         f.la = la;
         f.lb = lb;
         f.lout = lout;
@@ -999,7 +985,7 @@ static int host_mul(const uint64_t* a, size_t an, const uint64_t* b, size_t bn, 
         f.k = fp.k;
         f.k1 = fp.k1;
         f.k2 = fp.k2;
-        CK((cudaError_t)fft_launch(f, L.fft_args, st, nullptr, L.cap));
+        CK((cudaError_t)fft_launch(f, st));
     } else if (blocked) {
         if ((r = enqueue_blocked(c, L, d_a, la, d_b, lb, d_out, st, B, err))) return r;
     } else {
