@@ -267,9 +267,10 @@ struct Lane {
     uint64_t* pin = nullptr;  // small host products: operands and result in page-locked host memory
     uint64_t* blk = nullptr;  // blocked products: a block pair's product, then the add kernel's scratch
     size_t blk_cap = 0;       // limbs
-    int* d_err = nullptr;     // host products' device status: error bits at +0, FFT max distance at +8
-    int* h_err = nullptr;     // pinned copy of the status
-    double* d_maxdist = nullptr;
+    // host products' status in page-locked memory: error bits at +0, FFT max
+    // distance at +8 (the kernels write both)
+    int* h_err = nullptr;
+    double* d_maxdist = nullptr;  // the FFT distance while its kernels run
     double* h_maxdist = nullptr;
     cudaEvent_t last_done = nullptr, ev0 = nullptr, ev1 = nullptr;
     unsigned long long last_stream = 0;  // id of the stream last_done was recorded on (ids are never reused)
@@ -512,7 +513,7 @@ static void lane_destroy(Lane& L) {
     cudaFree(L.io);
     cudaFreeHost(L.pin);
     cudaFree(L.blk);
-    cudaFree(L.d_err);
+    cudaFree(L.d_maxdist);
     cudaFreeHost(L.h_err);
     cudaFree(L.chunk_words);
     cudaFree(L.direct_counter);
@@ -550,10 +551,8 @@ static int lane_create(Lane& L) {
         CK(cudaEventCreateWithFlags(&L.prime_streams.join[p], cudaEventDisableTiming));
     }
     CK(cudaEventCreateWithFlags(&L.prime_streams.fork, cudaEventDisableTiming));
-    CK(cudaMalloc(&L.d_err, kStatBytes));
-    CK(cudaMemset(L.d_err, 0, kStatBytes));
+    CK(cudaMalloc(&L.d_maxdist, sizeof(double)));
     CK(cudaMallocHost(&L.h_err, kStatBytes));
-    L.d_maxdist = reinterpret_cast<double*>(reinterpret_cast<char*>(L.d_err) + 8);
     L.h_maxdist = reinterpret_cast<double*>(reinterpret_cast<char*>(L.h_err) + 8);
     return 0;
 }
@@ -946,14 +945,15 @@ static int host_mul(const uint64_t* a, size_t an, const uint64_t* b, size_t bn, 
     uint64_t* d_a = buf;
     uint64_t* d_b = square ? d_a : buf + la_pad;
     uint64_t* d_out = buf + la_pad + lb_pad;
-    int* err = staged ? L.h_err : L.d_err;
+    // the kernels set error bits (and the FFT distance) in page-locked memory
+    int* err = L.h_err;
     cudaStream_t st = L.stream;
     NvtxRange range("prec_gpu_mul %zux%zu %s", la, lb, use_fft ? "fft" : (blocked ? "blocked" : "ntt"));
     if ((r = lane_begin(L, st))) return r;
+    *L.h_err = 0;
     if (staged) {
         memcpy(d_a, a, la * sizeof(uint64_t));
         if (!square) memcpy(d_b, b, lb * sizeof(uint64_t));
-        *L.h_err = 0;
     } else {
         CK(cudaMemcpyAsync(d_a, a, la * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
         if (chains) CK(cudaEventRecord(L.ev_a, st));
@@ -968,7 +968,7 @@ static int host_mul(const uint64_t* a, size_t an, const uint64_t* b, size_t bn, 
         f.a = d_a;
         f.bp = d_b;
         f.out = d_out;
-        f.host_dist = staged ? L.h_maxdist : nullptr;
+        f.host_dist = L.h_maxdist;
         f.work = reinterpret_cast<double2*>(L.ws);
         f.coef = reinterpret_cast<long long*>(L.ws + (sizeof(double2) << fp.k));
         f.maxdist = L.d_maxdist;
@@ -1020,12 +1020,8 @@ static int host_mul(const uint64_t* a, size_t an, const uint64_t* b, size_t bn, 
     }
     nvtxRangePop();
     CK(cudaEventRecord(L.ev1, st));
-    // error word and the FFT distance first: a failed product leaves `out` untouched
-    if (!staged) {
-        CK(cudaMemcpyAsync(L.h_err, L.d_err, kStatBytes, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemsetAsync(L.d_err, 0, sizeof(int), st));
-        if (use_fft) CK(cudaStreamSynchronize(st));
-    }
+    // a product that FP64 rounded too far leaves `out` untouched
+    if (!staged && use_fft) CK(cudaStreamSynchronize(st));
     bool fft_failed = !staged && use_fft && (*L.h_err & kDevErrFftRound);
     if (copied) CK(cudaStreamWaitEvent(st, L.copy_done, 0));
     else if (!staged && !fft_failed) CK(cudaMemcpyAsync(out, d_out, lout * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
