@@ -112,9 +112,10 @@ __device__ __forceinline__ void wide_sums(const uint32_t* __restrict__ work, con
     static_assert(kCarryLimbs >= 4 && kCarryLimbs % 4 == 0, "limbs per thread: whole 16-byte loads");
     constexpr int L = kCarryLimbs;
     const uint64_t N = 1ull << args.k;
+    const uint64_t nc = (uint64_t)args.keep << args.k >> 3;  // coefficients there are
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Coef3 c[L];
-    if (m0 >= 0 && (uint64_t)m0 + L <= N) {  // (block 0's thread 0 starts at -4)
+    if (m0 >= 0 && (uint64_t)m0 + L <= nc) {  // (block 0's thread 0 starts at -4)
 #pragma unroll
         for (int h = 0; h < L / 4; ++h) {
             uint4 r[5];
@@ -137,7 +138,7 @@ __device__ __forceinline__ void wide_sums(const uint32_t* __restrict__ work, con
         }
     } else {
 #pragma unroll
-        for (int k = 0; k < L; ++k) c[k] = coef5<LAZY>(work, N, m0 + k, args);
+        for (int k = 0; k < L; ++k) c[k] = (uint64_t)(m0 + k) < nc ? coef5<LAZY>(work, N, m0 + k, args) : Coef3{0, 0, 0};
     }
     const u128 s_last = limb_sum(c[L - 1], c[L - 2].w1, c[L - 3].w2);
     const uint32_t hi_last = (uint32_t)(s_last >> 64);
@@ -193,7 +194,8 @@ __device__ __forceinline__ void crt_carry_tile(const ProdArgs& args, const ProdP
         const uint32_t* __restrict__ r1 = work + 2 * N;
         const uint32_t* __restrict__ r2 = work + 4 * N;
         const uint64_t i0 = 2 * (uint64_t)m0;
-        if (i0 + 2 * kCarryLimbs <= N) {
+        const uint64_t nc = (uint64_t)args.keep << args.k >> 3;  // coefficients there are
+        if (i0 + 2 * kCarryLimbs <= nc) {
             uint32_t y[3][2 * kCarryLimbs];
 #pragma unroll
             for (int h = 0; h < 2 * kCarryLimbs / 4; ++h) {
@@ -218,7 +220,7 @@ __device__ __forceinline__ void crt_carry_tile(const ProdArgs& args, const ProdP
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const uint64_t i = i0 + 2 * k + e;
-                    c[e] = i < N ? crt3_folded<SET>(ld_work<COH>(r0 + i), ld_work<COH>(r1 + i), ld_work<COH>(r2 + i),
+                    c[e] = i < nc ? crt3_folded<SET>(ld_work<COH>(r0 + i), ld_work<COH>(r1 + i), ld_work<COH>(r2 + i),
                                                     args.crt, args.f)
                                  : (u128)0;
                 }
@@ -229,7 +231,7 @@ __device__ __forceinline__ void crt_carry_tile(const ProdArgs& args, const ProdP
         prev_hi = __shfl_up_sync(0xffffffffu, (uint64_t)(T[kCarryLimbs - 1] >> 64), 1);
         if (lane == 0) {
             prev_hi = 0;
-            if (m0 > 0 && i0 - 1 < N) {
+            if (m0 > 0 && i0 - 1 < nc) {
                 const u128 c0 = crt3_folded<SET>(ld_work<COH>(r0 + i0 - 2), ld_work<COH>(r1 + i0 - 2),
                                                  ld_work<COH>(r2 + i0 - 2), args.crt, args.f);
                 const u128 c1 = crt3_folded<SET>(ld_work<COH>(r0 + i0 - 1), ld_work<COH>(r1 + i0 - 1),

@@ -41,7 +41,8 @@ namespace precgpu {
 // first stage (x, 0) -> (x, x*w) needs one twiddle product per pair.
 // Set 2 stages 64-bit limbs as two words per element (stage_limbs): the
 // element's digit is read from its row and the row 2^(M-1) above it.
-template <int SET, int M, int C, int MR>
+// E: the transform is truncated to E eighths (ntt_engine.cuh).
+template <int SET, int M, int C, int MR, int E = 8>
 __device__ __forceinline__ void col_top_upper_zero(uint32_t* sm, const uint2* __restrict__ tw, const PrimeC& c) {
     using G = Geom<M, 0, MR>;
     static_assert(G::LO >= 5, "the top pass of a multi-pass transform");
@@ -61,26 +62,29 @@ __device__ __forceinline__ void col_top_upper_zero(uint32_t* sm, const uint2* __
             x[0][q] = d;
             x[0][q + H] = Ar<SET>::twiddle(d, wq, c);
         }
-        dif_regs<SET, G::LO, G::RB, 1, G::RB - 2>(x, ulo, tw, c);
+        constexpr int LIM = E * G::R / 8;
+        dif_regs<SET, G::LO, G::RB, 1, G::RB - 2, LIM>(x, ulo, tw, c);
 #pragma unroll
-        for (int q = 0; q < G::R; ++q) s[q * G::QS * C] = x[0][q];
+        for (int q = 0; q < LIM; ++q) s[q * G::QS * C] = x[0][q];
     }
 }
 
 // The forward column pass: column group x (C columns) and y = prime*2 +
 // operand (or just the prime for a square or a launch of one operand) of
 // product z; nx = column groups per (prime, operand).
-template <int SET, int M, int C, int MR, int K2 = 0>
+template <int SET, int M, int C, int MR, int K2 = 0, int E = 8>
 __global__ void __launch_bounds__(256, cols_minb(M, MR)) k_fwd_cols(ProdArgs args, const ProdPtrs* __restrict__ batch) {
     extern __shared__ uint32_t sm[];
     pdl_enter();
 #define PREC_K2 K2
+#define PREC_E E
 #define PREC_TILE_X blockIdx.x
 #define PREC_TILE_Y blockIdx.y
 #define PREC_TILE_NX gridDim.x
 #define PREC_TILE_PRODUCT select_product(args, batch)
 #include "ntt_cols_fwd_body.inc"
 #undef PREC_K2
+#undef PREC_E
 #undef PREC_TILE_X
 #undef PREC_TILE_Y
 #undef PREC_TILE_NX
@@ -174,12 +178,14 @@ template <int SET, int M, int C, int MR>
 __device__ __forceinline__ void fwd_cols_tile(const ProdArgs& args, const ProdPtrs* __restrict__ batch,
                                               const TileIdx& ix, uint32_t* sm) {
 #define PREC_K2 0
+#define PREC_E 8
 #define PREC_TILE_X ix.bx
 #define PREC_TILE_Y ix.by
 #define PREC_TILE_NX ix.nbx
 #define PREC_TILE_PRODUCT select_product_at(args, batch, ix.bz)
 #include "ntt_cols_fwd_body.inc"
 #undef PREC_K2
+#undef PREC_E
 #undef PREC_TILE_X
 #undef PREC_TILE_Y
 #undef PREC_TILE_NX
@@ -188,16 +194,18 @@ __device__ __forceinline__ void fwd_cols_tile(const ProdArgs& args, const ProdPt
 
 // The inverse column pass: column group x, prime args.prime0 + y of
 // product z.
-template <int SET, int M, int C, int MR, int K2 = 0>
+template <int SET, int M, int C, int MR, int K2 = 0, int E = 8>
 __global__ void __launch_bounds__(256, cols_minb(M, MR)) k_inv_cols(ProdArgs args, const ProdPtrs* __restrict__ batch) {
     extern __shared__ uint32_t sm[];
     pdl_enter();
 #define PREC_K2 K2
+#define PREC_E E
 #define PREC_TILE_X blockIdx.x
 #define PREC_TILE_Y blockIdx.y
 #define PREC_TILE_PRODUCT select_product(args, batch)
 #include "ntt_cols_inv_body.inc"
 #undef PREC_K2
+#undef PREC_E
 #undef PREC_TILE_X
 #undef PREC_TILE_Y
 #undef PREC_TILE_PRODUCT
@@ -208,11 +216,13 @@ template <int SET, int M, int C, int MR>
 __device__ __forceinline__ void inv_cols_tile(const ProdArgs& args, const ProdPtrs* __restrict__ batch,
                                               const TileIdx& ix, uint32_t* sm) {
 #define PREC_K2 0
+#define PREC_E 8
 #define PREC_TILE_X ix.bx
 #define PREC_TILE_Y ix.by
 #define PREC_TILE_PRODUCT select_product_at(args, batch, ix.bz)
 #include "ntt_cols_inv_body.inc"
 #undef PREC_K2
+#undef PREC_E
 #undef PREC_TILE_X
 #undef PREC_TILE_Y
 #undef PREC_TILE_PRODUCT
@@ -249,6 +259,19 @@ __device__ __forceinline__ void inv_cols_tile(const ProdArgs& args, const ProdPt
     X(0, 9, 8, 6, 10) X(0, 10, 8, 6, 10) X(0, 10, 8, 6, 11) X(0, 11, 8, 6, 11) X(0, 11, 8, 6, 12)           \
     X(1, 10, 8, 6, 13) X(1, 11, 8, 6, 13) X(1, 12, 4, 6, 13) X(1, 13, 4, 6, 13)
 
+// The same configurations with columns of at least 2^7 points for transforms
+// truncated to E eighths (E = 5, 7: 2^8 points and up; ntt_cols_trunc.inc).
+#define PREC_COLS_FWD_TRUNC6_CONFIGS(X) X(0, 7, 8, 6, 7) X(0, 7, 8, 6, 8)
+#define PREC_COLS_FWD_TRUNC_CONFIGS(X)                                                                      \
+    X(0, 8, 8, 6, 8) X(0, 8, 8, 6, 9) X(0, 9, 8, 6, 9) X(0, 9, 8, 6, 10) X(0, 10, 8, 6, 10)                 \
+    X(0, 10, 8, 6, 11) X(0, 11, 8, 6, 11) X(0, 11, 8, 6, 12) X(2, 9, 8, 6, 9) X(2, 9, 8, 6, 10)             \
+    X(2, 10, 8, 6, 10) X(2, 10, 8, 6, 11) X(2, 11, 8, 6, 11) X(1, 11, 8, 6, 13) X(1, 12, 4, 6, 13)          \
+    X(1, 13, 4, 6, 13) X(3, 10, 8, 6, 13) X(3, 11, 8, 6, 13) X(3, 12, 4, 6, 13)
+#define PREC_COLS_INV_TRUNC_CONFIGS(X)                                                                      \
+    X(0, 8, 8, 6, 8) X(0, 8, 8, 6, 9) X(0, 9, 8, 6, 9) X(0, 9, 8, 6, 10) X(0, 10, 8, 6, 10)                 \
+    X(0, 10, 8, 6, 11) X(0, 11, 8, 6, 11) X(0, 11, 8, 6, 12) X(1, 10, 8, 6, 13) X(1, 11, 8, 6, 13)          \
+    X(1, 12, 4, 6, 13) X(1, 13, 4, 6, 13)
+
 inline size_t col_smem(int m, int cg) { return (size_t)cg * astride_for(m) * sizeof(uint32_t); }
 
 // the K2 instantiations (ntt_cols_fwd_k2.cu, ntt_cols_inv_k2.cu): launch the
@@ -260,5 +283,18 @@ bool launch_inv_cols_k2(int set, const ProdArgs& a, int cg, int mr, dim3 grid, s
                         const ProdPtrs* batch);
 int configure_fwd_cols_k2();
 int configure_inv_cols_k2();
+// the truncated instantiations of E eighths (a.keep = E), one translation
+// unit per direction and E
+#define PREC_TRUNC_DECL(E)                                                                                     \
+    bool launch_fwd_cols_trunc##E(int set, const ProdArgs& a, int cg, int mr, dim3 grid, size_t smem, cudaStream_t st, \
+                                  const ProdPtrs* batch);                                                     \
+    bool launch_inv_cols_trunc##E(int set, const ProdArgs& a, int cg, int mr, dim3 grid, size_t smem, cudaStream_t st, \
+                                  const ProdPtrs* batch);                                                     \
+    int configure_fwd_cols_trunc##E();                                                                        \
+    int configure_inv_cols_trunc##E();
+PREC_TRUNC_DECL(5)
+PREC_TRUNC_DECL(6)
+PREC_TRUNC_DECL(7)
+#undef PREC_TRUNC_DECL
 
 }  // namespace precgpu

@@ -11,6 +11,13 @@ void launch_inv_cols(int set, const ProdArgs& a, cudaStream_t st, const ProdPtrs
     col_config(set, a.k1, a.cg, a.cmr, cg, mr);
     const dim3 grid((1u << a.k2) / cg, nprimes, count);
     const size_t smem = col_smem(a.k1, cg);
+    if (a.keep < 8) {
+        if (a.keep == 5) launch_inv_cols_trunc5(set, a, cg, mr, grid, smem, st, batch);
+        else if (a.keep == 6) launch_inv_cols_trunc6(set, a, cg, mr, grid, smem, st, batch);
+        else launch_inv_cols_trunc7(set, a, cg, mr, grid, smem, st, batch);
+        count_launches(1);
+        return;
+    }
     if (launch_inv_cols_k2(set, a, cg, mr, grid, smem, st, batch)) {
         count_launches(1);
         return;
@@ -27,6 +34,9 @@ void launch_inv_cols(int set, const ProdArgs& a, cudaStream_t st, const ProdPtrs
 
 int configure_inv_cols() {
     cudaError_t e = (cudaError_t)configure_inv_cols_k2();
+    if (!e) e = (cudaError_t)configure_inv_cols_trunc5();
+    if (!e) e = (cudaError_t)configure_inv_cols_trunc6();
+    if (!e) e = (cudaError_t)configure_inv_cols_trunc7();
 #define X(S, MM, CC, RR)                                                                                   \
     if (!e) e = cudaFuncSetAttribute(k_inv_cols<S, MM, CC, RR>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                      (int)col_smem(MM, CC));

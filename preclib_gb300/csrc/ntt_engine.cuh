@@ -91,8 +91,10 @@ struct Geom {
 
 // DIF stages over bits BTOP+LO .. LO of NA arrays held in registers
 // (BTOP = RB-1: all RB stages); element q of an item sits at index
-// base + (q << LO); ulo = base & LOMASK.
-template <int SET, int LO, int RB, int NA, int BTOP = RB - 1>
+// base + (q << LO); ulo = base & LOMASK.  LIM: only elements q < LIM are
+// wanted after the last stage (a truncated transform's top pass): blocks past
+// it are not computed.
+template <int SET, int LO, int RB, int NA, int BTOP = RB - 1, int LIM = (1 << RB)>
 __device__ __forceinline__ void dif_regs(uint32_t (&x)[NA][1 << RB], uint32_t ulo, const uint2* __restrict__ tw,
                                          const PrimeC& c) {
 #pragma unroll
@@ -120,7 +122,12 @@ __device__ __forceinline__ void dif_regs(uint32_t (&x)[NA][1 << RB], uint32_t ul
         } else {
 #pragma unroll
             for (int q = 0; q < (1 << RB); ++q) {
-                if (q & h) continue;
+                if (q & h || (q & ~(h - 1)) >= LIM) continue;
+                if (((q + h) & ~(h - 1)) >= LIM) {  // the difference's block is not wanted
+#pragma unroll
+                    for (int a = 0; a < NA; ++a) x[a][q] = Ar<SET>::half(Ar<SET>::add(x[a][q], x[a][q + h], c), c);
+                    continue;
+                }
                 const uint32_t j = ulo | ((uint32_t)(q & (h - 1)) << LO);
                 const uint2 w = __ldg(&tw[(1u << (LO + bb)) + j]);
 #pragma unroll
@@ -130,12 +137,13 @@ __device__ __forceinline__ void dif_regs(uint32_t (&x)[NA][1 << RB], uint32_t ul
     }
 }
 
-// DIT stages over bits LO .. LO+RB-1.
-template <int SET, int LO, int RB, int NA>
+// DIT stages over bits LO .. LO+BEND-1 (BEND = RB: all of the pass) of
+// elements q < LIM.
+template <int SET, int LO, int RB, int NA, int BEND = RB, int LIM = (1 << RB)>
 __device__ __forceinline__ void dit_regs(uint32_t (&x)[NA][1 << RB], uint32_t ulo, const uint2* __restrict__ tw,
                                          const PrimeC& c) {
 #pragma unroll
-    for (int bb = 0; bb < RB; ++bb) {
+    for (int bb = 0; bb < BEND; ++bb) {
         const int h = 1 << bb;
         if constexpr (LO == 0) {
 #pragma unroll
@@ -159,7 +167,7 @@ __device__ __forceinline__ void dit_regs(uint32_t (&x)[NA][1 << RB], uint32_t ul
         } else {
 #pragma unroll
             for (int q = 0; q < (1 << RB); ++q) {
-                if (q & h) continue;
+                if (q & h || q >= LIM) continue;
                 const uint32_t j = ulo | ((uint32_t)(q & (h - 1)) << LO);
                 const uint2 w = __ldg(&tw[(1u << (LO + bb)) + j]);
 #pragma unroll
@@ -175,6 +183,128 @@ __device__ __forceinline__ void regs_pass(uint32_t (&x)[NA][Geom<M, T, MR>::R], 
     using G = Geom<M, T, MR>;
     if constexpr (DIT) dit_regs<SET, G::LO, G::RB, NA>(x, u & G::LOMASK, tw, c);
     else dif_regs<SET, G::LO, G::RB, NA>(x, u & G::LOMASK, tw, c);
+}
+
+// ---- truncated transforms
+//
+// A product with at most E N/8 coefficients (E = 5, 6, 7) needs no full
+// cyclic transform of length N: it is fixed by its residue modulo the
+// factors of x^N - 1 whose leaves are the first E eighths of the
+// (bit-reversed) spectrum: with M = N/8 and w the root of order 8,
+//   eighths 0..3: x^4M - 1;  4, 5: x^2M - w^2 (4 alone: x^M - w);
+//   6: x^M - w^3.
+// The forward transform leaves the other eighths out, and so do the row pass
+// and every inverse stage but the top three, where the coefficients are
+// put together from the residues (below).  (J. van der Hoeven's truncated
+// Fourier transform, ISSAC 2004, at the granularity of eighths.)
+// Measured, whole transform -> 5, 6, 7 eighths: 2^20 points 89 -> 71, 77, 83 us,
+// 2^21 162 -> 117, 134, 150, 2^22 334 -> 223, 255, 299, 2^23 685 -> 479, 552,
+// 627; 2^18 and below, where a single product is bound by latency, up to 14%;
+// the 4096 products of 200 .. 65536 limbs 13.2 -> 11.8 ms.
+
+// the last step for 2 quarters and quarter 2 (x^2M' = w_4): c0, c1 as for a
+// DIT stage, c2 the third quarter's value, all unscaled by 1/4 of the
+// length already in them -> coefficients u0, u1, u2
+template <int SET>
+__device__ __forceinline__ void trunc3(uint32_t& c0, uint32_t& c1, uint32_t& c2, uint2 w1, uint2 w2, uint2 wi,
+                                       const PrimeC& c) {
+    using A = Ar<SET>;
+    const uint32_t n0 = A::half(c0, c);
+    const uint32_t t = A::twiddle(c1, w1, c);
+    const uint32_t e = A::half(A::add(n0, t, c), c), f = A::sub(n0, t, c);
+    const uint32_t fi = A::twiddle(f, wi, c), d = A::twiddle(c2, w2, c);
+    const uint32_t g = A::half(A::sub(A::half(A::add(d, d, c), c), fi, c), c);
+    const uint32_t fn = A::half(f, c);
+    c0 = A::add(e, g, c);
+    c1 = A::add(fn, fn, c);
+    c2 = A::sub(e, g, c);
+}
+
+// Top DIT pass (element q of an item at index base + (q << LO)) of a
+// transform truncated to E eighths: eighth k of the item's values is x[k *
+// R/8 + q0].  Stages below the top three as they are, then per q0 the
+// residues' combination; out: natural coefficient order, q < E R/8.
+template <int SET, int LO, int RB, int E>
+__device__ __forceinline__ void dit_top_trunc(uint32_t (&x)[1][1 << RB], uint32_t ulo, const uint2* __restrict__ twf,
+                                              const uint2* __restrict__ twi, const PrimeC& c) {
+    using A = Ar<SET>;
+    constexpr int R = 1 << RB;
+    if constexpr (E == 6) {
+        dit_regs<SET, LO, RB, 1, RB - 2, 3 * R / 4>(x, ulo, twi, c);
+        const uint2 wi = __ldg(&twf[3]);  // w_4
+#pragma unroll
+        for (int q = 0; q < R / 4; ++q) {
+            const uint32_t j = ulo | ((uint32_t)q << LO);
+            trunc3<SET>(x[0][q], x[0][q + R / 4], x[0][q + R / 2], __ldg(&twi[(1u << (LO + RB - 2)) + j]),
+                        __ldg(&twi[(1u << (LO + RB - 1)) + j]), wi, c);
+        }
+    } else {
+        static_assert(RB >= 3 && (E == 5 || E == 7), "eighths");
+        constexpr int G = R / 8;
+        dit_regs<SET, LO, RB, 1, RB - 3, E * G>(x, ulo, twi, c);
+        const uint2 wi = __ldg(&twf[3]);
+        const uint2 w8 = __ldg(&twf[E == 5 ? 5 : 7]);  // w_8, or w_8^3
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            uint32_t* v[E];
+#pragma unroll
+            for (int k = 0; k < E; ++k) v[k] = &x[0][q + k * G];
+            const uint32_t j = ulo | ((uint32_t)q << LO), j2 = j + ((uint32_t)G << LO);
+            {   // pairs of eighths
+                const uint2 w = __ldg(&twi[(1u << (LO + RB - 3)) + j]);
+#pragma unroll
+                for (int k = 0; k + 1 < E; k += 2) A::dit(*v[k], *v[k + 1], w, c);
+            }
+            const uint2 wq = __ldg(&twi[(1u << (LO + RB - 2)) + j]), wq2 = __ldg(&twi[(1u << (LO + RB - 2)) + j2]);
+            const uint2 wh = __ldg(&twi[(1u << (LO + RB - 1)) + j]);
+            if constexpr (E == 5) {
+                // v_k = half the coefficients modulo x^4M - 1, c = 1/8 of the
+                // value at x^M = w_8 = w: t = sum w^k v_k - 4c = u_4,
+                // u_0 = 2 v_0 - t, u_k = 2 v_k
+                A::dit(*v[0], *v[2], wq, c);
+                A::dit(*v[1], *v[3], wq2, c);
+                uint32_t n[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) n[k] = A::half(*v[k], c);
+                uint32_t s = A::twiddle(n[3], w8, c);
+                s = A::twiddle(A::add(s, n[2], c), w8, c);
+                s = A::twiddle(A::add(s, n[1], c), w8, c);
+                s = A::half(A::add(s, n[0], c), c);
+                uint32_t d = A::twiddle(*v[4], wh, c);
+                d = A::half(A::add(d, d, c), c);
+                d = A::half(A::add(d, d, c), c);
+                const uint32_t t = A::half(A::sub(s, d, c), c);
+                *v[0] = A::sub(A::half(A::add(n[0], n[0], c), c), t, c);
+#pragma unroll
+                for (int k = 1; k < 4; ++k) *v[k] = A::add(n[k], n[k], c);
+                *v[4] = t;
+            } else {
+                // v_0 .. v_5: the coefficients modulo (x^4M - 1)(x^2M - i);
+                // c = 1/8 of the value at x^M = w_8^3 = h:
+                // t = (8c - sum h^k v_k) / 4i = u_6, and
+                // u_4 = v_4 - it, u_2 = v_2 - t, u_0 = v_0 + it
+                const uint2 wh2 = __ldg(&twi[(1u << (LO + RB - 1)) + j2]);
+                trunc3<SET>(*v[0], *v[2], *v[4], wq, wh, wi, c);
+                trunc3<SET>(*v[1], *v[3], *v[5], wq2, wh2, wi, c);
+                uint32_t n[6];
+#pragma unroll
+                for (int k = 0; k < 6; ++k) n[k] = A::half(*v[k], c);
+                uint32_t s = A::twiddle(n[5], w8, c);
+#pragma unroll
+                for (int k = 4; k >= 1; --k) s = A::twiddle(A::add(s, n[k], c), w8, c);
+                s = A::half(A::add(s, n[0], c), c);
+                uint32_t d = A::twiddle(A::twiddle(*v[6], wq, c), wh, c);  // w^-3j
+#pragma unroll
+                for (int k = 0; k < 3; ++k) d = A::half(A::add(d, d, c), c);
+                const uint32_t t = A::twiddle(A::sub(d, s, c), make_uint2(c.q4, c.q4p), c);
+                const uint32_t ti = A::twiddle(t, wi, c);
+                *v[0] = A::add(n[0], ti, c);
+                *v[2] = A::sub(n[2], t, c);
+                *v[4] = A::sub(n[4], ti, c);
+                *v[6] = t;
+            }
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -336,12 +466,14 @@ __device__ __forceinline__ void row_passes(uint32_t* sm, int astride, int narr, 
     }
 }
 
-template <int SET, int M, int T, int TEND, bool DIT, int C, int MR = PREC_SCH_MAXRB>
+// E: the first E eighths of the items only (a truncated transform; below the
+// top pass an item lies in one eighth)
+template <int SET, int M, int T, int TEND, bool DIT, int C, int MR = PREC_SCH_MAXRB, int E = 8>
 __device__ __forceinline__ void col_passes(uint32_t* sm, const uint2* __restrict__ tw, const PrimeC& c) {
     if constexpr (DIT ? (T >= TEND) : (T <= TEND)) {
-        col_pass<SET, M, T, DIT, C, false, MR>(sm, tw, c);
+        col_pass<SET, M, T, DIT, C, false, MR>(sm, tw, c, 0, E * ((C << Geom<M, T, MR>::LGI) / 8));
         __syncthreads();
-        col_passes<SET, M, DIT ? T - 1 : T + 1, TEND, DIT, C, MR>(sm, tw, c);
+        col_passes<SET, M, DIT ? T - 1 : T + 1, TEND, DIT, C, MR, E>(sm, tw, c);
     }
 }
 

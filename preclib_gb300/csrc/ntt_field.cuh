@@ -71,6 +71,7 @@ struct PrimeC {
     uint32_t p2;      // 2p
     uint32_t r32;     // 2^32 mod p
     uint32_t r32p;    // its Shoup constant floor(r32 * 2^32 / p)
+    uint32_t q4, q4p; // 1 / (4 w_4) mod p and its Shoup constant (w_4: the set's root of order 4)
 };
 
 #ifdef __CUDACC__
@@ -150,6 +151,9 @@ struct Ar<0> {
     static __device__ __forceinline__ uint32_t half(uint32_t x, const PrimeC& c) {
         return min(x, x - c.p2);
     }
+    // forward-range operands -> inverse range
+    static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b, const PrimeC&) { return a + b; }
+    static __device__ __forceinline__ uint32_t sub(uint32_t a, uint32_t b, const PrimeC& c) { return a - b + c.p2; }
 };
 
 // set 2: set 0's arithmetic; a digit is a whole 64-bit limb hi*2^32 + lo
@@ -201,6 +205,8 @@ struct Ar<1> {
         return red1(shoup_lazy(x, w.x, w.y, c.p), c.p);
     }
     static __device__ __forceinline__ uint32_t half(uint32_t x, const PrimeC&) { return x; }
+    static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b, const PrimeC& c) { return red1(a + b, c.p); }
+    static __device__ __forceinline__ uint32_t sub(uint32_t a, uint32_t b, const PrimeC& c) { return sub_mod(a, b, c.p); }
 };
 
 // set 3: set 1's arithmetic; a digit is a whole 64-bit limb hi*2^32 + lo

@@ -64,6 +64,7 @@ struct ProdArgs {
     int rows;           // rows per CTA of the row pass
     int square;         // a == b: one operand transform, pointwise square
     int prime0;         // first prime of this launch of the transform kernels (grid.y covers the rest)
+    int keep;           // eighths of the transform kept (8: all; fewer: truncated, ntt_engine.cuh)
     int cg;             // columns per column-pass CTA (0: default)
     int cmr;            // column pass radix cap, 4 or 6 (0: default)
     int chain;          // per-prime chains (host side: how the kernels are launched)
@@ -323,6 +324,8 @@ void launch_crt_carry(int set, const ProdArgs& a, cudaStream_t st, const ProdPtr
                       int max_nblk = 0, int nblk_launch = 0);
 int configure_fwd_cols();
 int configure_inv_cols();
+// whether the column kernels of a configuration exist truncated to `keep` eighths
+bool cols_trunc_supported(int set, int k1, int k2, int cg, int mr, int keep);
 
 // Column-pass configuration instantiated for (set, m = log2 N1) closest to
 // the requested columns per CTA and radix cap (0 = default: 8 columns,

@@ -54,7 +54,8 @@ void launch_rows(int set, const ProdArgs& a, cudaStream_t st, const ProdPtrs* ba
     if (nprimes <= 0) nprimes = kSetPrimes[set];
     set = set_base(set);  // sets 2 and 3: the same kernel on their residues
     const int m = a.k2;
-    const dim3 grid((1u << a.k1) / a.rows, nprimes, count);
+    // (a truncated transform: the first a.keep eighths of the row slots)
+    const dim3 grid(((unsigned)a.keep << a.k1) / 8 / a.rows, nprimes, count);
     const int threads = a.rows << (m - 5);
     const size_t smem = row_smem(m, a.rows);
     const int mr = row_radix_cap(m, a.rmr);

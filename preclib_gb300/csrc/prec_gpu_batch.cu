@@ -138,6 +138,7 @@ static void batch_enqueue(prec_gpu_batch* b, cudaStream_t origin, bool branch) {
             args.k1 = c.pl.k1;
             args.k2 = c.pl.k2;
             args.rows = c.pl.rows;
+            args.keep = c.pl.keep;
             args.cg = c.pl.cg;
             args.cmr = c.pl.cmr;
             args.rmr = c.pl.rmr;
@@ -164,6 +165,34 @@ static void batch_enqueue(prec_gpu_batch* b, cudaStream_t origin, bool branch) {
     }
 }
 
+// The classes of one transform length that differ in the eighths they keep
+// are worth their own four launches only with enough work: a class whose
+// truncation saves less than kMergeButterflies moves into the next longer one
+// there is (a truncated transform of more eighths also fits its products).
+// 2^22 butterflies are about 1.5 us of the whole GPU, a class's launches.
+constexpr uint64_t kMergeButterflies = 1ull << 22;
+
+static void merge_small_classes(std::vector<int>& cls_of, std::vector<Cls>& found) {
+    for (int key = 0; key < 1 << 9; ++key) {
+        int last = -1;  // the longer class seen last
+        for (int e = 8; e >= 5; --e) {
+            int& ci = cls_of[(e - 5) << 9 | key];
+            if (ci < 0) continue;
+            Cls& c = found[ci];
+            const uint64_t saves = last < 0 ? 0 : (c.items.size() * c.pl.nprimes * 3 * c.pl.k << c.pl.k) / 2 *
+                                                      (found[last].pl.keep - c.pl.keep) / 8;
+            if (last >= 0 && saves < kMergeButterflies) {
+                std::vector<int>& to = found[last].items;
+                to.insert(to.end(), c.items.begin(), c.items.end());
+                c.items.clear();
+                ci = -1;
+            } else {
+                last = ci;
+            }
+        }
+    }
+}
+
 // Plans a batch and uploads its descriptors.  `oneshot` (prec_gpu_mul_batch):
 // the device memory comes stream-ordered from the library pool on that
 // stream (no device-wide allocation or free per call), and no stream
@@ -179,12 +208,15 @@ static int batch_build(const prec_gpu_product_t* items, size_t count, bool onesh
     b->oneshot = ost;
     b->items.assign(items, items + count);
     b->err = ctx_device_err();
-    // classes by key (64-bit digits << 8 | k << 1 | square, or the direct
-    // form's class past those): a dense table, not a map lookup per product
-    // (a binary-splitting level has ~10^6 of them)
-    constexpr int kDirectKey = 1 << 9;
+    // classes by key ((eighths of the transform - 5) << 9 | 64-bit digits << 8
+    // | k << 1 | square, or the direct form's class past those): a dense
+    // table, not a map lookup per product (a binary-splitting level has ~10^6
+    // of them)
+    constexpr int kDirectKey = 1 << 11;
     std::vector<int> cls_of(kDirectKey + kDirectClasses, -1);
     std::vector<Cls> found;
+    const char* pe = std::getenv("PREC_GPU_BATCH_PERSISTENT");
+    const bool persistent = pe && pe[0] == '1';
     const bool wide = wide_digits();
     for (size_t i = 0; i < count; ++i) {
         const prec_gpu_product_t& p = items[i];
@@ -220,14 +252,23 @@ static int batch_build(const prec_gpu_product_t* items, size_t count, bool onesh
         const int kw = wide ? wide_log2(p.an, p.bn, k) : 0;
         if (kw) k = kw;
         const int sq = (p.a == p.b && p.an == p.bn && k > kSmallMaxLog2) ? 1 : 0;
-        int& ci = cls_of[(kw ? 1 << 8 : 0) | k << 1 | sq];
+        // eighths of the transform the product needs (8 also where the
+        // operands do not fit its lower half: no truncated form)
+        int keep = 8;
+        const uint64_t per = kw ? 1 : 2, hi = std::max(p.an, p.bn);
+        if (!persistent && k > kSmallMaxLog2 && 2 * per * hi <= 1ull << k) {
+            const uint64_t eighth = 1ull << (k - 3);
+            keep = std::max(5, (int)((per * (p.an + p.bn) - 1 + eighth - 1) / eighth));
+        }
+        int& ci = cls_of[(keep - 5) << 9 | (kw ? 1 << 8 : 0) | k << 1 | sq];
         if (ci < 0) {
             ci = (int)found.size();
             found.emplace_back();
         }
         Cls& c = found[ci];
         if (c.items.empty()) {
-            if ((r = plan_for(2 * (uint64_t)p.an, 2 * (uint64_t)p.bn, p.an + p.bn, c.pl, wide))) {
+            if ((r = plan_for(2 * (uint64_t)p.an, 2 * (uint64_t)p.bn, p.an + p.bn, c.pl, wide,
+                              persistent))) {
                 batch_free(b);
                 return r;
             }
@@ -240,11 +281,10 @@ static int batch_build(const prec_gpu_product_t* items, size_t count, bool onesh
         }
         c.items.push_back((int)i);
     }
+    merge_small_classes(cls_of, found);
     // device layout: descriptors, then one workspace per four-step class
     // (and, for a persistent class, its scheduling words)
     const size_t budget = env_bytes("PREC_GPU_BATCH_CLASS_BYTES", (size_t)1 << 30);
-    const char* pe = std::getenv("PREC_GPU_BATCH_PERSISTENT");
-    const bool persistent = pe && pe[0] == '1';
     // a dependency wait gives up after about a second (PREC_GPU_BATCH_SPIN_LIMIT polls
     // of ~0.25 us; tests shorten it); PREC_GPU_BATCH_NEVER_SIGNAL=1 (tests)
     // makes every such wait run out

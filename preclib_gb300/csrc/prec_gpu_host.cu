@@ -105,6 +105,7 @@ PrimeC prime_constants(uint32_t p) {
     pc.p2 = 2 * p;
     pc.r32 = (uint32_t)((1ull << 32) % p);
     pc.r32p = (uint32_t)(((uint64_t)pc.r32 << 32) / p);
+    pc.q4 = pc.q4p = 0;  // needs the set's root: build_tables
     return pc;
 }
 
@@ -213,8 +214,20 @@ int wide_log2(uint64_t la, uint64_t lb, int k32) {
     return 0;
 }
 
+// Truncated transforms take both operands in the lower half (their only
+// first pass) and row slots in whole row CTAs.
+int plan_keep(const Plan& pl, uint64_t la, uint64_t lb) {
+    const uint64_t N = 1ull << pl.k, hi = la > lb ? la : lb;
+    if (pl.path != 1 || 2 * hi > N) return 8;
+    for (int e = 5; e < 8; ++e)
+        if (la + lb - 1 <= (N >> 3) * e && (e << pl.k1) / 8 % pl.rows == 0 &&
+            cols_trunc_supported(pl.set, pl.k1, pl.k2, pl.cg, pl.cmr, e))
+            return e;
+    return 8;
+}
+
 // da, db: 32-bit digit counts (upper bounds are fine)
-int plan_for(uint64_t da, uint64_t db, uint64_t lout, Plan& pl, bool wide) {
+int plan_for(uint64_t da, uint64_t db, uint64_t lout, Plan& pl, bool wide, bool whole) {
     int k = ceil_log2(da + db - 1);
     if (k < kSmallMinLog2) k = kSmallMinLog2;
     if (k > kMaxLog2) return PREC_GPU_E_TOO_LARGE;
@@ -239,6 +252,7 @@ int plan_for(uint64_t da, uint64_t db, uint64_t lout, Plan& pl, bool wide) {
         }
     }
     apply_config(pl, config_for(k, pl.set));
+    if (!whole) pl.keep = set_wide(pl.set) ? plan_keep(pl, (da + 1) / 2, (db + 1) / 2) : plan_keep(pl, da, db);
     const uint64_t bl = (uint64_t)crt_block_limbs(pl.set);
     pl.nblk = (int)((lout + bl - 1) / bl);
     pl.work_bytes = ((size_t)2 * pl.nprimes << k) * sizeof(uint32_t) + ((size_t)pl.nblk + 1) * sizeof(uint32_t);
@@ -427,6 +441,9 @@ static int build_tables(Ctx& c) {
             if (powmod(kG[set][j], (p - 1) / 2, p) != p - 1) return PREC_GPU_E_INTERNAL;
             if (((p - 1) >> L) << L != p - 1) return PREC_GPU_E_INTERNAL;
             const uint32_t wL = powmod(kG[set][j], (p - 1) >> L, p);
+            const ShoupC q4 = shoup(invmod(mulmod(4, powmod(wL, 1ull << (L - 2), p), p), p), p);
+            fa.pc[j].q4 = q4.w;
+            fa.pc[j].q4p = q4.wp;
             const size_t off = per_prime * (set * kMaxPrimes + j);
             uint2* tf = reinterpret_cast<uint2*>(host.data() + off);
             uint2* ti = tf + T;
@@ -720,6 +737,7 @@ static int enqueue_ntt(Ctx& c, Lane& L, const uint64_t* d_a, uint64_t la, const 
         args.k2 = pl.k2;
         args.nblk = pl.nblk;
         args.rows = pl.rows;
+        args.keep = pl.keep;
         args.cg = pl.cg;
         args.cmr = pl.cmr;
         args.rmr = pl.rmr;

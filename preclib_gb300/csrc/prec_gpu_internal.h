@@ -40,6 +40,7 @@ struct Plan {
     int path = 0;  // 0 single CTA, 1 four-step
     int nblk = 0;
     int rows = 0;  // rows per CTA of the row pass
+    int keep = 8;  // eighths of the transform kept (8: all)
     int cg = 0;    // columns per column-pass CTA (0: default)
     int cmr = 0;   // column pass radix cap (0: default)
     int rmr = 0;   // row pass radix cap (0: default)
@@ -57,7 +58,12 @@ struct Plan {
 // primes, half the points) where that costs fewer butterflies; single
 // products, the batch form and the serving loop pass wide_digits(), the
 // autotuner keeps 32-bit digits.
-int plan_for(uint64_t da, uint64_t db, uint64_t lout, Plan& pl, bool wide = false);
+// A product that needs at most 5, 6 or 7 eighths of its transform runs
+// truncated (keep) where such kernels exist; `whole` asks for all of it.
+int plan_for(uint64_t da, uint64_t db, uint64_t lout, Plan& pl, bool wide = false, bool whole = false);
+// eighths of the 2^k-point transform of plan `pl` (its configuration
+// applied) that a product of la x lb digits of the plan's width needs
+int plan_keep(const Plan& pl, uint64_t la, uint64_t lb);
 // log2 of the 64-bit-digit transform for la x lb limbs, or 0 where the
 // 32-bit plan of 2^k32 points stays: it needs 2^13 .. 2^25 points, both
 // operands in the lower half, min(la, lb) within the five primes' bound,

@@ -262,6 +262,7 @@ extern "C" int prec_gpu_mul_device_noalloc(const uint64_t* d_a, size_t an, const
         args.k = k;
         args.k1 = k / 2;
         args.k2 = k - args.k1;
+        args.keep = 8;
         ntt_row_threads(args.k2, 1 << args.k1, &args.rows);
         const uint64_t bl = (uint64_t)kCarryThreads * kCarryLimbs;
         args.nblk = (int)((lout + bl - 1) / bl);

@@ -123,6 +123,7 @@ static int launch_request(prec_gpu_server* s, Slot& sl) {
         args.k2 = r.pl.k2;
         args.nblk = r.pl.nblk;
         args.rows = r.pl.rows;
+        args.keep = r.pl.keep;
         args.cg = r.pl.cg;
         args.cmr = r.pl.cmr;
         args.rmr = r.pl.rmr;
