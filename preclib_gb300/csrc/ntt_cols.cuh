@@ -18,7 +18,7 @@
 // P(i)*C + c); a warp covers C columns x 32/C items, so every global access
 // moves whole 32-byte sectors.
 // Template parameters: SET prime set, M = log2 N1 (column length), C
-// columns per CTA (launched with 32*C threads), MR the pass radix cap (MR = 6: a 2^11-point column runs
+// columns per CTA (launched with 32*C threads, at most 256), MR the pass radix cap (MR = 6: a 2^11-point column runs
 // as a radix-64 and a radix-32 pass; MR = 4: radix-8, -8, -32), K2 =
 // log2 N2 (the row length, the stride between a column's elements) as a
 // constant, or 0: from the arguments.  The instantiated (SET, M, C, MR)
@@ -259,19 +259,32 @@ __device__ __forceinline__ void inv_cols_tile(const ProdArgs& args, const ProdPt
     X(0, 9, 8, 6, 10) X(0, 10, 8, 6, 10) X(0, 10, 8, 6, 11) X(0, 11, 8, 6, 11) X(0, 11, 8, 6, 12)           \
     X(1, 10, 8, 6, 13) X(1, 11, 8, 6, 13) X(1, 12, 4, 6, 13) X(1, 13, 4, 6, 13)
 
+// Batch classes with enough products take more short columns per CTA, 8192
+// points as the 2^10-point columns have (col_batch_group): the bottom pass
+// has 32 points per thread, so a tile of 8 columns of 2^8 points keeps 2 of its 8
+// warps busy there and the other six at the barrier.
+#define PREC_COLS_FWD_BATCH_CONFIGS(X) X(0, 8, 32, 6, 8) X(0, 8, 32, 6, 9) X(0, 9, 16, 6, 9) X(2, 9, 16, 6, 9) X(2, 9, 16, 6, 10)
+#define PREC_COLS_INV_BATCH_CONFIGS(X) X(0, 8, 32, 6, 8) X(0, 8, 32, 6, 9) X(0, 9, 16, 6, 9) X(0, 9, 16, 6, 10)
+#define PREC_COLS_FWD_BATCH_SHORT_CONFIGS(X) X(0, 7, 64, 6, 7) X(0, 7, 64, 6, 8)
+#define PREC_COLS_INV_BATCH_SHORT_CONFIGS(X) X(0, 7, 64, 6, 7) X(0, 7, 64, 6, 8)
+// (2^6-point columns: whole transforms only)
+#define PREC_COLS_BATCH_SHORTEST_CONFIGS(X) X(0, 6, 64, 6, 7)
+
 // The same configurations with columns of at least 2^7 points for transforms
 // truncated to E eighths (E = 5, 7: 2^8 points and up; ntt_cols_trunc.inc).
-#define PREC_COLS_FWD_TRUNC6_CONFIGS(X) X(0, 7, 8, 6, 7) X(0, 7, 8, 6, 8)
+#define PREC_COLS_FWD_TRUNC6_CONFIGS(X) X(0, 7, 8, 6, 7) X(0, 7, 8, 6, 8) PREC_COLS_FWD_BATCH_SHORT_CONFIGS(X)
+#define PREC_COLS_INV_TRUNC6_CONFIGS(X) X(0, 7, 8, 6, 7) X(0, 7, 8, 6, 8) PREC_COLS_INV_BATCH_SHORT_CONFIGS(X)
 #define PREC_COLS_FWD_TRUNC_CONFIGS(X)                                                                      \
     X(0, 8, 8, 6, 8) X(0, 8, 8, 6, 9) X(0, 9, 8, 6, 9) X(0, 9, 8, 6, 10) X(0, 10, 8, 6, 10)                 \
     X(0, 10, 8, 6, 11) X(0, 11, 8, 6, 11) X(0, 11, 8, 6, 12) X(2, 9, 8, 6, 9) X(2, 9, 8, 6, 10)             \
-    X(2, 10, 8, 6, 10) X(2, 10, 8, 6, 11) X(2, 11, 8, 6, 11) X(1, 11, 8, 6, 13) X(1, 12, 4, 6, 13)          \
+    PREC_COLS_FWD_BATCH_CONFIGS(X) X(2, 10, 8, 6, 10) X(2, 10, 8, 6, 11) X(2, 11, 8, 6, 11) X(1, 11, 8, 6, 13) X(1, 12, 4, 6, 13)          \
     X(1, 13, 4, 6, 13) X(3, 10, 8, 6, 13) X(3, 11, 8, 6, 13) X(3, 12, 4, 6, 13)
 #define PREC_COLS_INV_TRUNC_CONFIGS(X)                                                                      \
     X(0, 8, 8, 6, 8) X(0, 8, 8, 6, 9) X(0, 9, 8, 6, 9) X(0, 9, 8, 6, 10) X(0, 10, 8, 6, 10)                 \
     X(0, 10, 8, 6, 11) X(0, 11, 8, 6, 11) X(0, 11, 8, 6, 12) X(1, 10, 8, 6, 13) X(1, 11, 8, 6, 13)          \
-    X(1, 12, 4, 6, 13) X(1, 13, 4, 6, 13)
+    PREC_COLS_INV_BATCH_CONFIGS(X) X(1, 12, 4, 6, 13) X(1, 13, 4, 6, 13)
 
+inline int col_threads(int cg) { return cg < 8 ? 32 * cg : 256; }
 inline size_t col_smem(int m, int cg) { return (size_t)cg * astride_for(m) * sizeof(uint32_t); }
 
 // the K2 instantiations (ntt_cols_fwd_k2.cu, ntt_cols_inv_k2.cu): launch the

@@ -22,10 +22,13 @@ bool launch_fwd_cols_k2(int set, const ProdArgs& a, int cg, int mr, dim3 grid, s
     }
 #define X(S, MM, CC, RR, KK)                                                                   \
     if (set == S && a.k1 == MM && cg == CC && mr == RR && a.k2 == KK) {                         \
-        launch_pdl(a.chain != 0, k_fwd_cols<S, MM, CC, RR, KK>, grid, 32 * CC, smem, st, a, batch);        \
+        launch_pdl(a.chain != 0, k_fwd_cols<S, MM, CC, RR, KK>, grid, col_threads(CC), smem, st, a, batch);        \
         return true;                                                                            \
     }
     PREC_COLS_FWD_K2_CONFIGS(X)
+    PREC_COLS_FWD_BATCH_CONFIGS(X)
+    PREC_COLS_FWD_BATCH_SHORT_CONFIGS(X)
+    PREC_COLS_BATCH_SHORTEST_CONFIGS(X)
 #undef X
     return false;
 }
@@ -37,6 +40,9 @@ int configure_fwd_cols_k2() {
     if (!e) e = cudaFuncSetAttribute(k_fwd_cols<S, MM, CC, RR, KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                      (int)col_smem(MM, CC));
     PREC_COLS_FWD_K2_CONFIGS(X)
+    PREC_COLS_FWD_BATCH_CONFIGS(X)
+    PREC_COLS_FWD_BATCH_SHORT_CONFIGS(X)
+    PREC_COLS_BATCH_SHORTEST_CONFIGS(X)
 #undef X
     return (int)e;
 }

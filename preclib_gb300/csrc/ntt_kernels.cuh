@@ -328,7 +328,8 @@ int configure_inv_cols();
 bool cols_trunc_supported(int set, int k1, int k2, int cg, int mr, int keep);
 
 // Column-pass configuration instantiated for (set, m = log2 N1) closest to
-// the requested columns per CTA and radix cap (0 = default: 8 columns,
+// the requested columns per CTA (4, 8 or, for batch classes in the default
+// configuration, col_batch_group's) and radix cap (0 = default: 8 columns,
 // radix cap 6).  The radix cap only changes the schedule of 2^10- and
 // 2^11-point columns; set 1's 2^12- and 2^13-point columns take 4 columns.
 // Row-pass radix cap instantiated for m = log2 N2 (0 = default): the cap
@@ -340,9 +341,12 @@ inline int row_radix_cap(int m, int req) {
     return req == 4 || req == 6 ? req : (m == 10 ? 6 : 4);
 }
 
+// columns per CTA of a batch class with columns of 2^m points: 8192 points
+// per tile, at most 64 columns (set 0's arithmetic; 8 from 2^10 points on)
+inline int col_batch_group(int m) { return m >= 10 ? 8 : (m <= 7 ? 64 : 1 << (13 - m)); }
 inline void col_config(int set, int m, int req_cg, int req_mr, int& cg, int& mr) {
     set = set_base(set);
-    cg = (req_cg == 4 || req_cg == 8) ? req_cg : kColGroup;
+    cg = req_cg >= 4 ? req_cg : kColGroup;
     if (set == 1 && m >= 12) cg = 4;
     mr = (m == 10 || m == 11) && req_mr == 4 ? 4 : 6;
 }

@@ -193,6 +193,23 @@ static void merge_small_classes(std::vector<int>& cls_of, std::vector<Cls>& foun
     }
 }
 
+// More columns per column CTA (col_batch_group) where that leaves a CTA for
+// half the SMs, in the default configuration.  Per product, 8 columns -> the
+// group: 2467 products of 1700 limbs 0.79 -> 0.28 us, 699 of 6000 1.84 -> 0.83,
+// 174 of 24000 5.6 -> 3.5; 16 products of 3000 limbs (96 CTAs) 2.07 -> 1.82, of 6000
+// 2.7 -> 2.07.  A single product stays with 8 columns: 20011 x 13001 limbs
+// 19.6 us, 20.7 with 32.
+static void group_columns(Cls& c) {
+    if (c.direct >= 0 || c.pl.path != 1 || set_base(c.pl.set) != 0) return;
+    const KernelConfig d = default_config(c.pl.k);
+    if (d.k1 != c.pl.k1 || d.cg != c.pl.cg || d.cmr != c.pl.cmr) return;
+    const int g = col_batch_group(c.pl.k1);
+    // (instantiated: set 0 up to 2^18 points, set 2 up to 2^19)
+    if (g == c.pl.cg || c.pl.k > (set_wide(c.pl.set) ? 19 : 18)) return;
+    const uint64_t ctas = (uint64_t)c.items.size() * c.pl.nprimes << c.pl.k2;
+    if (ctas / g >= (uint64_t)device_sm_count() / 2) c.pl.cg = g;
+}
+
 // Plans a batch and uploads its descriptors.  `oneshot` (prec_gpu_mul_batch):
 // the device memory comes stream-ordered from the library pool on that
 // stream (no device-wide allocation or free per call), and no stream
@@ -282,6 +299,8 @@ static int batch_build(const prec_gpu_product_t* items, size_t count, bool onesh
         c.items.push_back((int)i);
     }
     merge_small_classes(cls_of, found);
+    for (int ci : cls_of)
+        if (ci >= 0 && !persistent) group_columns(found[ci]);
     // device layout: descriptors, then one workspace per four-step class
     // (and, for a persistent class, its scheduling words)
     const size_t budget = env_bytes("PREC_GPU_BATCH_CLASS_BYTES", (size_t)1 << 30);
