@@ -745,7 +745,7 @@ static int enqueue_ntt(Ctx& c, Lane& L, const uint64_t* d_a, uint64_t la, const 
         args.crt = pl.crt;
         args.crt5 = pl.crt5;
         args.f = c.field[pl.set];
-        const bool split = c.split_primes && pl.split;
+        const bool split = c.split_primes && (pl.split || a_ready);
         ntt_launch_4step(pl.set, args, st, ev, split ? &L.prime_streams : nullptr, a_ready, b_ready,
                          split ? chunks : nullptr);
     }
@@ -903,6 +903,11 @@ enum { kModeBands = 0, kModeNtt = 1, kModeFft = 2 };
 // cost more than the copy engine's.
 constexpr size_t kStagedLimbs = 32768;
 
+// Host products from 2^19 points run per-prime chains even where a device
+// product does not: a's transforms start while b is still on its way, and
+// the result goes out chunk by chunk.
+constexpr int kHostChainMinLog2 = 19;
+
 static int ensure_pin(Lane& L) {
     if (L.pin) return 0;
     // operands and result, each from a 256-byte boundary
@@ -956,7 +961,7 @@ static int host_mul(const uint64_t* a, size_t an, const uint64_t* b, size_t bn, 
     // operands and result each start on a 256-byte boundary (32 limbs)
     const size_t la_pad = (la + 31) & ~(size_t)31, lb_pad = square ? 0 : (lb + 31) & ~(size_t)31;
     // per-prime chains start on a's forward columns while b is copied
-    const bool chains = !use_fft && !blocked && pl.path == 1 && c.split_primes && pl.split;
+    const bool chains = !use_fft && !blocked && pl.path == 1 && c.split_primes && (pl.split || pl.k >= kHostChainMinLog2);
     const bool staged = !blocked && !chains && lout <= kStagedLimbs && ensure_pin(L) == 0;
     if ((r = ensure_io(L, la_pad + lb_pad + lout))) return r;
     uint64_t* buf = staged ? L.pin : L.io;

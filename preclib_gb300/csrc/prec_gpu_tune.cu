@@ -29,7 +29,12 @@ namespace {
 
 constexpr int kTuneMin = kSmallMaxLog2 + 1;         // first four-step length
 constexpr int kTuneMax = kMaxLog2;                 // 26
-constexpr int kSplitMinLog2 = 19;  // default: per-prime streams from 2^19 points
+// Default: per-prime streams from 2^21 points.  Below, four programmatic
+// launches over all primes are faster than 16 on six streams (64-bit digits,
+// chains -> one launch per pass: 2^19 points at 6/8 53.8 -> 45.9 us, whole 58.4 ->
+// 52.9; 2^20 76.8 -> 73.8 and 89.3 -> 87.1; 2^21 135.2 -> 134.6 and 162.0 ->
+// 164.1; 2^22 255 -> 264 and 333 -> 346).
+constexpr int kSplitMinLog2 = 21;
 
 struct Entry {
     bool tuned = false;
