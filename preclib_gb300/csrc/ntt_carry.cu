@@ -5,8 +5,10 @@
 
 namespace precgpu {
 
+// (5 resident CTAs, 48 registers: at 6 the five-prime CRT spills 40 bytes, no
+// faster; at 4 4M x 4M limbs take 691 us instead of 685)
 template <int SET>
-__global__ void __launch_bounds__(kCarryThreads, set_wide(SET) ? 6 : 5) k_crt_carry(ProdArgs args, const ProdPtrs* __restrict__ batch) {
+__global__ void __launch_bounds__(kCarryThreads, 5) k_crt_carry(ProdArgs args, const ProdPtrs* __restrict__ batch) {
     pdl_enter();
     crt_carry_tile<SET>(args, batch, GridIdx{});
 }

@@ -39,12 +39,13 @@ struct CrtConst {
 // Garner constants of the five-prime set for one transform length:
 // v_j = y_j * a_j - sum_{i<j} v_i * b_{ij} (mod p_j), with
 // a_j = 2^32 N^-1 (p_0 .. p_{j-1})^-1 and b_{ij} = (p_i .. p_{j-1})^-1 mod p_j;
-// b_{ij} is b[j(j-1)/2 + i] (primes counted from 0).  The inverse column
-// pass multiplies prime j's values by a_j (fold[j] = a_j * 2^32 mod p_j,
-// Montgomery form, on its running twiddle), so the CRT starts from
-// y_j * a_j directly.
+// n[j(j-1)/2 + i] = -b_{ij} * 2^32 mod p_j (primes counted from 0; the
+// Montgomery reduction takes the 2^32 away).  The inverse column pass
+// multiplies prime j's values by a_j, and by another 2^32 for j > 0 (fold[j] =
+// that factor * 2^32 mod p_j, Montgomery form, on its running twiddle), so the
+// CRT starts from y_j * a_j directly.
 struct Crt5Const {
-    ShoupC b[10];
+    uint32_t n[10];
     uint32_t fold[5];
 };
 

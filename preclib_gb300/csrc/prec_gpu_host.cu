@@ -158,11 +158,11 @@ static Crt5Const crt5_compute(int set, int k) {
         const uint32_t R = (uint32_t)((1ull << 32) % p);
         uint32_t a = mulmod(R, invmod((uint32_t)((1ull << k) % p), p), p);
         for (int i = 0; i < j; ++i) a = mulmod(a, invmod(P[i] % p, p), p);
-        c.fold[j] = mulmod(a, R, p);
+        c.fold[j] = mulmod(j ? mulmod(a, R, p) : a, R, p);
         for (int i = 0; i < j; ++i) {
             uint32_t b = 1;
             for (int l = i; l < j; ++l) b = mulmod(b, invmod(P[l] % p, p), p);
-            c.b[j * (j - 1) / 2 + i] = shoup(b, p);
+            c.n[j * (j - 1) / 2 + i] = (p - mulmod(b, R, p)) % p;
         }
     }
     return c;
