@@ -18,7 +18,7 @@
 // P(i)*C + c); a warp covers C columns x 32/C items, so every global access
 // moves whole 32-byte sectors.
 // Template parameters: SET prime set, M = log2 N1 (column length), C
-// columns per CTA (launched with 32*C threads, at most 256), MR the pass radix cap (MR = 6: a 2^11-point column runs
+// columns per CTA (launched with col_threads(C, M) threads), MR the pass radix cap (MR = 6: a 2^11-point column runs
 // as a radix-64 and a radix-32 pass; MR = 4: radix-8, -8, -32), K2 =
 // log2 N2 (the row length, the stride between a column's elements) as a
 // constant, or 0: from the arguments.  The instantiated (SET, M, C, MR)
@@ -73,7 +73,7 @@ __device__ __forceinline__ void col_top_upper_zero(uint32_t* sm, const uint2* __
 // operand (or just the prime for a square or a launch of one operand) of
 // product z; nx = column groups per (prime, operand).
 template <int SET, int M, int C, int MR, int K2 = 0, int E = 8>
-__global__ void __launch_bounds__(256, cols_minb(M, MR)) k_fwd_cols(ProdArgs args, const ProdPtrs* __restrict__ batch) {
+__global__ void __launch_bounds__(col_threads(C, M), cols_minb(M, MR, C)) k_fwd_cols(ProdArgs args, const ProdPtrs* __restrict__ batch) {
     extern __shared__ uint32_t sm[];
     pdl_enter();
 #define PREC_K2 K2
@@ -195,7 +195,7 @@ __device__ __forceinline__ void fwd_cols_tile(const ProdArgs& args, const ProdPt
 // The inverse column pass: column group x, prime args.prime0 + y of
 // product z.
 template <int SET, int M, int C, int MR, int K2 = 0, int E = 8>
-__global__ void __launch_bounds__(256, cols_minb(M, MR)) k_inv_cols(ProdArgs args, const ProdPtrs* __restrict__ batch) {
+__global__ void __launch_bounds__(col_threads(C, M), cols_minb(M, MR, C)) k_inv_cols(ProdArgs args, const ProdPtrs* __restrict__ batch) {
     extern __shared__ uint32_t sm[];
     pdl_enter();
 #define PREC_K2 K2
@@ -284,7 +284,6 @@ __device__ __forceinline__ void inv_cols_tile(const ProdArgs& args, const ProdPt
     X(0, 10, 8, 6, 11) X(0, 11, 8, 6, 11) X(0, 11, 8, 6, 12) X(1, 10, 8, 6, 13) X(1, 11, 8, 6, 13)          \
     PREC_COLS_INV_BATCH_CONFIGS(X) X(1, 12, 4, 6, 13) X(1, 13, 4, 6, 13)
 
-inline int col_threads(int cg) { return cg < 8 ? 32 * cg : 256; }
 inline size_t col_smem(int m, int cg) { return (size_t)cg * astride_for(m) * sizeof(uint32_t); }
 
 // the K2 instantiations (ntt_cols_fwd_k2.cu, ntt_cols_inv_k2.cu): launch the

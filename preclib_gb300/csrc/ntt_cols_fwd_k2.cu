@@ -22,7 +22,7 @@ bool launch_fwd_cols_k2(int set, const ProdArgs& a, int cg, int mr, dim3 grid, s
     }
 #define X(S, MM, CC, RR, KK)                                                                   \
     if (set == S && a.k1 == MM && cg == CC && mr == RR && a.k2 == KK) {                         \
-        launch_pdl(a.chain != 0, k_fwd_cols<S, MM, CC, RR, KK>, grid, col_threads(CC), smem, st, a, batch);        \
+        launch_pdl(a.chain != 0, k_fwd_cols<S, MM, CC, RR, KK>, grid, col_threads(CC, MM), smem, st, a, batch);        \
         return true;                                                                            \
     }
     PREC_COLS_FWD_K2_CONFIGS(X)

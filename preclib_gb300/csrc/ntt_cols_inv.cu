@@ -24,7 +24,7 @@ void launch_inv_cols(int set, const ProdArgs& a, cudaStream_t st, const ProdPtrs
     }
 #define X(S, MM, CC, RR)                                                     \
     if (set == S && a.k1 == MM && cg == CC && mr == RR) {                     \
-        launch_pdl(a.chain != 0, k_inv_cols<S, MM, CC, RR>, grid, 32 * CC, smem, st, a, batch); \
+        launch_pdl(a.chain != 0, k_inv_cols<S, MM, CC, RR>, grid, col_threads(CC, MM), smem, st, a, batch); \
         count_launches(1);                                                  \
         return;                                                             \
     }

@@ -9,7 +9,7 @@ bool launch_inv_cols_k2(int set, const ProdArgs& a, int cg, int mr, dim3 grid, s
                         const ProdPtrs* batch) {
 #define X(S, MM, CC, RR, KK)                                                                   \
     if (set == S && a.k1 == MM && cg == CC && mr == RR && a.k2 == KK) {                         \
-        launch_pdl(a.chain != 0, k_inv_cols<S, MM, CC, RR, KK>, grid, col_threads(CC), smem, st, a, batch);        \
+        launch_pdl(a.chain != 0, k_inv_cols<S, MM, CC, RR, KK>, grid, col_threads(CC, MM), smem, st, a, batch);        \
         return true;                                                                            \
     }
     PREC_COLS_INV_K2_CONFIGS(X)

@@ -18,17 +18,22 @@
 #ifndef PREC_ROWS_MINB
 #define PREC_ROWS_MINB 3
 #endif
-// column kernels: 4 CTAs (64 registers) unless a radix-64 pass of a
-// 2^11-point column holds 64 values per thread (3 CTAs, 85 registers: at 64
-// those kernels spill 300-450 bytes)
-#ifndef PREC_COLS_MINB
-#define PREC_COLS_MINB 4
+// Column kernels: 128 threads and 6 resident CTAs (85 registers; shared
+// memory takes no more tiles of 8192 points), 256 threads and 3 CTAs from
+// 2^11-point columns on (tiles of 16384 points and more; at 64 registers a
+// radix-64 pass spills 300-450 bytes).  Six half-size CTAs mix their phases --
+// staging, passes, stores -- better than four of 256 threads: 4096 products
+// of 200 .. 65536 limbs 9.03 -> 8.65 ms, 4M x 4M limbs 684 -> 671 us, 262144 x
+// 262144 51.7 -> 47.6.  64 threads with tiles of 4096 points: 9.18 ms.
+#ifndef PREC_COLS_THREADS
+#define PREC_COLS_THREADS 128
 #endif
-#ifndef PREC_COLS_MINB_R64
-#define PREC_COLS_MINB_R64 3
-#endif
-__host__ __device__ constexpr int cols_minb(int m, int mr) {
-    return m >= 11 && mr == 6 ? PREC_COLS_MINB_R64 : PREC_COLS_MINB;
+// threads of a column CTA of cg columns of 2^m points
+__host__ __device__ constexpr int col_threads(int cg, int m) {
+    return cg < 8 ? 32 * cg : (m >= 11 ? 256 : PREC_COLS_THREADS);
+}
+__host__ __device__ constexpr int cols_minb(int m, int mr, int cg) {
+    return (m >= 11 && mr == 6 ? 768 : (m >= 11 ? 1024 : 6 * PREC_COLS_THREADS)) / col_threads(cg, m);
 }
 // unroll factor of the item loops of the shared-memory passes
 #ifndef PREC_PASS_UNROLL
