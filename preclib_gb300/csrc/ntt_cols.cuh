@@ -91,88 +91,6 @@ __global__ void __launch_bounds__(col_threads(C, M), cols_minb(M, MR, C)) k_fwd_
 #undef PREC_TILE_PRODUCT
 }
 
-// The forward column pass of one prime of a 64-bit-digit product, software
-// pipelined: each CTA takes every gridDim.x-th column group of its (prime,
-// operand) and stages the next group's limbs into a second tile buffer while
-// it transforms the current one.  The single product's per-prime chains
-// launch it (five launches side by side) for the 1M x 1M class: there it
-// measured 0.1782 -> 0.1741-0.1751 ms, and with both kernels compiled for
-// the constant row length 0.1690 -> 0.1672 ms (2 or 4 tiles per CTA: 0.1679,
-// 0.1685-0.1692).  As one launch over all primes the one-tile kernel stays
-// faster (71 against 77 us), and on set 3's 4M x 4M it measured slower.
-constexpr int kFwdPipeTiles = 3;  // column groups per CTA
-template <int SET, int M, int C, int MR, int K2>
-__global__ void __launch_bounds__(256, 3) k_fwd_cols_pipe(ProdArgs args, const ProdPtrs* __restrict__ batch) {
-    static_assert(set_wide(SET), "64-bit digits: whole limbs staged");
-    static_assert(K2 > 0, "a constant row length");
-    extern __shared__ uint32_t sm[];
-    pdl_enter();
-    constexpr int NP = sch_np(M, MR);
-    constexpr int TW = C * astride_for(M);  // words per tile buffer
-    const ProdPtrs P = select_product(args, batch);
-    const bool one = args.square || args.operand_only;
-    const int prime = args.prime0 + (one ? blockIdx.y : blockIdx.y >> 1);
-    const int operand = args.operand_only ? args.operand_only - 1 : (one ? 0 : blockIdx.y & 1);
-    const PrimeC pc = args.f.pc[prime];
-    const uint2* __restrict__ tw = args.f.tf[prime];
-    constexpr uint32_t N2 = 1u << K2;
-    constexpr int KK = M + K2;  // log2 of the transform length
-    constexpr int nbx = (int)(N2 / C);
-    const uint64_t nl = operand ? P.lb : P.la;
-    if (nl > (1ull << (KK - 1))) {  // the plan puts both operands in the lower half
-        if (threadIdx.x == 0) atomicOr(args.err, kDevErrPlan);
-        return;
-    }
-    const uint64_t* src = operand ? P.b : P.a;
-    uint32_t* __restrict__ dst = P.work + ((uint64_t)(prime * 2 + operand) << KK);
-    uint32_t* cur = sm;
-    uint32_t* nxt = sm + TW;
-    int bx = blockIdx.x;
-    if (bx < nbx) stage_limbs_issue<M, C>(cur, src, N2, (uint64_t)bx * C, nl);
-    for (; bx < nbx; bx += gridDim.x) {
-        const int bn = bx + gridDim.x;
-        if (bn < nbx) {
-            stage_limbs_issue<M, C>(nxt, src, N2, (uint64_t)bn * C, nl);
-            cp_async_wait<1>();  // this tile's group done, the next one in flight
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
-        // the carry kernel's look-back words start at zero
-        if (blockIdx.y == 0 && args.prime0 == 0) {
-            for (int i = bx * blockDim.x + threadIdx.x; i <= P.nblk; i += nbx * blockDim.x) P.scratch[i] = 0;
-        }
-        const uint32_t c0 = (uint32_t)bx * C;
-        col_top_upper_zero<SET, M, C, MR>(cur, tw, pc);
-        __syncthreads();
-        col_passes<SET, M, 1, NP - 2, false, C, MR>(cur, tw, pc);
-        {   // bottom pass with the four-step twiddle, straight to HBM
-            using G = Geom<M, NP - 1, MR>;
-            static_assert(G::LO == 0 && G::RB == 5, "bottom pass covers bits 0..4");
-            const double ip = 4294967296.0 / (double)pc.p;  // 2^32 / p for twiddle32_shoup
-            for (int w = threadIdx.x; w < (C << G::LGI); w += blockDim.x) {
-                const int col = w & (C - 1);
-                const uint32_t u = w / C;
-                const uint32_t* s = cur + (33 * u) * C + col;
-                const uint32_t i2 = c0 + col;
-                const uint32_t t = fourstep_twiddle<SET>(args.f, prime, i2 * brev_bits(u, M - 5), KK);
-                const uint32_t g = fourstep_twiddle<SET>(args.f, prime, i2 << (M - 5), KK);
-                uint32_t x[1][32];
-#pragma unroll
-                for (int q = 0; q < 32; ++q) x[0][q] = s[q * C];
-                regs_pass<SET, M, NP - 1, false, 1, MR>(x, u, tw, pc);
-                twiddle32_shoup<SET>(x[0], t, g, pc, ip);
-#pragma unroll
-                for (int q = 0; q < 32; ++q) dst[(uint64_t)(32 * u + q) * N2 + i2] = x[0][q];
-            }
-        }
-        __syncthreads();  // every thread is done with `cur` before it is refilled
-        uint32_t* t = cur;
-        cur = nxt;
-        nxt = t;
-    }
-}
-
 // One tile of the forward column pass at the indices ix (a persistent kernel's).
 template <int SET, int M, int C, int MR>
 __device__ __forceinline__ void fwd_cols_tile(const ProdArgs& args, const ProdPtrs* __restrict__ batch,
@@ -288,9 +206,8 @@ inline size_t col_smem(int m, int cg) { return (size_t)cg * astride_for(m) * siz
 
 // the K2 instantiations (ntt_cols_fwd_k2.cu, ntt_cols_inv_k2.cu): launch the
 // one matching (set, a.k1, cg, mr, a.k2) and return true, or return false.
-// one_prime: a single product's launch for one prime (the per-prime chains)
 bool launch_fwd_cols_k2(int set, const ProdArgs& a, int cg, int mr, dim3 grid, size_t smem, cudaStream_t st,
-                        const ProdPtrs* batch, bool one_prime);
+                        const ProdPtrs* batch);
 bool launch_inv_cols_k2(int set, const ProdArgs& a, int cg, int mr, dim3 grid, size_t smem, cudaStream_t st,
                         const ProdPtrs* batch);
 int configure_fwd_cols_k2();

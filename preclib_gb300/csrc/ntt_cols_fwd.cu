@@ -17,7 +17,7 @@ void launch_fwd_cols(int set, const ProdArgs& a, cudaStream_t st, const ProdPtrs
         count_launches(1);
         return;
     }
-    if (launch_fwd_cols_k2(set, a, cg, mr, grid, smem, st, batch, nprimes == 1)) {
+    if (launch_fwd_cols_k2(set, a, cg, mr, grid, smem, st, batch)) {
         count_launches(1);
         return;
     }

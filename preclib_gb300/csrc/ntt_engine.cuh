@@ -412,24 +412,6 @@ __device__ __forceinline__ void stage_limbs(uint32_t* sm, const uint64_t* __rest
     cp_async_wait<0>();
 }
 
-// stage_limbs without the wait: the copies of one tile as one committed
-// group, left in flight (the pipelined forward columns prefetch the next tile)
-template <int M, int C>
-__device__ __forceinline__ void stage_limbs_issue(uint32_t* sm, const uint64_t* __restrict__ g, uint64_t ld,
-                                                  uint64_t c0, uint64_t valid) {
-    constexpr int H = 1 << (M - 1);
-    const uint32_t* __restrict__ g32 = reinterpret_cast<const uint32_t*>(g);
-    for (int w = threadIdx.x; w < H * C; w += blockDim.x) {
-        const int r = w / C, col = w % C;
-        const uint64_t idx = (uint64_t)r * ld + c0 + col;
-        const bool in = idx < valid;
-        const uint32_t* src = in ? g32 + 2 * idx : g32;  // 0 bytes read (zero fill) past the operand
-        cp_async4(sm + padded(r) * C + col, src, in ? 4 : 0);
-        cp_async4(sm + padded(r + H) * C + col, in ? src + 1 : g32, in ? 4 : 0);
-    }
-    cp_async_commit();
-}
-
 template <int M, int C>
 __device__ __forceinline__ void stage_cols(uint32_t* sm, const uint32_t* __restrict__ g, uint64_t ld, uint64_t c0,
                                            uint64_t valid) {
@@ -510,29 +492,6 @@ __device__ __forceinline__ void twiddle32(uint32_t (&x)[32], uint32_t t, uint32_
         const int q = brev5(j);
         x[q] = Ar<SET>::mul(x[q], t, pc);
         if (j < 31) t = Ar<SET>::mul(t, g, pc);
-    }
-}
-
-// twiddle32 with the chain's step t*g as a Shoup product (one high and two
-// low products instead of Montgomery's two wide and one low): g goes to
-// plain form below p, and its quotient floor(g 2^32 / p) comes from the
-// double estimate g * ip (ip = 2^32 / p; error far below 1) and one
-// correction.  Used by the pipelined forward columns (1M x 1M 0.1679 ->
-// 0.1661-0.1675 ms); in the other column kernels it measured slower (the
-// inverse kernels spilled 16-20 bytes more).
-template <int SET>
-__device__ __forceinline__ void twiddle32_shoup(uint32_t (&x)[32], uint32_t t, uint32_t g, const PrimeC& pc,
-                                                double ip) {
-    const uint32_t gp = red1(mont_lazy(g, 1u, pc), pc.p);
-    uint32_t gq = (uint32_t)((double)gp * ip);
-    const int64_t r = (int64_t)((uint64_t)gp << 32) - (int64_t)((uint64_t)gq * pc.p);
-    if (r < 0) --gq;
-    else if (r >= (int64_t)pc.p) ++gq;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-        const int q = brev5(j);
-        x[q] = Ar<SET>::mul(x[q], t, pc);
-        if (j < 31) t = shoup_lazy(t, gp, gq, pc.p);
     }
 }
 
