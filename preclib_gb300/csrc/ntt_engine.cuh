@@ -495,6 +495,26 @@ __device__ __forceinline__ void twiddle32(uint32_t (&x)[32], uint32_t t, uint32_
     }
 }
 
+// twiddle32 with the chain's step t*g as a Shoup product (one high and two
+// low products instead of Montgomery's two wide and one low): g goes to
+// plain form below p, and its quotient floor(g 2^32 / p) comes from
+// floor(2^61 / p), at most 2 below, and two corrections.  p in (2^29, 2^30).
+// 4096 products of 200 .. 65536 limbs 8.66 -> 8.53 ms, 1M x 1M limbs 157.6 -> 156.6 us.
+template <int SET>
+__device__ __forceinline__ void twiddle32_shoup(uint32_t (&x)[32], uint32_t t, uint32_t g, const PrimeC& pc) {
+    const uint32_t gp = red1(mont_lazy(g, 1u, pc), pc.p);
+    uint32_t gq = (uint32_t)((uint64_t)gp * pc.c61 >> 29);
+    uint32_t r = 0u - gq * pc.p;  // g 2^32 - gq p, below 3p < 2^32
+    if (r >= pc.p) r -= pc.p, ++gq;
+    if (r >= pc.p) ++gq;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+        const int q = brev5(j);
+        x[q] = Ar<SET>::mul(x[q], t, pc);
+        if (j < 31) t = shoup_lazy(t, gp, gq, pc.p);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // CRT and carries
 // ---------------------------------------------------------------------------

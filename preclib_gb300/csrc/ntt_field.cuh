@@ -71,6 +71,7 @@ struct PrimeC {
     uint32_t p2;      // 2p
     uint32_t r32;     // 2^32 mod p
     uint32_t r32p;    // its Shoup constant floor(r32 * 2^32 / p)
+    uint32_t c61;     // floor(2^61 / p) for p > 2^29 (else 0)
     uint32_t q4, q4p; // 1 / (4 w_4) mod p and its Shoup constant (w_4: the set's root of order 4)
 };
 

@@ -105,6 +105,7 @@ PrimeC prime_constants(uint32_t p) {
     pc.p2 = 2 * p;
     pc.r32 = (uint32_t)((1ull << 32) % p);
     pc.r32p = (uint32_t)(((uint64_t)pc.r32 << 32) / p);
+    pc.c61 = p >> 29 ? (uint32_t)((1ull << 61) / p) : 0;
     pc.q4 = pc.q4p = 0;  // needs the set's root: build_tables
     return pc;
 }
