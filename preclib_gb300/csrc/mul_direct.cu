@@ -102,7 +102,8 @@ __device__ __forceinline__ void group_sync() {
 }
 
 template <int R, int G>
-__global__ void __launch_bounds__(DirectGeom<R, G>::THREADS) k_direct(const SmallDesc* __restrict__ descs, int count) {
+__global__ void __launch_bounds__(DirectGeom<R, G>::THREADS) k_direct(const DirectItem* __restrict__ items, int count,
+                                                                   int cls) {
     using D = DirectGeom<R, G>;
     constexpr int S = Blk<R>::S;
     extern __shared__ __align__(16) uint32_t dsm[];
@@ -111,12 +112,14 @@ __global__ void __launch_bounds__(DirectGeom<R, G>::THREADS) k_direct(const Smal
     pdl_next();
     const int sub = threadIdx.x / G;
     const int item = blockIdx.x * D::PER_CTA + sub;
-    const bool live = item < count;  // a group past the end runs an empty product
+    // a group past the end, or with a product of another class, runs an empty product
+    const DirectItem d = items[item < count ? item : count - 1];
+    const bool live = item < count && direct_class(d.la, d.lb) == cls;
+    if (G <= 32 ? !__any_sync(0xffffffffu, live) : !live) return;
     const int g = threadIdx.x & (G - 1);
     uint32_t* sa = dsm + sub * D::WORDS;  // block i of a at (i + 1) * S
     uint32_t* sb = sa + D::A_BLKS * S;
     uint32_t* cols = sb + D::B_BLKS * S;
-    const SmallDesc& d = descs[live ? item : count - 1];
     const bool swap = d.la < d.lb;
     const uint64_t* __restrict__ pa = swap ? d.b : d.a;
     const uint64_t* __restrict__ pb = swap ? d.a : d.b;
@@ -206,26 +209,12 @@ __global__ void __launch_bounds__(DirectGeom<R, G>::THREADS) k_direct(const Smal
 // (class, R, G): the longer operand up to R G / 2 limbs
 #define PREC_DIRECT(X) X(0, 8, 16) X(1, 8, 32) X(2, 8, 64) X(3, 8, 128)
 
-// Direct where it measured below the single-CTA transform (ns per product of
-// a large batch, direct / transform, equal operands of n limbs): 16: 1.2 / 18.7,
-// 32: 1.8 / 18.8, 64: 3.2 / 21.0, 96: 8.9 / 23.5, 128: 11.3 / 24.6,
-// 192: 29.1 / 27.8, 256: 37.1 / 29.0, 512: 139 / 70.  The direct time goes
-// with the shorter operand, the transform's with the sum: operands up to 256
-// limbs cross near 180 x 180 limbs, operands up to 512 limbs at a shorter
-// one of about 100 limbs (27 ns against 29 of the 2^10-point transform).
-int direct_class(uint64_t la, uint64_t lb) {
-    const uint64_t hi = la > lb ? la : lb, lo = la > lb ? lb : la;
-    if (hi <= 64) return 0;
-    if (hi <= 128) return 1;
-    if (hi <= 256) return lo <= 160 ? 2 : -1;
-    return hi <= kDirectBatchMax && lo <= 96 ? 3 : -1;
-}
-
-void launch_direct_batch(const SmallDesc* d_descs, int count, int cls, cudaStream_t st) {
+void launch_direct_batch(const DirectItem* d_items, int count, int cls, cudaStream_t st) {
 #define X(C, R, G)                                                                                              \
     if (cls == C) {                                                                                             \
         using D = DirectGeom<R, G>;                                                                             \
-        launch_pdl(false, k_direct<R, G>, (count + D::PER_CTA - 1) / D::PER_CTA, D::THREADS, D::SMEM, st, d_descs, count); \
+        launch_pdl(false, k_direct<R, G>, (count + D::PER_CTA - 1) / D::PER_CTA, D::THREADS, D::SMEM, st, d_items, count, \
+                   cls);                                                                                        \
         count_launches(1);                                                                                      \
     }
     PREC_DIRECT(X)

@@ -17,14 +17,40 @@ constexpr uint64_t kDirectBatchMax = 512;
 // single product over the whole GPU: longer operand up to kDirectGridMax limbs
 constexpr uint64_t kDirectGridMax = 4096;
 
-// class of a batch product, or -1: the transform is faster (see the rule)
-int direct_class(uint64_t la, uint64_t lb);
+// One product of a batch: the layout of prec_gpu_product_t, so that a batch of
+// direct products alone takes the caller's array as it is.
+struct DirectItem {
+    const uint64_t* a;
+    uint64_t la;
+    const uint64_t* b;
+    uint64_t lb;
+    uint64_t* out;
+};
+
+// Class of a batch product, or -1: the transform is faster (or an operand is
+// empty).  Direct where it measured below the single-CTA transform (ns per
+// product of a large batch, direct / transform, equal operands of n limbs):
+// 16: 1.2 / 18.7, 32: 1.8 / 18.8, 64: 3.2 / 21.0, 96: 8.9 / 23.5, 128: 11.3 /
+// 24.6, 192: 29.1 / 27.8, 256: 37.1 / 29.0, 512: 139 / 70.  The direct time
+// goes with the shorter operand, the transform's with the sum: operands up to
+// 256 limbs cross near 180 x 180 limbs, operands up to 512 limbs at a
+// shorter one of about 100 limbs (27 ns against 29 of the 2^10-point
+// transform).
+__host__ __device__ inline int direct_class(uint64_t la, uint64_t lb) {
+    const uint64_t hi = la > lb ? la : lb, lo = la > lb ? lb : la;
+    if (lo == 0) return -1;
+    if (hi <= 64) return 0;
+    if (hi <= 128) return 1;
+    if (hi <= 256) return lo <= 160 ? 2 : -1;
+    return hi <= kDirectBatchMax && lo <= 96 ? 3 : -1;
+}
 // whether a single device product runs directly
 bool direct_single(uint64_t la, uint64_t lb);
 // scratch bytes of a single direct product (column sums)
 size_t direct_scratch_bytes(uint64_t la, uint64_t lb);
 
-void launch_direct_batch(const SmallDesc* d_descs, int count, int cls, cudaStream_t st);
+// the products of class `cls` among `count` items (others are passed over)
+void launch_direct_batch(const DirectItem* d_items, int count, int cls, cudaStream_t st);
 // counter: one device word, zero before the first call, left zero by every
 // call; calls that share it must not overlap
 void launch_direct_single(const uint64_t* a, uint64_t la, const uint64_t* b, uint64_t lb, uint64_t* out,

@@ -47,7 +47,8 @@ struct Cls {
     size_t ws_per = 0;            // workspace bytes per product (four-step)
     int per_chunk = 0;            // products per chunk
     std::vector<Chunk> chunks;
-    SmallDesc* d_small = nullptr; // device descriptors (direct and single-CTA classes)
+    SmallDesc* d_small = nullptr; // device descriptors (single-CTA classes)
+    DirectItem* d_direct = nullptr; // device descriptors (direct classes)
     ProdPtrs* d_ptrs = nullptr;   // device descriptors (four-step classes)
     uint8_t* ws = nullptr;        // workspace of one chunk
     bool persistent = false;      // one persistent kernel per chunk (ntt_class.cu)
@@ -80,6 +81,10 @@ struct prec_gpu_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     uint64_t graph_launches = 0;  // kernels in the recorded graph
+    // every product direct (or empty): the caller's items as they are, one
+    // launch per class of direct_mask over all of them
+    size_t direct_count = 0;
+    uint32_t direct_mask = 0;
     int* err = nullptr;
     uint32_t spin_limit = 0;      // persistent class kernels: polls per dependency wait
     int never_signal = 0;         // tests: their forward tiles never complete a counter
@@ -124,11 +129,14 @@ static void batch_enqueue(prec_gpu_batch* b, cudaStream_t origin, bool branch) {
         if (rec) rec->add_memset(p.out, (p.an + p.bn) * sizeof(uint64_t), origin);
         else cudaMemsetAsync(p.out, 0, (p.an + p.bn) * sizeof(uint64_t), origin);
     }
+    for (int k = 0; k < kDirectClasses; ++k)
+        if (b->direct_mask >> k & 1)
+            launch_direct_batch(static_cast<const DirectItem*>(b->d_mem), (int)b->direct_count, k, origin);
     for (Cls& c : b->classes) {
         cudaStream_t st = branch ? c.stream : origin;
         if (branch && !rec) cudaStreamWaitEvent(st, b->fork, 0);
         if (c.direct >= 0) {
-            launch_direct_batch(c.d_small, (int)c.items.size(), c.direct, st);
+            launch_direct_batch(c.d_direct, (int)c.items.size(), c.direct, st);
         } else if (c.pl.path == 0) {
             ntt_launch_small(c.d_small, nullptr, (int)c.items.size(), c.k, ctx_field(0), c.pl.crt, st);
         } else {
@@ -223,8 +231,41 @@ static int batch_build(const prec_gpu_product_t* items, size_t count, bool onesh
     if (r) return r;
     prec_gpu_batch* b = new prec_gpu_batch();
     b->oneshot = ost;
-    b->items.assign(items, items + count);
     b->err = ctx_device_err();
+    // all of them direct products (the low levels of a product tree): no
+    // descriptors are built, the kernels find their class's products
+    static_assert(sizeof(DirectItem) == sizeof(prec_gpu_product_t), "same layout");
+    size_t n_zero = 0;
+    uint32_t mask = 0;
+    size_t i0 = 0;
+    for (; i0 < count; ++i0) {
+        const prec_gpu_product_t& p = items[i0];
+        if (p.an == 0 || p.bn == 0) {
+            ++n_zero;
+            continue;
+        }
+        const int k = p.a && p.b && p.out ? direct_class(p.an, p.bn) : -1;
+        if (k < 0) break;
+        mask |= 1u << k;
+    }
+    if (i0 == count && mask && n_zero == 0 && count <= 0x7fffffff) {
+        b->direct_count = count;
+        b->direct_mask = mask;
+        b->d_bytes = count * sizeof(DirectItem);
+        if (oneshot) {
+            BCK(cudaMallocFromPoolAsync(&b->d_mem, b->d_bytes, ctx_pool(), ost));
+            b->pooled = true;
+            BCK(cudaMemcpyAsync(b->d_mem, items, b->d_bytes, cudaMemcpyHostToDevice, ost));
+        } else {
+            BCK(cudaMalloc(&b->d_mem, b->d_bytes));
+            BCK(cudaMemcpy(b->d_mem, items, b->d_bytes, cudaMemcpyHostToDevice));
+            BCK(cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking));
+            BCK(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+        }
+        *out = b;
+        return PREC_GPU_OK;
+    }
+    b->items.assign(items, items + count);
     // classes by key ((eighths of the transform - 5) << 9 | 64-bit digits << 8
     // | k << 1 | square, or the direct form's class past those): a dense
     // table, not a map lookup per product (a binary-splitting level has ~10^6
@@ -318,7 +359,7 @@ static int batch_build(const prec_gpu_product_t* items, size_t count, bool onesh
         Cls& c = found[ci];
         const size_t n = c.items.size();
         desc_off.push_back(bytes);
-        bytes += align256(n * (c.pl.path == 0 ? sizeof(SmallDesc) : sizeof(ProdPtrs)));
+        bytes += align256(n * (c.direct >= 0 ? sizeof(DirectItem) : c.pl.path == 0 ? sizeof(SmallDesc) : sizeof(ProdPtrs)));
         if (c.pl.path == 1) {
             // a product of 2^k points has at most 2^(k-1) + 1 limbs on 32-bit
             // digits, 2^k + 1 on 64-bit digits
@@ -352,7 +393,15 @@ static int batch_build(const prec_gpu_product_t* items, size_t count, bool onesh
     for (size_t ci = 0; ci < b->classes.size(); ++ci) {
         Cls& c = b->classes[ci];
         const size_t n = c.items.size();
-        if (c.pl.path == 0) {
+        if (c.direct >= 0) {
+            std::vector<DirectItem> h(n);
+            for (size_t j = 0; j < n; ++j) {
+                const prec_gpu_product_t& p = items[c.items[j]];
+                h[j] = DirectItem{p.a, p.an, p.b, p.bn, p.out};
+            }
+            c.d_direct = reinterpret_cast<DirectItem*>(base + desc_off[ci]);
+            BCK(upload(c.d_direct, h.data(), n * sizeof(DirectItem)));
+        } else if (c.pl.path == 0) {
             std::vector<SmallDesc> h(n);
             for (size_t j = 0; j < n; ++j) {
                 const prec_gpu_product_t& p = items[c.items[j]];
@@ -445,7 +494,7 @@ int prec_gpu_batch_run(prec_gpu_batch_t* b, void* stream) {
 
 int prec_gpu_batch_info(const prec_gpu_batch_t* b, size_t* classes, size_t* device_bytes) {
     if (!b) return PREC_GPU_E_ARG;
-    if (classes) *classes = b->classes.size();
+    if (classes) *classes = b->classes.size() + __builtin_popcount(b->direct_mask);
     if (device_bytes) *device_bytes = b->d_bytes;
     return PREC_GPU_OK;
 }
