@@ -17,7 +17,7 @@
 // What bounds it: the 32x32->64-bit multiply-add, one per digit pair; 8192
 // products of 512 x 512 limbs reach 7.5 T multiply-adds/s, 40000 of 64 x 64
 // limbs 5.2 T/s (there the flushes and the carry stage show).  44643 products of
-// 58 .. 66 limbs: kernels 0.98 -> 0.14 ms against the single-CTA transform.
+// 58 .. 66 limbs: kernels 0.98 -> 0.18 ms against the single-CTA transform.
 // A single product is bound by latency instead: launch, two trips to L2 and
 // the carries of the last CTA; 1024 x 1000 limbs 28.7 -> 8.1 us.
 #include "mul_direct.cuh"
@@ -39,7 +39,8 @@ __device__ __forceinline__ void mac96(uint32_t& lo, uint32_t& mid, uint32_t& hi,
 // loads of consecutive blocks by consecutive lanes free of bank conflicts
 template <int R>
 struct Blk {
-    static constexpr int S = R == 4 ? 4 : R + 4;
+    static constexpr int S = R == 8 ? 12 : R;  // (12 words: 8 lanes cover the 32 banks once)
+    static_assert(S == 12, "bank-conflict-free strides");
     static __device__ __forceinline__ void load(uint32_t (&x)[R], const uint32_t* p) {
 #pragma unroll
         for (int h = 0; h < R / 4; ++h) {
@@ -101,121 +102,151 @@ __device__ __forceinline__ void group_sync() {
     else __syncthreads();
 }
 
+// Classes by list: a warp's lanes of one class take their places together.
+// (With every class's launch going over all items, mostly empty groups kept
+// the shared memory of half-empty CTAs: 44643 products of 58 .. 66 limbs,
+// two classes, 299 us of kernels; with lists 175.)
+__global__ void __launch_bounds__(256) k_direct_lists(const DirectItem* __restrict__ items, int count, uint32_t* lists,
+                                                      uint32_t* n) {
+    pdl_enter();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const int cls = i < count ? direct_class(items[i].la, items[i].lb) : -1;
+    const uint32_t same = __match_any_sync(0xffffffffu, cls);
+    const int leader = __ffs(same) - 1;
+    uint32_t at = 0;
+    if (cls >= 0 && lane == leader) at = atomicAdd(&n[cls], (uint32_t)__popc(same));
+    at = __shfl_sync(0xffffffffu, at, leader) + __popc(same & ((1u << lane) - 1));
+    if (cls >= 0) lists[(size_t)cls * count + at] = i;
+}
+
 template <int R, int G>
 __global__ void __launch_bounds__(DirectGeom<R, G>::THREADS) k_direct(const DirectItem* __restrict__ items, int count,
-                                                                   int cls) {
+                                                                   const uint32_t* __restrict__ list,
+                                                                   const uint32_t* n) {
     using D = DirectGeom<R, G>;
     constexpr int S = Blk<R>::S;
     extern __shared__ __align__(16) uint32_t dsm[];
     __shared__ BlockCarryShared sh;
     pdl_enter();
     pdl_next();
+    if (n) count = (int)*after_entry(n);
+    list = after_entry(list);
     const int sub = threadIdx.x / G;
-    const int item = blockIdx.x * D::PER_CTA + sub;
-    // a group past the end, or with a product of another class, runs an empty product
-    const DirectItem d = items[item < count ? item : count - 1];
-    const bool live = item < count && direct_class(d.la, d.lb) == cls;
-    if (G <= 32 ? !__any_sync(0xffffffffu, live) : !live) return;
     const int g = threadIdx.x & (G - 1);
     uint32_t* sa = dsm + sub * D::WORDS;  // block i of a at (i + 1) * S
     uint32_t* sb = sa + D::A_BLKS * S;
     uint32_t* cols = sb + D::B_BLKS * S;
-    const bool swap = d.la < d.lb;
-    const uint64_t* __restrict__ pa = swap ? d.b : d.a;
-    const uint64_t* __restrict__ pb = swap ? d.a : d.b;
-    const int la = live ? (int)(swap ? d.lb : d.la) : 0, lb = live ? (int)(swap ? d.la : d.lb) : 0;
-    const int na = (2 * la + R - 1) / R, nb = (2 * lb + R - 1) / R;  // digit blocks
-    for (int i = g; i < na * (R / 2); i += G) Blk<R>::put(sa + S, i, i < la ? __ldg(&pa[i]) : 0ull);
-    for (int i = g; i < (nb + 1) * (R / 2); i += G) Blk<R>::put(sb, i, i < lb ? __ldg(&pb[i]) : 0ull);
-    if (g < R) {
-        sa[g] = 0;
-        sa[(na + 1) * S + g] = 0;
-    }
-    group_sync<G>();
-
-    const bool active = g < na;
-    const int c = g;  // column block
-    if (active) {
-        Acc<R> acc;
-        acc.zero();
-        auto flush = [&](int blk) {
-            uint32_t* p = cols + blk * (R + 1);
-#pragma unroll
-            for (int k = 0; k < 3; ++k)
-#pragma unroll
-                for (int r = 0; r < R; ++r) p[k * D::PCOLS + r] = acc.w[k][r];
-        };
-        uint32_t upper[R];
-        Blk<R>::load(upper, sa + (c + 1) * S);
-        int jb = 0, ab = c;
-        bool high = false;
-        for (int t = 0; t <= nb; ++t) {
-            if (t == c + 1) {  // from column block c to block c + na
-                flush(c);
-                acc.zero();
-                high = true;
-                jb = c;
-                ab = na;
-#pragma unroll
-                for (int r = 0; r < R; ++r) upper[r] = 0;
-            }
-            uint32_t lower[R], y[R];
-            Blk<R>::load(lower, sa + ab * S);  // block ab - 1
-            Blk<R>::load(y, sb + jb * S);
-            acc.step(lower, upper, y);
-#pragma unroll
-            for (int r = 0; r < R; ++r) upper[r] = lower[r];
-            ++jb;
-            --ab;
+    for (int base = blockIdx.x * D::PER_CTA; base < count; base += gridDim.x * D::PER_CTA) {
+        const bool live = base + sub < count;  // a group past the end runs an empty product
+        const int at = live ? base + sub : count - 1;
+        const DirectItem d = items[list ? list[at] : at];
+        const bool swap = d.la < d.lb;
+        const uint64_t* __restrict__ pa = swap ? d.b : d.a;
+        const uint64_t* __restrict__ pb = swap ? d.a : d.b;
+        const int la = live ? (int)(swap ? d.lb : d.la) : 0, lb = live ? (int)(swap ? d.la : d.lb) : 0;
+        const int na = (2 * la + R - 1) / R, nb = (2 * lb + R - 1) / R;  // digit blocks
+        for (int i = g; i < na * (R / 2); i += G) Blk<R>::put(sa + S, i, i < la ? __ldg(&pa[i]) : 0ull);
+        for (int i = g; i < (nb + 1) * (R / 2); i += G) Blk<R>::put(sb, i, i < lb ? __ldg(&pb[i]) : 0ull);
+        if (g < R) {
+            sa[g] = 0;
+            sa[(na + 1) * S + g] = 0;
         }
-        flush(high ? na + c : c);
-    }
-    group_sync<G>();
+        group_sync<G>();
 
-    // limbs g*R .. g*R + R - 1
-    const int lout = la + lb;
-    const int m0 = g * R;
-    auto col = [&](int i) -> u128 {
-        const uint32_t* p = cols + i + i / R;
-        return ((u128)p[2 * D::PCOLS] << 64) | ((uint64_t)p[D::PCOLS] << 32) | p[0];
-    };
-    u128 T[R];
+        const bool active = g < na;
+        const int c = g;  // column block
+        if (active) {
+            Acc<R> acc;
+            acc.zero();
+            auto flush = [&](int blk) {
+                uint32_t* p = cols + blk * (R + 1);
 #pragma unroll
-    for (int k = 0; k < R; ++k) T[k] = m0 + k < lout ? col(2 * (m0 + k)) + (col(2 * (m0 + k) + 1) << 32) : (u128)0;
-    uint64_t prev_hi = 0;
-    if (g > 0 && m0 - 1 < lout) prev_hi = (uint64_t)((col(2 * m0 - 2) + (col(2 * m0 - 1) << 32)) >> 64);
-    uint64_t v[R];
-    uint32_t gbits;
-    bool cg, cp;
-    limbs_from_sums<R>(T, prev_hi, v, gbits, cg, cp);
-    bool cin;
-    if constexpr (G <= 32) {
-        constexpr uint32_t mask = G == 32 ? 0xffffffffu : (1u << G) - 1;
-        const int sh0 = (threadIdx.x & 31) & ~(G - 1);  // the group's first lane
-        const uint32_t gm = (__ballot_sync(0xffffffffu, cg) >> sh0) & mask;
-        const uint32_t pm = (__ballot_sync(0xffffffffu, cp) >> sh0) & mask;
-        cin = (carry_chain(gm, pm, false) >> g) & 1;
-        __syncwarp();
-    } else {
-        cin = block_carry(cg, cp, sh, [](bool, bool) { return false; });
+                for (int k = 0; k < 3; ++k)
+#pragma unroll
+                    for (int r = 0; r < R; ++r) p[k * D::PCOLS + r] = acc.w[k][r];
+            };
+            uint32_t upper[R];
+            Blk<R>::load(upper, sa + (c + 1) * S);
+            int jb = 0, ab = c;
+            bool high = false;
+            for (int t = 0; t <= nb; ++t) {
+                if (t == c + 1) {  // from column block c to block c + na
+                    flush(c);
+                    acc.zero();
+                    high = true;
+                    jb = c;
+                    ab = na;
+#pragma unroll
+                    for (int r = 0; r < R; ++r) upper[r] = 0;
+                }
+                uint32_t lower[R], y[R];
+                Blk<R>::load(lower, sa + ab * S);  // block ab - 1
+                Blk<R>::load(y, sb + jb * S);
+                acc.step(lower, upper, y);
+#pragma unroll
+                for (int r = 0; r < R; ++r) upper[r] = lower[r];
+                ++jb;
+                --ab;
+            }
+            flush(high ? na + c : c);
+        }
+        group_sync<G>();
+
+        // limbs g*R .. g*R + R - 1
+        const int lout = la + lb;
+        const int m0 = g * R;
+        auto col = [&](int i) -> u128 {
+            const uint32_t* p = cols + i + i / R;
+            return ((u128)p[2 * D::PCOLS] << 64) | ((uint64_t)p[D::PCOLS] << 32) | p[0];
+        };
+        u128 T[R];
+#pragma unroll
+        for (int k = 0; k < R; ++k) T[k] = m0 + k < lout ? col(2 * (m0 + k)) + (col(2 * (m0 + k) + 1) << 32) : (u128)0;
+        uint64_t prev_hi = 0;
+        if (g > 0 && m0 - 1 < lout) prev_hi = (uint64_t)((col(2 * m0 - 2) + (col(2 * m0 - 1) << 32)) >> 64);
+        uint64_t v[R];
+        uint32_t gbits;
+        bool cg, cp;
+        limbs_from_sums<R>(T, prev_hi, v, gbits, cg, cp);
+        bool cin;
+        if constexpr (G <= 32) {
+            constexpr uint32_t mask = G == 32 ? 0xffffffffu : (1u << G) - 1;
+            const int sh0 = (threadIdx.x & 31) & ~(G - 1);  // the group's first lane
+            const uint32_t gm = (__ballot_sync(0xffffffffu, cg) >> sh0) & mask;
+            const uint32_t pm = (__ballot_sync(0xffffffffu, cp) >> sh0) & mask;
+            cin = (carry_chain(gm, pm, false) >> g) & 1;
+            __syncwarp();
+        } else {
+            cin = block_carry(cg, cp, sh, [](bool, bool) { return false; });
+        }
+        // the limbs through shared memory (limb m at m + m / R) to whole-line stores
+        uint64_t* st = reinterpret_cast<uint64_t*>(cols);
+        limbs_finish<R>(m0, (uint64_t)lout, v, gbits, cin, st + g);
+        group_sync<G>();
+        for (int m = g; m < lout; m += G) d.out[m] = st[m + m / R];
+        group_sync<G>();  // the next product's operands
     }
-    // the limbs through shared memory (limb m at m + m / R) to whole-line stores
-    uint64_t* st = reinterpret_cast<uint64_t*>(cols);
-    limbs_finish<R>(m0, (uint64_t)lout, v, gbits, cin, st + g);
-    group_sync<G>();
-    for (int m = g; m < lout; m += G) d.out[m] = st[m + m / R];
 }
 
 // (class, R, G): the longer operand up to R G / 2 limbs
-#define PREC_DIRECT(X) X(0, 8, 16) X(1, 8, 32) X(2, 8, 64) X(3, 8, 128)
+#define PREC_DIRECT(X) X(0, 8, 16) X(1, 12, 16) X(2, 8, 32) X(3, 8, 64) X(4, 8, 128)
 
-void launch_direct_batch(const DirectItem* d_items, int count, int cls, cudaStream_t st) {
-#define X(C, R, G)                                                                                              \
-    if (cls == C) {                                                                                             \
-        using D = DirectGeom<R, G>;                                                                             \
-        launch_pdl(false, k_direct<R, G>, (count + D::PER_CTA - 1) / D::PER_CTA, D::THREADS, D::SMEM, st, d_items, count, \
-                   cls);                                                                                        \
-        count_launches(1);                                                                                      \
+void launch_direct_lists(const DirectItem* d_items, int count, uint32_t* lists, uint32_t* n, cudaStream_t st) {
+    launch_pdl(false, k_direct_lists, (count + 255) / 256, 256, 0, st, d_items, count, lists, n);
+    count_launches(1);
+}
+
+void launch_direct_batch(const DirectItem* d_items, int count, int cls, cudaStream_t st, const uint32_t* list,
+                         const uint32_t* n) {
+    // with a list of unknown length: as many CTAs as stay resident, a few times over
+    const int cap = n ? device_sm_count() * 64 : 0x7fffffff;
+#define X(C, R, G)                                                                                          \
+    if (cls == C) {                                                                                         \
+        using D = DirectGeom<R, G>;                                                                         \
+        const int grid = (count + D::PER_CTA - 1) / D::PER_CTA;                                             \
+        launch_pdl(false, k_direct<R, G>, grid < cap ? grid : cap, D::THREADS, D::SMEM, st, d_items, count, \
+                   list, n);                                                                                \
+        count_launches(1);                                                                                  \
     }
     PREC_DIRECT(X)
 #undef X

@@ -81,10 +81,11 @@ struct prec_gpu_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     uint64_t graph_launches = 0;  // kernels in the recorded graph
-    // every product direct (or empty): the caller's items as they are, one
-    // launch per class of direct_mask over all of them
+    // every product direct: the caller's items as they are and, for more than
+    // one class in direct_mask, the classes' index lists, made on the device
     size_t direct_count = 0;
     uint32_t direct_mask = 0;
+    uint32_t* direct_n = nullptr;  // list lengths, then the lists
     int* err = nullptr;
     uint32_t spin_limit = 0;      // persistent class kernels: polls per dependency wait
     int never_signal = 0;         // tests: their forward tiles never complete a counter
@@ -129,9 +130,20 @@ static void batch_enqueue(prec_gpu_batch* b, cudaStream_t origin, bool branch) {
         if (rec) rec->add_memset(p.out, (p.an + p.bn) * sizeof(uint64_t), origin);
         else cudaMemsetAsync(p.out, 0, (p.an + p.bn) * sizeof(uint64_t), origin);
     }
-    for (int k = 0; k < kDirectClasses; ++k)
-        if (b->direct_mask >> k & 1)
-            launch_direct_batch(static_cast<const DirectItem*>(b->d_mem), (int)b->direct_count, k, origin);
+    if (b->direct_mask) {
+        const DirectItem* d = static_cast<const DirectItem*>(b->d_mem);
+        const int n = (int)b->direct_count;
+        uint32_t* lists = b->direct_n ? b->direct_n + 32 : nullptr;
+        if (lists) {
+            if (rec) rec->add_memset(b->direct_n, kDirectClasses * sizeof(uint32_t), origin);
+            else cudaMemsetAsync(b->direct_n, 0, kDirectClasses * sizeof(uint32_t), origin);
+            launch_direct_lists(d, n, lists, b->direct_n, origin);
+        }
+        for (int k = 0; k < kDirectClasses; ++k)
+            if (b->direct_mask >> k & 1)
+                launch_direct_batch(d, n, k, origin, lists ? lists + (size_t)k * n : nullptr,
+                                    lists ? b->direct_n + k : nullptr);
+    }
     for (Cls& c : b->classes) {
         cudaStream_t st = branch ? c.stream : origin;
         if (branch && !rec) cudaStreamWaitEvent(st, b->fork, 0);
@@ -251,17 +263,20 @@ static int batch_build(const prec_gpu_product_t* items, size_t count, bool onesh
     if (i0 == count && mask && n_zero == 0 && count <= 0x7fffffff) {
         b->direct_count = count;
         b->direct_mask = mask;
-        b->d_bytes = count * sizeof(DirectItem);
+        const size_t item_bytes = align256(count * sizeof(DirectItem));
+        const bool lists = (mask & (mask - 1)) != 0;
+        b->d_bytes = item_bytes + (lists ? (32 + kDirectClasses * count) * sizeof(uint32_t) : 0);
         if (oneshot) {
             BCK(cudaMallocFromPoolAsync(&b->d_mem, b->d_bytes, ctx_pool(), ost));
             b->pooled = true;
-            BCK(cudaMemcpyAsync(b->d_mem, items, b->d_bytes, cudaMemcpyHostToDevice, ost));
+            BCK(cudaMemcpyAsync(b->d_mem, items, count * sizeof(DirectItem), cudaMemcpyHostToDevice, ost));
         } else {
             BCK(cudaMalloc(&b->d_mem, b->d_bytes));
-            BCK(cudaMemcpy(b->d_mem, items, b->d_bytes, cudaMemcpyHostToDevice));
+            BCK(cudaMemcpy(b->d_mem, items, count * sizeof(DirectItem), cudaMemcpyHostToDevice));
             BCK(cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking));
             BCK(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
         }
+        if (lists) b->direct_n = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(b->d_mem) + item_bytes);
         *out = b;
         return PREC_GPU_OK;
     }
