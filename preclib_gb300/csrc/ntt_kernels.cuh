@@ -298,6 +298,11 @@ struct CrtChunks {
 void ntt_launch_4step(int set, const ProdArgs& args, cudaStream_t st, cudaEvent_t* ev = nullptr,
                       const PrimeStreams* ps = nullptr, cudaEvent_t a_ready = nullptr,
                       cudaEvent_t b_ready = nullptr, const CrtChunks* chunks = nullptr);
+// One product of 2^13 .. 2^18 points in a default configuration, by the
+// kernels built for latency (ntt_lat.cu).  lat_keep: the eighths they keep for
+// a product that needs `keep` (0: no such kernels).
+int lat_keep(int set, int k1, int k2, int keep);
+void ntt_launch_lat(int set, const ProdArgs& args, cudaStream_t st, cudaEvent_t* ev = nullptr);
 // the batch form: `count` products of one length class (class-wide fields
 // from `args`, per-product fields from the device array `batch`);
 // max_nblk = the largest carry grid of the class

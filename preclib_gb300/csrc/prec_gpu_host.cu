@@ -703,6 +703,16 @@ static int ensure_io(Lane& L, size_t limbs) {
 // Enqueues one NTT-band product on device pointers.
 // A square (d_a == d_b, la == lb) transforms its one operand only on the
 // four-step path; the single-CTA path reads the operand twice.
+// The eighths kept by the kernels built for latency, which a single product
+// of up to 2^18 points in a default configuration takes; else 0.
+static int plan_latency(const Plan& pl) {
+    if (pl.k > 18) return 0;
+    const KernelConfig d = default_config(pl.k);
+    if (d.k1 != pl.k1 || d.cg != pl.cg || d.cmr != pl.cmr || d.rmr != pl.rmr || d.rows != pl.rows || d.split != pl.split)
+        return 0;
+    return lat_keep(pl.set, pl.k1, pl.k2, pl.keep);
+}
+
 // Device error bits go to `err` (the lane's status block for host
 // products, the library-wide word otherwise).
 static int enqueue_ntt(Ctx& c, Lane& L, const uint64_t* d_a, uint64_t la, const uint64_t* d_b, uint64_t lb,
@@ -747,6 +757,13 @@ static int enqueue_ntt(Ctx& c, Lane& L, const uint64_t* d_a, uint64_t la, const 
         args.crt5 = pl.crt5;
         args.f = c.field[pl.set];
         const bool split = c.split_primes && (pl.split || a_ready);
+        const int lat = split ? 0 : plan_latency(pl);
+        if (lat) {
+            args.keep = lat;
+            ntt_launch_lat(pl.set, args, st, ev);
+            CK(cudaGetLastError());
+            return 0;
+        }
         ntt_launch_4step(pl.set, args, st, ev, split ? &L.prime_streams : nullptr, a_ready, b_ready,
                          split ? chunks : nullptr);
     }
@@ -898,10 +915,9 @@ enum { kModeBands = 0, kModeNtt = 1, kModeFft = 2 };
 // page-locked buffer: the host copies the operands in, the kernels read them
 // and write the result and the status over the host link, the host copies
 // the result out.  No copy engine, no second wait.  Measured per call, with
-// copies and this way: 256 x 193 limbs 66.8 -> 45.5 us, 3000 x 3000 81 -> 60,
-// 8192 x 8192 65.7 -> 47.4, 16384 x 16384 72.7 -> 61.7, 24000 x 20000
-// 74.1 -> 71.7, 32768 x 32768 75.2 -> 94.0: past that the host's own copies
-// cost more than the copy engine's.
+// copies and this way: 4000 x 4000 limbs 61.4 -> 49.3 us, 6500 x 6500 42.9 ->
+// 37.9, 8192 x 8192 49.3 -> 41.1, 12000 x 12000 54.4 -> 48.8, 16384 x 16384 56.2 ->
+// 54.8; past that the host's own copies cost more than the copy engine's.
 constexpr size_t kStagedLimbs = 32768;
 
 // Host products from 2^19 points run per-prime chains even where a device
