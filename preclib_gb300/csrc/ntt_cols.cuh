@@ -34,6 +34,13 @@
 
 namespace precgpu {
 
+// the batch classes' configurations (more than 8 columns per CTA) read their
+// four-step twiddles from a table, one Shoup product per value instead of a
+// Montgomery product and a chain step (a third of the forward pass's
+// multiplier time).  4096 products of 200 .. 65536 limbs 8.52 -> 8.23 ms.  Past
+// 2^19 points the tables no longer stay in L2 beside the residues: 2^20
+// points 86 -> 109 us, 2^21 157 -> 197.
+__host__ __device__ constexpr bool col_table(int cg) { return cg > 8; }
 
 // Top DIF pass of a digit tile whose upper half (rows 2^(M-1) and up) is
 // zero -- every operand of at most N/2 digits, i.e. both operands of a

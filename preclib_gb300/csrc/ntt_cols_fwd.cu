@@ -32,6 +32,37 @@ void launch_fwd_cols(int set, const ProdArgs& a, cudaStream_t st, const ProdPtrs
 #undef X
 }
 
+struct TableArgs {
+    FieldArgs f;
+    uint32_t fold[kMaxPrimes];
+};
+
+__global__ void __launch_bounds__(256) k_fourstep_table(uint2* t4, TableArgs a, int k1, int k2) {
+    const int prime = blockIdx.y, np = gridDim.y, k = k1 + k2;
+    const PrimeC pc = a.f.pc[prime];
+    const uint32_t N = 1u << k;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+        const uint32_t e = (i & ((1u << k2) - 1)) * brev_bits(i >> k2, k1);
+#pragma unroll
+        for (int dir = 0; dir < 2; ++dir) {
+            uint32_t w = fourstep_twiddle<0>(a.f, prime, dir ? (0u - e) & (N - 1) : e, k);
+            if (dir) w = mont_lazy(w, a.fold[prime], pc);
+            w = red1(mont_lazy(w, 1u, pc), pc.p);
+            t4[((size_t)(dir * np + prime) << k) + i] = make_uint2(w, (uint32_t)(((uint64_t)w << 32) / pc.p));
+        }
+    }
+}
+
+void launch_fourstep_table(uint2* t4, const FieldArgs& f, const uint32_t* fold, int nprimes, int k1, int k2,
+                           cudaStream_t st) {
+    TableArgs a;
+    a.f = f;
+    for (int j = 0; j < nprimes; ++j) a.fold[j] = fold[j];
+    k_fourstep_table<<<dim3((1u << (k1 + k2)) / 256 > 1024 ? 1024 : (1u << (k1 + k2)) / 256, nprimes), 256, 0, st>>>(
+        t4, a, k1, k2);
+    count_launches(1);
+}
+
 bool cols_trunc_supported(int set, int k1, int k2, int cg, int mr, int keep) {
     col_config(set_base(set), k1, cg, mr, cg, mr);
 #define X(S, MM, CC, RR, KK) \

@@ -51,6 +51,15 @@ struct Crt5Const {
 
 struct ProdPtrs;
 
+// Four-step twiddle table of one set and length: Shoup pairs in the column
+// passes' own order, entry (direction * primes + prime) * N + s * N2 + i2 is
+// w^(+-i2 bitrev(s)); the inverse one also carries the prime's CRT scale.
+// Built once at start-up for the lengths that batches use (tables of a few
+// MB that stay in L2 while a class's products go by).
+constexpr int kTabMinLog2 = 13;
+constexpr int kTabMaxLog2[2] = {18, 19};  // sets 0 and 2
+inline size_t fourstep_entries(int nprimes, int k) { return (size_t)2 * nprimes << k; }
+
 // One product of the multi-pass (four-step) path.
 struct ProdArgs {
     const uint64_t* a;
@@ -71,6 +80,7 @@ struct ProdArgs {
     int chain;          // per-prime chains (host side: how the kernels are launched)
     int operand_only;   // forward columns of one operand: 1 = a, 2 = b (0: both)
     int rmr;            // row pass radix cap, 4 or 6 (0: default)
+    const uint2* t4;    // four-step twiddle table of the set and length (fourstep_entries), or nullptr
     int crt_chunk;      // CRT in limb chunks (chunk_words set): this launch's chunk
     int crt_blk0;       //   its first carry block
     int crt_last;       //   whether it is the last chunk
@@ -330,6 +340,10 @@ void launch_crt_carry(int set, const ProdArgs& a, cudaStream_t st, const ProdPtr
                       int max_nblk = 0, int nblk_launch = 0);
 int configure_fwd_cols();
 int configure_inv_cols();
+// fills a table for column length 2^k1, row length 2^k2 (set 0's arithmetic;
+// fold: the CRT scales in Montgomery form)
+void launch_fourstep_table(uint2* t4, const FieldArgs& f, const uint32_t* fold, int nprimes, int k1, int k2,
+                           cudaStream_t st);
 // whether the column kernels of a configuration exist truncated to `keep` eighths
 bool cols_trunc_supported(int set, int k1, int k2, int cg, int mr, int keep);
 

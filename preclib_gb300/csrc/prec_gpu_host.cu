@@ -309,6 +309,8 @@ struct Ctx {
     int* d_err = nullptr;
     int* h_err = nullptr;
     double2* fft_tw = nullptr;  // FP64 band twiddles
+    void* t4_mem = nullptr;     // four-step twiddle tables: sets 0 and 2, by log2 of the length
+    const uint2* t4[2][kMaxLog2 + 1] = {};
     FieldArgs field[kSets] = {};
     cudaMemPool_t pool = nullptr;
     bool split_primes = true;  // PREC_GPU_PRIME_STREAMS=0 runs the primes in one launch per kernel
@@ -484,6 +486,33 @@ static int build_tables(Ctx& c) {
     return 0;
 }
 
+// The four-step tables of every length in its default configuration (90 MB).
+static int build_fourstep_tables(Ctx& c) {
+    size_t total = 0;
+    for (int w = 0; w < 2; ++w)
+        for (int k = kTabMinLog2; k <= kTabMaxLog2[w]; ++k)
+            if (!w || k >= kWideMinLog2) total += fourstep_entries(kSetPrimes[w ? kWideSet : 0], k);
+    CK(cudaMalloc(&c.t4_mem, total * sizeof(uint2)));
+    uint2* p = static_cast<uint2*>(c.t4_mem);
+    for (int w = 0; w < 2; ++w)
+        for (int k = kTabMinLog2; k <= kTabMaxLog2[w]; ++k) {
+            if (w && k < kWideMinLog2) continue;
+            const int set = w ? kWideSet : 0, k1 = default_config(k).k1;
+            const CrtConst cc = w ? CrtConst{} : crt_for(0, k);
+            const Crt5Const c5 = w ? crt5_for(set, k) : Crt5Const{};
+            launch_fourstep_table(p, c.field[set], w ? c5.fold : cc.fold, kSetPrimes[set], k1, k - k1, nullptr);
+            c.t4[w][k] = p;
+            p += fourstep_entries(kSetPrimes[set], k);
+        }
+    CK(cudaGetLastError());
+    return 0;
+}
+
+const uint2* ctx_fourstep(int set, int k) {
+    if (set != 0 && set != kWideSet) return nullptr;
+    return g_ctx.t4[set == kWideSet][k];
+}
+
 static int init_locked(Ctx& c, int device) {
     if (c.ready) return 0;
     int n = 0;
@@ -516,6 +545,7 @@ static int init_locked(Ctx& c, int device) {
     CK(cudaGetLastError());
     int r = build_tables(c);
     if (r) return r;
+    if ((r = build_fourstep_tables(c))) return r;
     CK(cudaDeviceSynchronize());
     c.ready.store(true, std::memory_order_release);
     // a saved tuning table (an invalid file leaves the defaults in place)
@@ -1113,6 +1143,9 @@ void prec_gpu_shutdown(void) {
     c.gen.fetch_add(1, std::memory_order_relaxed);  // every thread takes a new lane next time
     cudaFree(c.tables);
     cudaFree(c.fft_tw);
+    cudaFree(c.t4_mem);
+    c.t4_mem = nullptr;
+    std::memset(c.t4, 0, sizeof(c.t4));
     cudaFree(c.d_err);
     cudaFreeHost(c.h_err);
     if (c.pool) cudaMemPoolDestroy(c.pool);
