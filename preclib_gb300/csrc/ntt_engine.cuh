@@ -534,23 +534,27 @@ __device__ __forceinline__ u128 crt3(uint32_t y1, uint32_t y2, uint32_t y3, cons
 }
 
 // crt3 of the four-step path: the inverse column pass has already
-// multiplied y_j by s1, k22, k33 (CrtConst::fold), so y_j is v1's, and
-// v2's and v3's first term.  Set 0 leaves y_j in [0, 4p), set 1 in [0, p).
+// multiplied y_1 by s1, y_2 by k22 2^32 and y_3 by k33 2^32 (CrtConst::fold), so
+// y_1 is v1, and v2 = (y_2 + v1 n21) / 2^32, v3 = (y_3 + v1 n31 + v2 n32) / 2^32
+// mod p: one sum of products and one Montgomery reduction each (sums below
+// 0.6 * 2^32 p).  Set 0 leaves y_j in [0, 4p), set 1 in [0, p).
 template <int SET>
 __device__ __forceinline__ u128 crt3_folded(uint32_t y1, uint32_t y2, uint32_t y3, const CrtConst& cc,
                                             const FieldArgs& f) {
     const uint32_t p1 = f.pc[0].p, p2 = f.pc[1].p, p3 = f.pc[2].p;
-    if constexpr (SET == 0) {
-        y1 = red1(red1(y1, f.pc[0].p2), p1);
-        y2 = red1(red1(y2, f.pc[1].p2), p2);
-        y3 = red1(red1(y3, f.pc[2].p2), p3);
-    }
+    if constexpr (SET == 0) y1 = red1(red1(y1, f.pc[0].p2), p1);
     const uint32_t v1 = y1;
-    const uint32_t v2 = sub_mod(y2, shoup_mul(v1, cc.k21, p2), p2);
-    uint32_t v3 = sub_mod(y3, shoup_mul(v1, cc.k31, p3), p3);
-    v3 = sub_mod(v3, shoup_mul(v2, cc.k32, p3), p3);
-    const uint64_t t = (uint64_t)v2 + (uint64_t)p2 * v3;
-    return (u128)t * p1 + v1;
+    auto redc = [](uint64_t t, const PrimeC& c) -> uint32_t {
+        const uint32_t m = (uint32_t)t * c.pinv;
+        return red1((uint32_t)((t + (uint64_t)m * c.p) >> 32), c.p);
+    };
+    const uint32_t v2 = redc((uint64_t)v1 * cc.n21 + y2, f.pc[1]);
+    const uint32_t v3 = redc((uint64_t)v1 * cc.n31 + ((uint64_t)v2 * cc.n32 + y3), f.pc[2]);
+    // v1 + p1 (v2 + p2 v3) in 32-bit words, one multiply-add each
+    const uint64_t t = (uint64_t)p2 * v3 + v2;
+    const uint64_t lo = (uint64_t)(uint32_t)t * p1 + v1;
+    const uint64_t hi = (t >> 32) * p1 + (lo >> 32);
+    return (u128)hi << 32 | (uint32_t)lo;
 }
 
 // Carry-in of every lane from the lanes' (G, P) bits: the chain

@@ -27,12 +27,14 @@ struct FieldArgs {
 // CRT constants of one transform length (Garner with the transform's
 // scale 2^32 * N^-1 folded in; see crt3 in ntt_engine.cuh).  The
 // single-CTA path multiplies prime j's outputs by sigma_j in the CRT (s1,
-// k22, k33 hold sigma_1, sigma_2 c12, sigma_3 c13 c23); the four-step path
-// applies those products in its inverse column pass instead, through
-// fold[j] = (that constant) * 2^32 mod p_j (Montgomery form) on the running
-// twiddle, and its CRT multiplies by k21, k31, k32 only.
+// k22, k33 hold sigma_1, sigma_2 c12, sigma_3 c13 c23; k21, k31, k32 the
+// others); the four-step path applies those products in its inverse column
+// pass instead, through fold[j] = (that constant, times 2^32 for j > 0) * 2^32
+// mod p_j (Montgomery form) on the running twiddle, and its CRT multiplies
+// by n21, n31, n32 = -k21, -k31, -k32 * 2^32 and divides by 2^32.
 struct CrtConst {
     ShoupC s1, k21, k22, k31, k32, k33;
+    uint32_t n21, n31, n32;
     uint32_t fold[3];
 };
 

@@ -143,8 +143,12 @@ static CrtConst crt_compute(int set, int k) {
     c.k32 = shoup(c23, p3);
     c.k33 = shoup(mulmod(s[2], c1323, p3), p3);
     c.fold[0] = mulmod(c.s1.w, (uint32_t)((1ull << 32) % p1), p1);
-    c.fold[1] = mulmod(c.k22.w, (uint32_t)((1ull << 32) % p2), p2);
-    c.fold[2] = mulmod(c.k33.w, (uint32_t)((1ull << 32) % p3), p3);
+    const uint32_t R2 = (uint32_t)((1ull << 32) % p2), R3 = (uint32_t)((1ull << 32) % p3);
+    c.fold[1] = mulmod(mulmod(c.k22.w, R2, p2), R2, p2);
+    c.fold[2] = mulmod(mulmod(c.k33.w, R3, p3), R3, p3);
+    c.n21 = p2 - mulmod(c.k21.w, R2, p2);  // (no constant is 0 mod p)
+    c.n31 = p3 - mulmod(c.k31.w, R3, p3);
+    c.n32 = p3 - mulmod(c.k32.w, R3, p3);
     return c;
 }
 
