@@ -28,21 +28,21 @@ struct DirectItem {
 };
 
 // Class of a batch product, or -1: the transform is faster (or an operand is
-// empty).  Direct where it measured below the single-CTA transform (ns per
-// product of a large batch, direct / transform, equal operands of n limbs):
-// 16: 1.2 / 18.7, 32: 1.8 / 18.8, 64: 3.2 / 21.0, 96: 6.2 / 23.5 (8.9 in the
-// class up to 128 limbs), 128: 11.4 / 24.6, 192: 29.1 / 27.8, 256: 37.1 / 29.0, 512: 139 / 70.  The direct time
-// goes with the shorter operand, the transform's with the sum: operands up to
-// 256 limbs cross near 180 x 180 limbs, operands up to 512 limbs at a
-// shorter one of about 100 limbs (27 ns against 29 of the 2^10-point
-// transform).
+// empty).  Direct where it measured below the single-CTA transform.  The
+// direct time goes with the class and the shorter operand, the transform's
+// with the points (ns per product of a large batch; 13.1 for 2^9 points, a sum of
+// up to 256 limbs, 19.9 for 2^10, 37.8 for 2^11):
+//   up to 128 limbs: 16 x 16 1.2, 32 1.8, 64 3.2, 96 6.2, 128 11.4
+//   up to 256, shorter operand 32: 7.7, 64: 13.3, 96: 18.6, 112: 21.3, 160: 28.9
+//   up to 512, shorter operand 32: 11.5 - 13.8, 48: 15.4 - 18.5, 64: 19.0 -
+//   23.3, 80: 28.2, 96: 33.3
 __host__ __device__ inline int direct_class(uint64_t la, uint64_t lb) {
     const uint64_t hi = la > lb ? la : lb, lo = la > lb ? lb : la;
     if (lo == 0) return -1;
     if (hi <= 96) return hi <= 64 ? 0 : 1;
     if (hi <= 128) return 2;
-    if (hi <= 256) return lo <= 160 ? 3 : -1;
-    return hi <= kDirectBatchMax && lo <= 96 ? 4 : -1;
+    if (hi <= 256) return lo <= (hi + lo <= 256 ? 64 : 104) ? 3 : -1;
+    return hi <= kDirectBatchMax && lo <= (hi + lo <= 512 ? 52 : 96) ? 4 : -1;
 }
 // whether a single device product runs directly
 bool direct_single(uint64_t la, uint64_t lb);

@@ -519,18 +519,31 @@ __device__ __forceinline__ void twiddle32_shoup(uint32_t (&x)[32], uint32_t t, u
 // CRT and carries
 // ---------------------------------------------------------------------------
 
-// Garner recombination of the three inverse-transform outputs (any value
-// below 2^32 of each residue class) into the exact coefficient below
+// Montgomery's reduction of a sum of products, t 2^-32 mod p below
+// p (t < 3 * 2^32 p)
+__device__ __forceinline__ uint32_t crt_redc(uint64_t t, const PrimeC& c) {
+    const uint32_t m = (uint32_t)t * c.pinv;
+    return red1(red1((uint32_t)((t + (uint64_t)m * c.p) >> 32), c.p2), c.p);
+}
+// v1 + p1 (v2 + p2 v3) in 32-bit words, one multiply-add each
+__device__ __forceinline__ u128 crt_value(uint32_t v1, uint32_t v2, uint32_t v3, const FieldArgs& f) {
+    const uint32_t p1 = f.pc[0].p, p2 = f.pc[1].p;
+    const uint64_t t = (uint64_t)p2 * v3 + v2;
+    const uint64_t lo = (uint64_t)(uint32_t)t * p1 + v1;
+    const uint64_t hi = (t >> 32) * p1 + (lo >> 32);
+    return (u128)hi << 32 | (uint32_t)lo;
+}
+
+// Garner recombination of the three inverse-transform outputs (in [0, 4p), set 0)
+// into the exact coefficient below
 // p1*p2*p3, with the transform scale folded into the constants
-// (src/mul_ntt.cpp:405-424 recombines its primes the same way).
+// (src/mul_ntt.cpp:405-424 recombines its primes the same way): one sum
+// of products and one Montgomery reduction per residue, sums below 6 p^2.
 __device__ __forceinline__ u128 crt3(uint32_t y1, uint32_t y2, uint32_t y3, const CrtConst& cc, const FieldArgs& f) {
-    const uint32_t p1 = f.pc[0].p, p2 = f.pc[1].p, p3 = f.pc[2].p;
-    const uint32_t v1 = shoup_mul(y1, cc.s1, p1);
-    const uint32_t v2 = sub_mod(shoup_mul(y2, cc.k22, p2), shoup_mul(v1, cc.k21, p2), p2);
-    uint32_t v3 = sub_mod(shoup_mul(y3, cc.k33, p3), shoup_mul(v1, cc.k31, p3), p3);
-    v3 = sub_mod(v3, shoup_mul(v2, cc.k32, p3), p3);
-    const uint64_t t = (uint64_t)v2 + (uint64_t)p2 * v3;
-    return (u128)t * p1 + v1;
+    const uint32_t v1 = shoup_mul(y1, cc.s1, f.pc[0].p);
+    const uint32_t v2 = crt_redc((uint64_t)y2 * cc.m22 + (uint64_t)v1 * cc.n21, f.pc[1]);
+    const uint32_t v3 = crt_redc((uint64_t)y3 * cc.m33 + (uint64_t)v1 * cc.n31 + (uint64_t)v2 * cc.n32, f.pc[2]);
+    return crt_value(v1, v2, v3, f);
 }
 
 // crt3 of the four-step path: the inverse column pass has already
@@ -550,11 +563,7 @@ __device__ __forceinline__ u128 crt3_folded(uint32_t y1, uint32_t y2, uint32_t y
     };
     const uint32_t v2 = redc((uint64_t)v1 * cc.n21 + y2, f.pc[1]);
     const uint32_t v3 = redc((uint64_t)v1 * cc.n31 + ((uint64_t)v2 * cc.n32 + y3), f.pc[2]);
-    // v1 + p1 (v2 + p2 v3) in 32-bit words, one multiply-add each
-    const uint64_t t = (uint64_t)p2 * v3 + v2;
-    const uint64_t lo = (uint64_t)(uint32_t)t * p1 + v1;
-    const uint64_t hi = (t >> 32) * p1 + (lo >> 32);
-    return (u128)hi << 32 | (uint32_t)lo;
+    return crt_value(v1, v2, v3, f);
 }
 
 // Carry-in of every lane from the lanes' (G, P) bits: the chain

@@ -25,15 +25,16 @@ struct FieldArgs {
 };
 
 // CRT constants of one transform length (Garner with the transform's
-// scale 2^32 * N^-1 folded in; see crt3 in ntt_engine.cuh).  The
-// single-CTA path multiplies prime j's outputs by sigma_j in the CRT (s1,
-// k22, k33 hold sigma_1, sigma_2 c12, sigma_3 c13 c23; k21, k31, k32 the
-// others); the four-step path applies those products in its inverse column
-// pass instead, through fold[j] = (that constant, times 2^32 for j > 0) * 2^32
-// mod p_j (Montgomery form) on the running twiddle, and its CRT multiplies
-// by n21, n31, n32 = -k21, -k31, -k32 * 2^32 and divides by 2^32.
+// scale 2^32 * N^-1 folded in; see crt3 in ntt_engine.cuh), c_ij = p_i^-1 mod
+// p_j and sigma_j prime j's scale.  The single-CTA path multiplies prime j's outputs in
+// the CRT (s1 = sigma_1; m22, m33 = sigma_2 c12, sigma_3 c13 c23 times 2^32); the
+// four-step path applies those products in its inverse column pass instead,
+// through fold[j] = (that constant, times 2^32 for j > 0) * 2^32 mod p_j
+// (Montgomery form) on the running twiddle.  n21, n31, n32 = -c12, -c13 c23, -c23
+// times 2^32: a Montgomery reduction takes the 2^32 away.
 struct CrtConst {
-    ShoupC s1, k21, k22, k31, k32, k33;
+    ShoupC s1;
+    uint32_t m22, m33;
     uint32_t n21, n31, n32;
     uint32_t fold[3];
 };
@@ -282,7 +283,6 @@ void uncount_launches(uint64_t n);
 // host-side launchers; `ev` (optional) gets an event recorded before the
 // first kernel and after each kernel.
 size_t ntt_small_smem_bytes(int k);
-int ntt_small_threads(int k);
 void ntt_launch_small(const SmallDesc* d_descs, const SmallDesc* single, int count, int k,
                       const FieldArgs& f, const CrtConst& crt, cudaStream_t st, cudaEvent_t* ev = nullptr);
 // Side streams of a single product: each prime's transform kernels run as

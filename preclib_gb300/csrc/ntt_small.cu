@@ -5,157 +5,163 @@
 // pointwise product and inverse DIT for each of the three primes, then CRT
 // and the carry chain (block-wide scan).  With a descriptor array the same
 // kernel runs one product per CTA for a whole batch of a length class.
+//
+// Bound by the integer multiply pipe.  A third of the threads to each prime: the
+// bottom pass, half of the work, has an item for every thread and the barriers
+// are those of one prime's transform.  (The primes in turn, with eight
+// points per thread: three quarters of the threads had no bottom item.  ns per
+// product of a large batch, before -> now: 256 x 256 limbs 29.1 -> 20.2, 512 x 512
+// 70 -> 39, 1024 x 1024 111 -> 91; 200 products of 256 limbs 22.6 -> 14.7 us; one of
+// 128 limbs between host arrays 41 -> 30.)
 #include "ntt_engine.cuh"
 
 namespace precgpu {
 
-// coefficient i of the product from the three residue arrays (0 outside)
-template <int M>
-__device__ __forceinline__ u128 small_coef(const uint32_t* sm, int64_t i, const CrtConst& cc, const FieldArgs& f) {
+// Threads per prime: one for each of the bottom pass's items (32 points), a warp
+// at least.  The three primes run side by side.
+constexpr int small_tp(int m) { return m <= 10 ? 32 : 1 << (m - 5); }
+constexpr int small_threads(int m) { return kPrimes * small_tp(m); }
+constexpr int kSmallRadix = 5;  // register passes of up to 5 stages
+// Resident CTAs the registers are limited for: what shared memory holds
+// (six arrays of 2^m words); short lengths run alone and are not limited.
+constexpr int small_minb(int m) { return m < 9 ? 1 : 768 / small_threads(m); }
+
+// pass T over NA arrays of one prime by its TP threads
+template <int M, int T, bool DIT, int NA>
+__device__ __forceinline__ void small_pass(uint32_t* s0, int t, const uint2* __restrict__ tw, const PrimeC& pc) {
+    using G = Geom<M, T, kSmallRadix>;
     constexpr int AS = astride_for(M);
-    if (i < 0 || i >= (1 << M)) return 0;
-    const int pi = padded((int)i);
-    return crt3(sm[2 * AS + pi], sm[3 * AS + pi], sm[4 * AS + pi], cc, f);
+    for (uint32_t u = t; u < (1u << G::LGI); u += small_tp(M)) {
+        uint32_t* s = s0 + G::pbase(u);
+        uint32_t x[NA][G::R];
+#pragma unroll
+        for (int a = 0; a < NA; ++a)
+#pragma unroll
+            for (int q = 0; q < G::R; ++q) x[a][q] = s[a * AS + q * G::QS];
+        regs_pass<0, M, T, DIT, NA, kSmallRadix>(x, u, tw, pc);
+#pragma unroll
+        for (int a = 0; a < NA; ++a)
+#pragma unroll
+            for (int q = 0; q < G::R; ++q) s[a * AS + q * G::QS] = x[a][q];
+    }
 }
 
 template <int M>
-__global__ void __launch_bounds__(256) k_small(const SmallDesc* __restrict__ descs, SmallDesc single, FieldArgs f,
-                                               CrtConst crt) {
+__global__ void __launch_bounds__(small_threads(M), small_minb(M))
+    k_small(const SmallDesc* __restrict__ descs, SmallDesc single, FieldArgs f, CrtConst crt) {
     extern __shared__ uint32_t sm[];
     __shared__ BlockCarryShared sh;
-    constexpr int NP = sch_np(M);
+    __shared__ uint64_t s_hi[small_threads(M) / 32];
+    constexpr int MR = kSmallRadix;
+    constexpr int NP = sch_np(M, MR);
     constexpr int AS = astride_for(M);
+    constexpr int TP = small_tp(M);
+    const int prime = threadIdx.x / TP, t = threadIdx.x % TP;
+    const PrimeC pc = f.pc[prime];
+    const uint2* __restrict__ twf = f.tf[prime];
+    const uint2* __restrict__ twi = f.ti[prime];
+    uint32_t* const s0 = sm + prime * 2 * AS;  // this prime's arrays: a (then the product), b
     pdl_enter();
     SmallDesc d = descs ? descs[blockIdx.x] : single;
     d.a = after_entry(d.a);
     d.b = after_entry(d.b);
     const uint32_t* __restrict__ da = reinterpret_cast<const uint32_t*>(d.a);
     const uint32_t* __restrict__ db = reinterpret_cast<const uint32_t*>(d.b);
-    const uint64_t nda = 2 * d.la, ndb = 2 * d.lb;
+    const uint32_t nda = 2 * (uint32_t)d.la, ndb = 2 * (uint32_t)d.lb;
 
-    for (int prime = 0; prime < kPrimes; ++prime) {
-        const PrimeC pc = f.pc[prime];
-        const uint2* __restrict__ twf = f.tf[prime];
-        const uint2* __restrict__ twi = f.ti[prime];
-        uint32_t* res = sm + (2 + prime) * AS;
-        if constexpr (NP == 1) {
-            // 32 points: one register pass does everything
-            if (threadIdx.x == 0) {
-                uint32_t x[2][32];
+    {   // top DIF pass from the limbs
+        using G = Geom<M, 0, MR>;
+        for (uint32_t u = t; u < (1u << G::LGI); u += TP) {
+            const uint32_t base = G::base(u);
+            uint32_t x[2][G::R];
 #pragma unroll
-                for (int q = 0; q < 32; ++q) {
-                    x[0][q] = (uint64_t)q < nda ? Ar<0>::digit(__ldg(&da[q]), pc) : 0u;
-                    x[1][q] = (uint64_t)q < ndb ? Ar<0>::digit(__ldg(&db[q]), pc) : 0u;
-                }
-                regs_pass<0, M, 0, false, 2>(x, 0, twf, pc);
-                uint32_t y[1][32];
-#pragma unroll
-                for (int q = 0; q < 32; ++q) y[0][q] = Ar<0>::mul(x[0][q], x[1][q], pc);
-                regs_pass<0, M, 0, true, 1>(y, 0, twi, pc);
-#pragma unroll
-                for (int q = 0; q < 32; ++q) res[q] = y[0][q];
+            for (int q = 0; q < G::R; ++q) {
+                const uint32_t i = base + ((uint32_t)q << G::LO);
+                x[0][q] = i < nda ? Ar<0>::digit(__ldg(&da[i]), pc) : 0u;
+                x[1][q] = i < ndb ? Ar<0>::digit(__ldg(&db[i]), pc) : 0u;
             }
-        } else {
-            {   // top DIF pass from the limbs
-                using G = Geom<M, 0>;
-                for (int w = threadIdx.x; w < (1 << G::LGI); w += blockDim.x) {
-                    const uint32_t u = w;
-                    const uint32_t base = G::base(u);
-                    uint32_t x[2][G::R];
+            regs_pass<0, M, 0, false, 2, MR>(x, u, twf, pc);
+            if constexpr (NP == 1) {  // 32 points: one register pass does everything
+                uint32_t y[1][G::R];
 #pragma unroll
-                    for (int q = 0; q < G::R; ++q) {
-                        const uint32_t i = base + ((uint32_t)q << G::LO);
-                        x[0][q] = i < nda ? Ar<0>::digit(__ldg(&da[i]), pc) : 0u;
-                        x[1][q] = i < ndb ? Ar<0>::digit(__ldg(&db[i]), pc) : 0u;
-                    }
-                    regs_pass<0, M, 0, false, 2>(x, u, twf, pc);
-                    uint32_t* s = sm + G::pbase(u);
+                for (int q = 0; q < G::R; ++q) y[0][q] = Ar<0>::mul(x[0][q], x[1][q], pc);
+                regs_pass<0, M, 0, true, 1, MR>(y, 0, twi, pc);
 #pragma unroll
-                    for (int q = 0; q < G::R; ++q) {
-                        s[q * G::QS] = x[0][q];
-                        s[AS + q * G::QS] = x[1][q];
-                    }
-                }
-                __syncthreads();
-            }
-            row_passes<0, M, 1, NP - 2, false, 2>(sm, AS, 2, twf, pc);
-            {   // bottom: last DIF stages, product, first DIT stages
-                using G = Geom<M, NP - 1>;
-                for (int w = threadIdx.x; w < (1 << G::LGI); w += blockDim.x) {
-                    const uint32_t u = w;
-                    uint32_t* s = sm + 33 * u;
-                    uint32_t x[2][32];
+                for (int q = 0; q < G::R; ++q) s0[padded(q)] = y[0][q];
+            } else {
+                uint32_t* s = s0 + G::pbase(u);
 #pragma unroll
-                    for (int q = 0; q < 32; ++q) {
-                        x[0][q] = s[q];
-                        x[1][q] = s[AS + q];
-                    }
-                    regs_pass<0, M, NP - 1, false, 2>(x, u, twf, pc);
-                    uint32_t y[1][32];
-#pragma unroll
-                    for (int q = 0; q < 32; ++q) y[0][q] = Ar<0>::mul(x[0][q], x[1][q], pc);
-                    regs_pass<0, M, NP - 1, true, 1>(y, u, twi, pc);
-#pragma unroll
-                    for (int q = 0; q < 32; ++q) s[q] = y[0][q];
-                }
-                __syncthreads();
-            }
-            row_passes<0, M, NP - 2, 1, true, 1>(sm, AS, 1, twi, pc);
-            {   // top DIT pass into this prime's residue array
-                using G = Geom<M, 0>;
-                for (int w = threadIdx.x; w < (1 << G::LGI); w += blockDim.x) {
-                    const uint32_t u = w;
-                    const uint32_t pb = G::pbase(u);
-                    uint32_t x[1][G::R];
-#pragma unroll
-                    for (int q = 0; q < G::R; ++q) x[0][q] = sm[pb + q * G::QS];
-                    regs_pass<0, M, 0, true, 1>(x, u, twi, pc);
-#pragma unroll
-                    for (int q = 0; q < G::R; ++q) res[pb + q * G::QS] = x[0][q];
+                for (int q = 0; q < G::R; ++q) {
+                    s[q * G::QS] = x[0][q];
+                    s[AS + q * G::QS] = x[1][q];
                 }
             }
         }
         __syncthreads();
     }
-
-    // CRT + carries over the block, L limbs per thread per round
-    constexpr int L = 8;
-    bool carry = false;
-    for (int64_t r0 = 0; r0 < (int64_t)d.lout; r0 += (int64_t)blockDim.x * L) {
-        const int64_t m0 = r0 + threadIdx.x * L;
-        u128 T[L];
-#pragma unroll
-        for (int k = 0; k < L; ++k)
-            T[k] = small_coef<M>(sm, 2 * (m0 + k), crt, f) + (small_coef<M>(sm, 2 * (m0 + k) + 1, crt, f) << 32);
-        uint64_t prev_hi = 0;
-        if (m0 > 0) {
-            const u128 tp = small_coef<M>(sm, 2 * m0 - 2, crt, f) + (small_coef<M>(sm, 2 * m0 - 1, crt, f) << 32);
-            prev_hi = (uint64_t)(tp >> 64);
+    if constexpr (NP > 1) {
+        if constexpr (NP > 2) {
+            static_assert(NP == 3);
+            small_pass<M, 1, false, 2>(s0, t, twf, pc);
+            __syncthreads();
         }
-        uint64_t v[L];
-        uint32_t gbits;
-        bool G, P;
-        limbs_from_sums<L>(T, prev_hi, v, gbits, G, P);
-        auto cin_fn = [&](bool Gb, bool Pb) -> bool {
-            sh.block_cin = (Gb || (Pb && carry)) ? 1u : 0u;
-            return carry;
-        };
-        const bool cin = block_carry(G, P, sh, cin_fn);
-        limbs_finish<L>(m0, d.lout, v, gbits, cin, d.out);
+        if (t < (1 << (M - 5))) {  // bottom: last DIF stages, product, first DIT stages
+            uint32_t* s = s0 + 33 * t;
+            uint32_t x[2][32];
+#pragma unroll
+            for (int q = 0; q < 32; ++q) {
+                x[0][q] = s[q];
+                x[1][q] = s[AS + q];
+            }
+            regs_pass<0, M, NP - 1, false, 2, MR>(x, t, twf, pc);
+            uint32_t y[1][32];
+#pragma unroll
+            for (int q = 0; q < 32; ++q) y[0][q] = Ar<0>::mul(x[0][q], x[1][q], pc);
+            regs_pass<0, M, NP - 1, true, 1, MR>(y, t, twi, pc);
+#pragma unroll
+            for (int q = 0; q < 32; ++q) s[q] = y[0][q];
+        }
         __syncthreads();
-        carry = sh.block_cin != 0;
+        if constexpr (NP > 2) {
+            small_pass<M, 1, true, 1>(s0, t, twi, pc);
+            __syncthreads();
+        }
+        small_pass<M, 0, true, 1>(s0, t, twi, pc);
         __syncthreads();
     }
+
+    // CRT + carries over the block, L limbs per thread
+    constexpr int L = 6;
+    static_assert(small_threads(M) * L >= (1 << M) / 2, "every limb in one round");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int m0 = (int)threadIdx.x * L;
+    u128 T[L];
+#pragma unroll
+    for (int k = 0; k < L; ++k) {
+        u128 c[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int i = 2 * (m0 + k) + e, pi = padded(i);
+            c[e] = i < (1 << M) ? crt3(sm[pi], sm[2 * AS + pi], sm[4 * AS + pi], crt, f) : (u128)0;
+        }
+        T[k] = c[0] + (c[1] << 32);
+    }
+    const uint64_t hi = (uint64_t)(T[L - 1] >> 64);
+    uint64_t prev_hi = __shfl_up_sync(0xffffffffu, hi, 1);
+    if (lane == 31) s_hi[warp] = hi;
+    __syncthreads();
+    if (lane == 0) prev_hi = warp ? s_hi[warp - 1] : 0;
+    uint64_t v[L];
+    uint32_t gbits;
+    bool G, P;
+    limbs_from_sums<L>(T, prev_hi, v, gbits, G, P);
+    const bool cin = block_carry_in0(G, P, sh, [](bool, bool) {});  // (no carry out: the product fits)
+    limbs_finish<L>(m0, d.lout, v, gbits, cin, d.out);
 }
 
 // ---------------------------------------------------------------------------
 
-size_t ntt_small_smem_bytes(int k) { return (size_t)5 * astride_for(k) * sizeof(uint32_t); }
-
-int ntt_small_threads(int k) {
-    int t = 1 << (k > 3 ? k - 3 : 0);
-    return t < 64 ? 64 : (t > 256 ? 256 : t);
-}
+size_t ntt_small_smem_bytes(int k) { return (size_t)2 * kPrimes * astride_for(k) * sizeof(uint32_t); }
 
 #define PREC_SMALL(X) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12)
 
@@ -164,7 +170,7 @@ void ntt_launch_small(const SmallDesc* d_descs, const SmallDesc* single, int cou
     SmallDesc one{};
     if (single) one = *single;
     if (ev) cudaEventRecord(ev[0], st);
-    const int threads = ntt_small_threads(k);
+    const int threads = small_threads(k);
     const size_t smem = ntt_small_smem_bytes(k);
 #define X(MM) \
     if (k == MM) {                                                     \

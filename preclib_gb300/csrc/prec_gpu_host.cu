@@ -136,19 +136,16 @@ static CrtConst crt_compute(int set, int k) {
     const uint32_t c12 = invmod(p1 % p2, p2), c13 = invmod(p1 % p3, p3), c23 = invmod(p2 % p3, p3);
     CrtConst c;
     c.s1 = shoup(s[0], p1);
-    c.k21 = shoup(c12, p2);
-    c.k22 = shoup(mulmod(s[1], c12, p2), p2);
     const uint32_t c1323 = mulmod(c13, c23, p3);
-    c.k31 = shoup(c1323, p3);
-    c.k32 = shoup(c23, p3);
-    c.k33 = shoup(mulmod(s[2], c1323, p3), p3);
-    c.fold[0] = mulmod(c.s1.w, (uint32_t)((1ull << 32) % p1), p1);
-    const uint32_t R2 = (uint32_t)((1ull << 32) % p2), R3 = (uint32_t)((1ull << 32) % p3);
-    c.fold[1] = mulmod(mulmod(c.k22.w, R2, p2), R2, p2);
-    c.fold[2] = mulmod(mulmod(c.k33.w, R3, p3), R3, p3);
-    c.n21 = p2 - mulmod(c.k21.w, R2, p2);  // (no constant is 0 mod p)
-    c.n31 = p3 - mulmod(c.k31.w, R3, p3);
-    c.n32 = p3 - mulmod(c.k32.w, R3, p3);
+    const uint32_t R1 = (uint32_t)((1ull << 32) % p1), R2 = (uint32_t)((1ull << 32) % p2), R3 = (uint32_t)((1ull << 32) % p3);
+    c.m22 = mulmod(mulmod(s[1], c12, p2), R2, p2);
+    c.m33 = mulmod(mulmod(s[2], c1323, p3), R3, p3);
+    c.n21 = p2 - mulmod(c12, R2, p2);  // (no constant is 0 mod p)
+    c.n31 = p3 - mulmod(c1323, R3, p3);
+    c.n32 = p3 - mulmod(c23, R3, p3);
+    c.fold[0] = mulmod(c.s1.w, R1, p1);
+    c.fold[1] = mulmod(c.m22, R2, p2);
+    c.fold[2] = mulmod(c.m33, R3, p3);
     return c;
 }
 

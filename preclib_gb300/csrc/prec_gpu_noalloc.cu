@@ -129,18 +129,15 @@ static CrtConst na_crt(int k) {
     const uint32_t c23 = na_hpow(p2 % p3, p3 - 2, p3), c1323 = na_mulmod(c13, c23, p3);
     CrtConst c;
     c.s1 = na_shoup(s[0], p1);
-    c.k21 = na_shoup(c12, p2);
-    c.k22 = na_shoup(na_mulmod(s[1], c12, p2), p2);
-    c.k31 = na_shoup(c1323, p3);
-    c.k32 = na_shoup(c23, p3);
-    c.k33 = na_shoup(na_mulmod(s[2], c1323, p3), p3);
-    c.fold[0] = na_mulmod(c.s1.w, (uint32_t)((1ull << 32) % p1), p1);
-    const uint32_t R2 = (uint32_t)((1ull << 32) % p2), R3 = (uint32_t)((1ull << 32) % p3);
-    c.fold[1] = na_mulmod(na_mulmod(c.k22.w, R2, p2), R2, p2);
-    c.fold[2] = na_mulmod(na_mulmod(c.k33.w, R3, p3), R3, p3);
-    c.n21 = p2 - na_mulmod(c.k21.w, R2, p2);
-    c.n31 = p3 - na_mulmod(c.k31.w, R3, p3);
-    c.n32 = p3 - na_mulmod(c.k32.w, R3, p3);
+    const uint32_t R1 = (uint32_t)((1ull << 32) % p1), R2 = (uint32_t)((1ull << 32) % p2), R3 = (uint32_t)((1ull << 32) % p3);
+    c.m22 = na_mulmod(na_mulmod(s[1], c12, p2), R2, p2);
+    c.m33 = na_mulmod(na_mulmod(s[2], c1323, p3), R3, p3);
+    c.n21 = p2 - na_mulmod(c12, R2, p2);  // (no constant is 0 mod p)
+    c.n31 = p3 - na_mulmod(c1323, R3, p3);
+    c.n32 = p3 - na_mulmod(c23, R3, p3);
+    c.fold[0] = na_mulmod(c.s1.w, R1, p1);
+    c.fold[1] = na_mulmod(c.m22, R2, p2);
+    c.fold[2] = na_mulmod(c.m33, R3, p3);
     return c;
 }
 
