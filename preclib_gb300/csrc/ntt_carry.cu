@@ -88,6 +88,23 @@ void ntt_launch_4step(int set, const ProdArgs& args, cudaStream_t st, cudaEvent_
     if (ev) cudaEventRecord(ev[4], st);
 }
 
+void ntt_launch_4step_staged(int set, const ProdArgs& args, cudaStream_t s, cudaEvent_t a_ready, cudaEvent_t b_ready,
+                             const CrtChunks* chunks) {
+    cudaStreamWaitEvent(s, a_ready, 0);
+    ProdArgs a = args;
+    if (!args.square) {
+        a.operand_only = 1;
+        launch_fwd_cols(set, a, s);
+        cudaStreamWaitEvent(s, b_ready, 0);
+        a.operand_only = 2;
+    }
+    launch_fwd_cols(set, a, s);
+    launch_rows(set, args, s);
+    launch_inv_cols(set, args, s);
+    if (chunks) launch_crt_chunks(set, args, s, *chunks);
+    else launch_crt_carry(set, args, s);
+}
+
 int ntt_configure_kernels() {
     int e = configure_fwd_cols();
     if (!e) e = configure_inv_cols();

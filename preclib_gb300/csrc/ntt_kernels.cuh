@@ -310,6 +310,10 @@ struct CrtChunks {
 void ntt_launch_4step(int set, const ProdArgs& args, cudaStream_t st, cudaEvent_t* ev = nullptr,
                       const PrimeStreams* ps = nullptr, cudaEvent_t a_ready = nullptr,
                       cudaEvent_t b_ready = nullptr, const CrtChunks* chunks = nullptr);
+// A product whose operands are still being copied (events a_ready, b_ready), on one
+// side stream s with every prime in one launch per pass.
+void ntt_launch_4step_staged(int set, const ProdArgs& args, cudaStream_t s, cudaEvent_t a_ready, cudaEvent_t b_ready,
+                             const CrtChunks* chunks);
 // One product of 2^13 .. 2^18 points in a default configuration, by the
 // kernels built for latency (ntt_lat.cu).  lat_keep: the eighths they keep for
 // a product that needs `keep` (0: no such kernels).

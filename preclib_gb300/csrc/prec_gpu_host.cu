@@ -787,7 +787,14 @@ static int enqueue_ntt(Ctx& c, Lane& L, const uint64_t* d_a, uint64_t la, const 
         args.crt = pl.crt;
         args.crt5 = pl.crt5;
         args.f = c.field[pl.set];
-        const bool split = c.split_primes && (pl.split || a_ready);
+        if (a_ready && !pl.split) {
+            ntt_launch_4step_staged(pl.set, args, L.prime_streams.s[0], a_ready, b_ready, chunks);
+            CK(cudaEventRecord(L.prime_streams.join[0], L.prime_streams.s[0]));
+            CK(cudaStreamWaitEvent(st, L.prime_streams.join[0], 0));
+            CK(cudaGetLastError());
+            return 0;
+        }
+        const bool split = c.split_primes && pl.split;
         const int lat = split ? 0 : plan_latency(pl);
         if (lat) {
             args.keep = lat;
@@ -951,10 +958,16 @@ enum { kModeBands = 0, kModeNtt = 1, kModeFft = 2 };
 // 54.8; past that the host's own copies cost more than the copy engine's.
 constexpr size_t kStagedLimbs = 32768;
 
-// Host products from 2^19 points run per-prime chains even where a device
-// product does not: a's transforms start while b is still on its way, and
-// the result goes out chunk by chunk.
-constexpr int kHostChainMinLog2 = 19;
+// Host products from 2^19 points overlap with their copies: a's forward columns
+// run while b is still on its way, and the result goes out chunk by
+// chunk.  Where a device product runs per-prime chains (2^21 points on) so does
+// a host product; below, one launch per pass on a side stream: the chains'
+// 24 and more launches took the host longer than the copies did (200000 x 200000
+// limbs 123.5 -> 101 us, 262144 128.5 -> 111, 400000 164 -> 155, 524288 181 -> 176;
+// but 1M x 1M 306 with chains, 318 without).  At 2^18 points copies
+// and the kernels built for latency in turn are faster: 65536 x 65536 limbs 54,
+// overlapped 66; 131072 x 131072 76 and 83.
+constexpr int kHostOverlapMinLog2 = 19;
 
 static int ensure_pin(Lane& L) {
     if (L.pin) return 0;
@@ -1008,9 +1021,9 @@ static int host_mul(const uint64_t* a, size_t an, const uint64_t* b, size_t bn, 
     }
     // operands and result each start on a 256-byte boundary (32 limbs)
     const size_t la_pad = (la + 31) & ~(size_t)31, lb_pad = square ? 0 : (lb + 31) & ~(size_t)31;
-    // per-prime chains start on a's forward columns while b is copied
-    const bool chains = !use_fft && !blocked && pl.path == 1 && c.split_primes && (pl.split || pl.k >= kHostChainMinLog2);
-    const bool staged = !blocked && !chains && lout <= kStagedLimbs && ensure_pin(L) == 0;
+    // the kernels start on a's forward columns while b is copied
+    const bool overlap = !use_fft && !blocked && pl.path == 1 && c.split_primes && (pl.split || pl.k >= kHostOverlapMinLog2);
+    const bool staged = !blocked && !overlap && lout <= kStagedLimbs && ensure_pin(L) == 0;
     if ((r = ensure_io(L, la_pad + lb_pad + lout))) return r;
     uint64_t* buf = staged ? L.pin : L.io;
     uint64_t* d_a = buf;
@@ -1027,9 +1040,9 @@ static int host_mul(const uint64_t* a, size_t an, const uint64_t* b, size_t bn, 
         if (!square) memcpy(d_b, b, lb * sizeof(uint64_t));
     } else {
         CK(cudaMemcpyAsync(d_a, a, la * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-        if (chains) CK(cudaEventRecord(L.ev_a, st));
+        if (overlap) CK(cudaEventRecord(L.ev_a, st));
         if (!square) CK(cudaMemcpyAsync(d_b, b, lb * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-        if (chains) CK(cudaEventRecord(L.ev_b, st));
+        if (overlap) CK(cudaEventRecord(L.ev_b, st));
     }
     CK(cudaEventRecord(L.ev0, st));
     bool copied = false;  // the result went out chunk by chunk
@@ -1063,17 +1076,18 @@ static int host_mul(const uint64_t* a, size_t an, const uint64_t* b, size_t bn, 
         // a large product's CRT runs in limb chunks; each chunk's limbs copy
         // out on the copy stream while the next chunks run
         CrtChunks ch{};
-        const bool chunked = chains && pl.nblk >= 2 * kCrtMaxChunks;
+        const bool chunked = overlap && pl.nblk >= 2 * kCrtMaxChunks;
         if (chunked) {
             const int per = (pl.nblk + kCrtMaxChunks - 1) / kCrtMaxChunks;
             ch.count = (pl.nblk + per - 1) / per;  // every chunk nonempty
             ch.words = L.chunk_words;
             for (int i = 0; i <= ch.count; ++i) ch.blk0[i] = std::min(i * per, pl.nblk);
             for (int i = 0; i < ch.count; ++i) ch.done[i] = L.chunk_done[i];
-            CK(cudaMemsetAsync(L.chunk_words, 0, 2 * kCrtMaxChunks * sizeof(uint32_t), st));
+            CK(cudaMemsetAsync(L.chunk_words, 0, 2 * kCrtMaxChunks * sizeof(uint32_t),
+                               pl.split ? st : L.prime_streams.s[0]));
         }
-        if ((r = enqueue_ntt(c, L, d_a, la, d_b, lb, d_out, pl, st, err, nullptr, chains ? L.ev_a : nullptr,
-                             chains ? L.ev_b : nullptr, chunked ? &ch : nullptr)))
+        if ((r = enqueue_ntt(c, L, d_a, la, d_b, lb, d_out, pl, st, err, nullptr, overlap ? L.ev_a : nullptr,
+                             overlap ? L.ev_b : nullptr, chunked ? &ch : nullptr)))
             return r;
         if (chunked) {
             const uint64_t bl = (uint64_t)crt_block_limbs(pl.set);
