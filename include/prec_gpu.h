@@ -99,7 +99,9 @@ int prec_gpu_sqr(const uint64_t *a, size_t an, uint64_t *out);
  * runs each prime's kernels on its own stream.  Every product (single, batch,
  * serving loop) uses the configuration of its length.  Defaults apply until
  * a length is tuned, set or loaded; PREC_GPU_TUNE_FILE names a table that
- * prec_gpu_init loads. */
+ * prec_gpu_init loads.  (Tables are tuned on 32-bit digits.  On 64-bit digits
+ * a length whose entry is the default takes the default of that digit width,
+ * which differs at 2^22 points.) */
 typedef struct {
     int log2_n;
     int log2_cols;      /* column length 2^log2_cols, row length 2^(log2_n - log2_cols) */

@@ -170,18 +170,20 @@ __device__ __forceinline__ void inv_cols_tile(const ProdArgs& args, const ProdPt
     X(2, 11, 8, 4) X(2, 11, 4, 6) X(2, 11, 8, 6) X(3, 10, 4, 6) X(3, 10, 8, 6) X(3, 11, 4, 4)             \
     X(3, 11, 8, 4) X(3, 11, 4, 6) X(3, 11, 8, 6) X(3, 12, 4, 6)
 
-// (SET, M, C, MR, K2) of the default configurations (sets 0 and 2: N1 =
-// 2^floor(k/2); sets 1 and 3: N2 = 2^13), compiled with a constant row
-// length.  The inverse columns of sets 2 and 3 are set 0's and set 1's.
+// (SET, M, C, MR, K2) of the default configurations (set 0: N1 =
+// 2^floor(k/2), set 2 also wide_column_log2's; sets 1 and 3: N2 = 2^13), compiled
+// with a constant row length.  The inverse columns of sets 2 and 3 are set 0's and set 1's.
 #define PREC_COLS_FWD_K2_CONFIGS(X)                                                                        \
     X(0, 6, 8, 6, 7) X(0, 7, 8, 6, 7) X(0, 7, 8, 6, 8) X(0, 8, 8, 6, 8) X(0, 8, 8, 6, 9) X(0, 9, 8, 6, 9)   \
     X(0, 9, 8, 6, 10) X(0, 10, 8, 6, 10) X(0, 10, 8, 6, 11) X(0, 11, 8, 6, 11) X(0, 11, 8, 6, 12)           \
     X(2, 9, 8, 6, 9) X(2, 9, 8, 6, 10) X(2, 10, 8, 6, 10) X(2, 10, 8, 6, 11) X(2, 11, 8, 6, 11)             \
+    X(2, 10, 8, 6, 12)                                                                                     \
     X(1, 11, 8, 6, 13) X(1, 12, 4, 6, 13) X(1, 13, 4, 6, 13) X(3, 10, 8, 6, 13) X(3, 11, 8, 6, 13)         \
     X(3, 12, 4, 6, 13)
 #define PREC_COLS_INV_K2_CONFIGS(X)                                                                        \
     X(0, 6, 8, 6, 7) X(0, 7, 8, 6, 7) X(0, 7, 8, 6, 8) X(0, 8, 8, 6, 8) X(0, 8, 8, 6, 9) X(0, 9, 8, 6, 9)   \
     X(0, 9, 8, 6, 10) X(0, 10, 8, 6, 10) X(0, 10, 8, 6, 11) X(0, 11, 8, 6, 11) X(0, 11, 8, 6, 12)           \
+    X(0, 10, 8, 6, 12)                                                                                     \
     X(1, 10, 8, 6, 13) X(1, 11, 8, 6, 13) X(1, 12, 4, 6, 13) X(1, 13, 4, 6, 13)
 
 // Batch classes with enough products take more short columns per CTA, 8192
@@ -202,12 +204,12 @@ __device__ __forceinline__ void inv_cols_tile(const ProdArgs& args, const ProdPt
 #define PREC_COLS_FWD_TRUNC_CONFIGS(X)                                                                      \
     X(0, 8, 8, 6, 8) X(0, 8, 8, 6, 9) X(0, 9, 8, 6, 9) X(0, 9, 8, 6, 10) X(0, 10, 8, 6, 10)                 \
     X(0, 10, 8, 6, 11) X(0, 11, 8, 6, 11) X(0, 11, 8, 6, 12) X(2, 9, 8, 6, 9) X(2, 9, 8, 6, 10)             \
-    PREC_COLS_FWD_BATCH_CONFIGS(X) X(2, 10, 8, 6, 10) X(2, 10, 8, 6, 11) X(2, 11, 8, 6, 11) X(1, 11, 8, 6, 13) X(1, 12, 4, 6, 13)          \
+    PREC_COLS_FWD_BATCH_CONFIGS(X) X(2, 10, 8, 6, 10) X(2, 10, 8, 6, 11) X(2, 10, 8, 6, 12) X(1, 11, 8, 6, 13) X(1, 12, 4, 6, 13)          \
     X(1, 13, 4, 6, 13) X(3, 10, 8, 6, 13) X(3, 11, 8, 6, 13) X(3, 12, 4, 6, 13)
 #define PREC_COLS_INV_TRUNC_CONFIGS(X)                                                                      \
     X(0, 8, 8, 6, 8) X(0, 8, 8, 6, 9) X(0, 9, 8, 6, 9) X(0, 9, 8, 6, 10) X(0, 10, 8, 6, 10)                 \
     X(0, 10, 8, 6, 11) X(0, 11, 8, 6, 11) X(0, 11, 8, 6, 12) X(1, 10, 8, 6, 13) X(1, 11, 8, 6, 13)          \
-    PREC_COLS_INV_BATCH_CONFIGS(X) X(1, 12, 4, 6, 13) X(1, 13, 4, 6, 13)
+    X(0, 10, 8, 6, 12) PREC_COLS_INV_BATCH_CONFIGS(X) X(1, 12, 4, 6, 13) X(1, 13, 4, 6, 13)
 
 inline size_t col_smem(int m, int cg) { return (size_t)cg * astride_for(m) * sizeof(uint32_t); }
 

@@ -49,15 +49,28 @@ int set_of(int k) { return k <= kSetMaxLog2[0] ? 0 : 1; }
 
 bool pow2(int x) { return x > 0 && (x & (x - 1)) == 0; }
 
+bool same(const KernelConfig& a, const KernelConfig& b) {
+    return a.k1 == b.k1 && a.cg == b.cg && a.cmr == b.cmr && a.rmr == b.rmr && a.rows == b.rows &&
+           a.split == b.split;
+}
+
 }  // namespace
+
+// Column length of set 2: at most 2^10, so 2^22 points run as 2^10 x 2^12.  2^10-point
+// columns run in 128-thread CTAs, six to an SM, 2^11-point ones take 256 threads,
+// three to an SM: 1.2M x 1.2M limbs 215.8 -> 207.6 us, 1.5M 251.6 -> 237.7, 2M 330.9
+// -> 307.1.  (2^20 points as 2^9 x 2^11: whole 84.1 -> 81.8, but the
+// square of 300007 limbs, 5 eighths, 46.4 -> 47.6.)
+static int wide_column_log2(int k) { return k / 2 < 10 ? k / 2 : 10; }
 
 static KernelConfig default_config_set(int k, int set) {
     KernelConfig c;
     // column length N1 = 2^k1, row length N2 = 2^k2; set 1 keeps the rows at
     // 2^13 so its column CTAs stay within a third of shared memory
-    c.k1 = set == 0 ? k / 2 : k - 13;
+    const int base = set_base(set);
+    c.k1 = base == 1 ? k - 13 : (set == kWideSet ? wide_column_log2(k) : k / 2);
     int cg, mr;
-    col_config(set, c.k1, 0, 0, cg, mr);
+    col_config(base, c.k1, 0, 0, cg, mr);
     c.cg = cg;
     c.cmr = mr;
     c.rmr = row_radix_cap(k - c.k1, 0);
@@ -94,9 +107,13 @@ KernelConfig tuned_config(int k) {
     return default_config(k);
 }
 
+// The table holds one configuration per length, tuned on 32-bit digits; a length
+// left at its default keeps set 2's own default.
 KernelConfig config_for(int k, int set) {
     const int base = set_base(set);
-    return base == set_of(k) ? tuned_config(k) : default_config_set(k, base);
+    if (base != set_of(k)) return default_config_set(k, base);
+    const KernelConfig c = tuned_config(k);
+    return set == kWideSet && same(c, default_config(k)) ? default_config_set(k, kWideSet) : c;
 }
 
 void apply_config(Plan& pl, const KernelConfig& c) {
@@ -146,11 +163,6 @@ KernelConfig from_entry(const prec_gpu_tune_entry_t* e) {
     c.rows = e->rows_per_cta;
     c.split = e->split_primes;
     return c;
-}
-
-bool same(const KernelConfig& a, const KernelConfig& b) {
-    return a.k1 == b.k1 && a.cg == b.cg && a.cmr == b.cmr && a.rmr == b.rmr && a.rows == b.rows &&
-           a.split == b.split;
 }
 
 // Device buffers and timing of one tuning run.

@@ -53,6 +53,20 @@ def test_host_wide(gpu, k):
             O.spot_check(got, a, b, 7 * k + i)
 
 
+def test_host_wide_long_rows(gpu):
+    """2^22 points of 64-bit digits (2^10 columns, 2^12-point rows), and the same
+    length once its table entry holds another configuration."""
+    try:
+        for i, (an, bn) in enumerate(_sizes(22, True)):
+            a, b = _operands(22, i, an, bn)
+            O.spot_check(gpu.mul(a, b, ntt=True), a, b, 22 + i)
+        gpu.tune_set(**dict(gpu.tune_get(22), rows_per_cta=2))
+        a, b = _operands(22, 0, 1500000, 1400001)
+        O.spot_check(gpu.mul(a, b, ntt=True), a, b, 22)
+    finally:
+        gpu.tune_reset()
+
+
 def test_long_32bit(gpu):
     """2^24 points of 32-bit digits: the reduced-residue set's kernels."""
     prev = gpu.set_wide_digits(False)
