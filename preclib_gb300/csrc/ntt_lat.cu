@@ -12,8 +12,8 @@
 // Shared memory has one spare word per eight (element i at P(i) = i + i/8):
 // conflict-free for both radix-8 passes.
 // Whole products, throughput kernels -> these: 2^14 points 18.4 -> 11.4 us, 2^15
-// 18.2 -> 12.5, 2^16 18.9 -> 13.8, 2^17 19.6 -> 16.0, 2^18 (64-bit digits) 31.6 ->
-// 29.4, at 5/8 27.2 -> 23.8.  From 2^19 points, and in batches, the GPU is full
+// 18.2 -> 12.5, 2^16 18.9 -> 13.8, 2^17 19.6 -> 14.9, 2^18 (64-bit digits) 31.6 ->
+// 28.1.  From 2^19 points, and in batches, the GPU is full
 // and the fewer passes of the throughput kernels count.
 #include <cooperative_groups.h>
 

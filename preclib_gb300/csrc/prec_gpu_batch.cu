@@ -4,8 +4,10 @@
 // src/mul_basic.cpp:278-284); its only producer of many independent products
 // is binary splitting (pi/pi_chudnovsky.cpp:141-144), one tree level at a
 // time.  Here a batch of device-resident products is planned once:
-//   * every product gets its transform length 2^k (the same plan as a single
-//     product), and products of one length form a length class;
+//   * short products run directly (direct_class, mul_direct.cuh); every other
+//     gets its transform length 2^k (the same plan as a single product), and
+//     products of one length, digit width and number of eighths kept form a
+//     class;
 //   * classes up to 2^12 points run one single-CTA product per CTA in one
 //     launch; larger classes run the four-step kernels once per pass over
 //     all their products (grid.z = product, per-product pointers in a
