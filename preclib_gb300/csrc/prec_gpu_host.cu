@@ -1211,6 +1211,16 @@ int prec_gpu_mul_device(const uint64_t* d_a, size_t an, const uint64_t* d_b, siz
         if ((r = lane_end(L, st))) return r;
         return 0;
     }
+    // A product of up to 2^12 points that goes into a caller's graph runs as the
+    // one kernel that uses nothing of the lane: a replay is outside the lane's
+    // order, and the direct kernel's column sums and counter are lane memory
+    // (allocated, too, which a capture refuses).
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone && 2 * ((uint64_t)an + bn) - 1 <= 1ull << kSmallMaxLog2) {
+        if ((r = plan_for(2 * (uint64_t)an, 2 * (uint64_t)bn, an + bn, pl))) return r;
+        return enqueue_ntt(c, L, d_a, an, d_b, bn, d_out, pl, st, c.d_err);
+    }
     if (direct_single(an, bn)) {
         if ((r = ensure_ws(L, direct_scratch_bytes(an, bn)))) return r;
         if ((r = lane_begin(L, st))) return r;
