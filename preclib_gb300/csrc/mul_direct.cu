@@ -102,21 +102,24 @@ __device__ __forceinline__ void group_sync() {
     else __syncthreads();
 }
 
+constexpr int kListThreads = 256;
+
 // Classes by list: a warp's lanes of one class take their places together.
 // (With every class's launch going over all items, mostly empty groups kept
 // the shared memory of half-empty CTAs: 44643 products of 58 .. 66 limbs,
 // two classes, 299 us of kernels; with lists 175.)
-__global__ void __launch_bounds__(256) k_direct_lists(const DirectItem* __restrict__ items, int count, uint32_t* lists,
+__global__ void __launch_bounds__(kListThreads) k_direct_lists(const DirectItem* __restrict__ items, int count, uint32_t* lists,
                                                       uint32_t* n) {
     pdl_enter();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const int64_t i = direct_first(blockIdx.x, kListThreads) + threadIdx.x;
+    const int lane = threadIdx.x & 31;
     const int cls = i < count ? direct_class(items[i].la, items[i].lb) : -1;
     const uint32_t same = __match_any_sync(0xffffffffu, cls);
     const int leader = __ffs(same) - 1;
     uint32_t at = 0;
     if (cls >= 0 && lane == leader) at = atomicAdd(&n[cls], (uint32_t)__popc(same));
     at = __shfl_sync(0xffffffffu, at, leader) + __popc(same & ((1u << lane) - 1));
-    if (cls >= 0) lists[(size_t)cls * count + at] = i;
+    if (cls >= 0) lists[(size_t)cls * count + at] = (uint32_t)i;
 }
 
 template <int R, int G>
@@ -136,9 +139,10 @@ __global__ void __launch_bounds__(DirectGeom<R, G>::THREADS) k_direct(const Dire
     uint32_t* sa = dsm + sub * D::WORDS;  // block i of a at (i + 1) * S
     uint32_t* sb = sa + D::A_BLKS * S;
     uint32_t* cols = sb + D::B_BLKS * S;
-    for (int base = blockIdx.x * D::PER_CTA; base < count; base += gridDim.x * D::PER_CTA) {
+    const int64_t stride = direct_first(gridDim.x, D::PER_CTA);
+    for (int64_t base = direct_first(blockIdx.x, D::PER_CTA); base < count; base += stride) {
         const bool live = base + sub < count;  // a group past the end runs an empty product
-        const int at = live ? base + sub : count - 1;
+        const int64_t at = live ? base + sub : count - 1;
         const DirectItem d = items[list ? list[at] : at];
         const bool swap = d.la < d.lb;
         const uint64_t* __restrict__ pa = swap ? d.b : d.a;
@@ -232,7 +236,7 @@ __global__ void __launch_bounds__(DirectGeom<R, G>::THREADS) k_direct(const Dire
 #define PREC_DIRECT(X) X(0, 8, 16) X(1, 12, 16) X(2, 8, 32) X(3, 8, 64) X(4, 8, 128)
 
 void launch_direct_lists(const DirectItem* d_items, int count, uint32_t* lists, uint32_t* n, cudaStream_t st) {
-    launch_pdl(false, k_direct_lists, (count + 255) / 256, 256, 0, st, d_items, count, lists, n);
+    launch_pdl(false, k_direct_lists, direct_ctas(count, kListThreads, 0x7fffffff), kListThreads, 0, st, d_items, count, lists, n);
     count_launches(1);
 }
 
@@ -243,9 +247,8 @@ void launch_direct_batch(const DirectItem* d_items, int count, int cls, cudaStre
 #define X(C, R, G)                                                                                          \
     if (cls == C) {                                                                                         \
         using D = DirectGeom<R, G>;                                                                         \
-        const int grid = (count + D::PER_CTA - 1) / D::PER_CTA;                                             \
-        launch_pdl(false, k_direct<R, G>, grid < cap ? grid : cap, D::THREADS, D::SMEM, st, d_items, count, \
-                   list, n);                                                                                \
+        launch_pdl(false, k_direct<R, G>, direct_ctas(count, D::PER_CTA, cap), D::THREADS, D::SMEM, st,     \
+                   d_items, count, list, n);                                                                \
         count_launches(1);                                                                                  \
     }
     PREC_DIRECT(X)

@@ -49,6 +49,15 @@ bool direct_single(uint64_t la, uint64_t lb);
 // scratch bytes of a single direct product (column sums)
 size_t direct_scratch_bytes(uint64_t la, uint64_t lb);
 
+// CTAs that take `count` items `per` at a time, at most `cap`.  A CTA's items are
+// per * block, and per * (CTAs) further each round: 64-bit, as a batch may hold
+// 2^31 - 1 products and the round past the last one lies beyond that.
+__host__ __device__ inline int direct_ctas(int count, int per, int cap) {
+    const int64_t n = ((int64_t)count + per - 1) / per;
+    return n < cap ? (int)n : cap;
+}
+__host__ __device__ inline int64_t direct_first(uint32_t block, int per) { return (int64_t)block * per; }
+
 // Every item's index into its class's list: lists[cls * count ..], their
 // lengths in n[kDirectClasses], zero before.
 void launch_direct_lists(const DirectItem* d_items, int count, uint32_t* lists, uint32_t* n, cudaStream_t st);
