@@ -349,6 +349,11 @@ __global__ void __launch_bounds__(ColGeom<M>::THREADS) k_fft_inv_cols(FftArgs f)
         coef[(uint64_t)pos * N2h + c] = make_longlong2(x0, x1);
         coef[(uint64_t)(pos + H) * N2h + c] = make_longlong2(y0, y1);
     }
+    {   // no coefficient past the last digits' product
+        const uint64_t end = f.da + f.db - 1, i = 2 * ((uint64_t)pos * N2h + c), j = i + 2 * (uint64_t)H * N2h;
+        const bool past = on && ((i >= end && x0) || (i + 1 >= end && x1) || (j >= end && y0) || (j + 1 >= end && y1));
+        if (__any_sync(0xffffffffu, past) && (threadIdx.x & 31) == 0) atomicOr(f.err, kDevErrCarry);
+    }
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long v = __shfl_xor_sync(0xffffffffu, dmax, o);
         dmax = v > dmax ? v : dmax;
@@ -362,22 +367,15 @@ __global__ void __launch_bounds__(ColGeom<M>::THREADS) k_fft_inv_cols(FftArgs f)
     if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned long long*>(f.maxdist), dmax);
 }
 
-// Carry: limbs of the product sum c_i 2^(bi) from the signed coefficients.
-// c_i + 2^62 - 2^(62-b) (for i = 0: c_i + 2^62) is positive and adds up to the
-// same number plus 2^(bN + 62 - b), past every limb of the product, so the
-// carries are 0 or 1: S_m, the sum of the coefficients that start in limb m,
-// gives limb lo64(S_m) + hi64(S_m-1) + carry, as in the NTT band.  The
-// product runs as one cluster of up to 8 CTAs: each puts its carry aggregate
+// Carry: limbs of the product sum c_i 2^(bi) from the signed coefficients
+// (fft_limb_sum).  The product runs as one cluster of up to 8 CTAs: each puts its carry aggregate
 // into every CTA's shared memory, one cluster barrier, and every limb is
 // written once, final.  (As separate CTAs joined by the last one over the
 // carry maps of signed limbs this kernel took 9 - 11 us.)
-constexpr int kFftCarryThreads = 512;
-constexpr int kFftCarryCluster = 8;
-
-template <int L>
-__global__ void __launch_bounds__(kFftCarryThreads) k_fft_carry(FftArgs f) {
+template <int L, int NW>
+__global__ void __launch_bounds__(32 * NW) k_fft_carry(FftArgs f) {
     namespace cg = cooperative_groups;
-    __shared__ uint32_t s_wg[kFftCarryThreads / 32], s_wp[kFftCarryThreads / 32];
+    __shared__ uint32_t s_wg[NW], s_wp[NW];
     __shared__ uint32_t s_blk[kFftCarryCluster];
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t rank = blockIdx.x, ranks = gridDim.x;
@@ -392,28 +390,13 @@ __global__ void __launch_bounds__(kFftCarryThreads) k_fft_carry(FftArgs f) {
         return;
     }
     const int b = f.b;
-    const int64_t m0 = ((int64_t)rank * kFftCarryThreads + threadIdx.x) * L;
-    // one limb past the product, checked to be zero, where the coefficients cover it
-    const int64_t lim = (int64_t)f.lout + ((uint64_t)b * f.ncoef >= 64 * (f.lout + 1) ? 1 : 0);
+    const int64_t m0 = ((int64_t)rank * 32 * NW + threadIdx.x) * L;
+    const int64_t lim = (int64_t)f.lout + kFftPastLimbs;
     u128 T[L + 1];  // S of limbs m0 - 1 .. m0 + L - 1
 #pragma unroll
     for (int k = 0; k <= L; ++k) {
         const int64_t m = m0 + k - 1;
-        T[k] = 0;
-        if (m < 0 || m >= lim) continue;
-        const uint32_t bit = (uint32_t)m * 64;
-        const uint32_t i0 = (bit + b - 1) / b;
-        const uint32_t off = i0 * b - bit;
-        long long c[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) c[u] = off + u * b < 64 && i0 + u < f.ncoef ? coef[i0 + u] : 0;
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            if (off + u * b < 64 && i0 + u < f.ncoef) {
-                const uint64_t v = (uint64_t)c[u] + (1ull << 62) - (i0 + u ? 1ull << (62 - b) : 0);
-                T[k] += (u128)v << (off + u * b);
-            }
-        }
+        T[k] = m < lim ? fft_limb_sum([&](uint32_t i) { return coef[i]; }, f.ncoef, b, m) : (u128)0;
     }
     u128 S[L];
 #pragma unroll
@@ -430,9 +413,8 @@ __global__ void __launch_bounds__(kFftCarryThreads) k_fft_carry(FftArgs f) {
     }
     __syncthreads();
     // warp aggregates as bits; the CTA's own aggregate to every CTA of the cluster
-    constexpr int NW = kFftCarryThreads / 32;
-    const uint32_t bg = __ballot_sync(0xffffffffu, lane < NW && s_wg[lane & (NW - 1)] != 0);
-    const uint32_t bp = __ballot_sync(0xffffffffu, lane < NW && s_wp[lane & (NW - 1)] != 0);
+    const uint32_t bg = __ballot_sync(0xffffffffu, lane < NW && s_wg[lane] != 0);
+    const uint32_t bp = __ballot_sync(0xffffffffu, lane < NW && s_wp[lane] != 0);
     cluster.barrier_wait();
     if (ranks > 1) {
         if (warp == 0 && lane < (int)ranks) {
@@ -451,7 +433,7 @@ __global__ void __launch_bounds__(kFftCarryThreads) k_fft_carry(FftArgs f) {
         c = ((gbits >> k) & 1) || (v[k] == ~0ull && c);
         const int64_t m = m0 + k;
         if (m < (int64_t)f.lout) f.out[m] = x;
-        else if (m < lim && x != 0) atomicOr(f.err, kDevErrCarry);  // a product fits La+Lb limbs
+        else if (m < lim && x != fft_past_value(b, f.ncoef, m)) atomicOr(f.err, kDevErrCarry);  // a product fits La+Lb limbs
     }
 }
 
@@ -477,24 +459,22 @@ void fft_build_table(double2* tw, cudaStream_t st) {
     count_launches(1);
 }
 
-template <int L>
+template <int L, int NW>
 static void launch_carry(const FftArgs& f, cudaStream_t st) {
-    const uint64_t per = (uint64_t)kFftCarryThreads * L;
-    uint64_t n = (f.lout + 1 + per - 1) / per;
-    if (n > kFftCarryCluster) n = kFftCarryCluster;
+    const unsigned n = fft_carry_ctas(f.lout);
     cudaLaunchAttribute attr[2] = {};
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = (unsigned)n;
+    attr[1].val.clusterDim.x = n;
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = (unsigned)n;
-    cfg.blockDim = kFftCarryThreads;
+    cfg.gridDim = n;
+    cfg.blockDim = 32 * NW;
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    cudaLaunchKernelEx(&cfg, k_fft_carry<L>, f);
+    cudaLaunchKernelEx(&cfg, k_fft_carry<L, NW>, f);
 }
 
 #define PREC_FFT_LOG2(X) X(3) X(4) X(5) X(6) X(7) X(8)
@@ -514,11 +494,12 @@ int fft_launch(const FftArgs& f, cudaStream_t st) {
     if (f.k1 == M) launch_pdl(false, k_fft_inv_cols<M>, ((1u << f.k2) / 2 + ColGeom<M>::C - 1) / ColGeom<M>::C, ColGeom<M>::THREADS, 0, st, f);
     PREC_FFT_LOG2(X)
 #undef X
-    // limbs per thread: 8 CTAs of 512 threads cover 4096 limbs of one each
-    const uint64_t one = (uint64_t)kFftCarryThreads * kFftCarryCluster;
-    if (f.lout <= one) launch_carry<1>(f, st);
-    else if (f.lout <= 2 * one) launch_carry<2>(f, st);
-    else launch_carry<3>(f, st);
+    static_assert(fft_carry_limbs(2 * 6144) == 3, "the band's longest product");
+    const int L = fft_carry_limbs(f.lout), NW = fft_carry_warps(f.lout);
+#define X(LL, W) \
+    if (L == LL && NW == W) launch_carry<LL, W>(f, st);
+    X(1, 16) X(1, 17) X(2, 16) X(2, 17) X(3, 16) X(3, 17)
+#undef X
     count_launches(5);
     return (int)cudaGetLastError();
 }
