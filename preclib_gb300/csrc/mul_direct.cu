@@ -268,6 +268,7 @@ struct DirectArgs {
     uint64_t* out;
     uint64_t* sums;     // per limb m: T_m = S_2m + 2^32 S_2m+1, two words
     uint32_t* counter;
+    int* err;
     int la, lb, na, nb; // limbs and digit blocks
 };
 
@@ -411,6 +412,8 @@ __global__ void __launch_bounds__(kGridThreads) k_direct_grid(DirectArgs f) {
         };
         const bool cin = block_carry(G, P, sh, cin_fn);
         limbs_finish<L>(m0, (uint64_t)lout, v, gbits, cin, f.out);
+        const int last = lout - 1 - m0;  // a product fits La+Lb limbs
+        if (last >= 0 && last < L && limbs_overflow<L>(last, T, v, gbits, cin)) atomicOr(f.err, kDevErrCarry);
         __syncthreads();
         carry = sh.block_cin != 0;
         __syncthreads();
@@ -439,7 +442,7 @@ size_t direct_scratch_bytes(uint64_t la, uint64_t lb) {
 #define PREC_DIRECT_GRID(X) X(1) X(2) X(4) X(8)
 
 void launch_direct_single(const uint64_t* a, uint64_t la, const uint64_t* b, uint64_t lb, uint64_t* out,
-                          uint8_t* scratch, uint32_t* counter, cudaStream_t st) {
+                          uint8_t* scratch, uint32_t* counter, int* err, cudaStream_t st) {
     const bool swap = la < lb;
     DirectArgs f;
     f.a = swap ? b : a;
@@ -451,6 +454,7 @@ void launch_direct_single(const uint64_t* a, uint64_t la, const uint64_t* b, uin
     f.out = out;
     f.sums = reinterpret_cast<uint64_t*>(scratch);
     f.counter = counter;
+    f.err = err;
     int cb = 1;
     while (cb < 8 && (f.na + cb - 1) / cb > device_sm_count()) cb *= 2;
 #define X(C)                                                                                           \

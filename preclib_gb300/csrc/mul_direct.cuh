@@ -66,9 +66,10 @@ void launch_direct_lists(const DirectItem* d_items, int count, uint32_t* lists, 
 void launch_direct_batch(const DirectItem* d_items, int count, int cls, cudaStream_t st,
                          const uint32_t* list = nullptr, const uint32_t* n = nullptr);
 // counter: one device word, zero before the first call, left zero by every
-// call; calls that share it must not overlap
+// call; calls that share it must not overlap.  A carry out of the product sets
+// kDevErrCarry in *err.
 void launch_direct_single(const uint64_t* a, uint64_t la, const uint64_t* b, uint64_t lb, uint64_t* out,
-                          uint8_t* scratch, uint32_t* counter, cudaStream_t st);
+                          uint8_t* scratch, uint32_t* counter, int* err, cudaStream_t st);
 int configure_direct();
 
 }  // namespace precgpu

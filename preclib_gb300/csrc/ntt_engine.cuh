@@ -649,7 +649,7 @@ __device__ __forceinline__ bool block_carry_in0(bool G, bool P, BlockCarryShared
 // v_k = lo64(T_k) + hi(T_{k-1}) with generate bit g_k.  Returns (G, P):
 // the carry out with carry-in 0, and whether a carry-in passes through.
 template <int L>
-__device__ __forceinline__ void limbs_from_sums(const u128 (&T)[L], uint64_t prev_hi, uint64_t (&v)[L],
+__host__ __device__ __forceinline__ void limbs_from_sums(const u128 (&T)[L], uint64_t prev_hi, uint64_t (&v)[L],
                                                 uint32_t& gbits, bool& G, bool& P) {
     gbits = 0;
     bool c = false;
@@ -679,6 +679,23 @@ __device__ __forceinline__ void limbs_finish(int64_t m0, uint64_t lout, const ui
         c = g || (v[k] == ~0ull && c);
         if (m0 + k < (int64_t)lout) out[m0 + k] = r;
     }
+}
+
+// Whether a product that ends with this thread's limb `last` runs on past it:
+// the carry out of that limb, or what its own sum leaves for the next one.
+template <int L>
+__host__ __device__ __forceinline__ bool limbs_overflow(int last, const u128 (&T)[L], const uint64_t (&v)[L],
+                                                       uint32_t gbits, bool cin) {
+    bool c = cin;
+    uint64_t hi = 0;
+#pragma unroll
+    for (int k = 0; k < L; ++k) {
+        if (k <= last) {
+            c = ((gbits >> k) & 1) || (v[k] == ~0ull && c);
+            hi = (uint64_t)(T[k] >> 64);
+        }
+    }
+    return c || hi != 0;
 }
 
 }  // namespace precgpu

@@ -1224,7 +1224,7 @@ int prec_gpu_mul_device(const uint64_t* d_a, size_t an, const uint64_t* d_b, siz
     if (direct_single(an, bn)) {
         if ((r = ensure_ws(L, direct_scratch_bytes(an, bn)))) return r;
         if ((r = lane_begin(L, st))) return r;
-        launch_direct_single(d_a, an, d_b, bn, d_out, L.ws, L.direct_counter, st);
+        launch_direct_single(d_a, an, d_b, bn, d_out, L.ws, L.direct_counter, c.d_err, st);
         CK(cudaGetLastError());
         if ((r = lane_end(L, st))) return r;
         return 0;
