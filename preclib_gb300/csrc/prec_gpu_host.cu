@@ -1024,7 +1024,7 @@ static int host_mul(const uint64_t* a, size_t an, const uint64_t* b, size_t bn, 
     // the kernels start on a's forward columns while b is copied
     const bool overlap = !use_fft && !blocked && pl.path == 1 && c.split_primes && (pl.split || pl.k >= kHostOverlapMinLog2);
     const bool staged = !blocked && !overlap && lout <= kStagedLimbs && ensure_pin(L) == 0;
-    if ((r = ensure_io(L, la_pad + lb_pad + lout))) return r;
+    if (!staged && (r = ensure_io(L, la_pad + lb_pad + lout))) return r;
     uint64_t* buf = staged ? L.pin : L.io;
     uint64_t* d_a = buf;
     uint64_t* d_b = square ? d_a : buf + la_pad;
