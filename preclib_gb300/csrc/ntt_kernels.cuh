@@ -57,7 +57,7 @@ struct ProdPtrs;
 // Four-step twiddle table of one set and length: Shoup pairs in the column
 // passes' own order, entry (direction * primes + prime) * N + s * N2 + i2 is
 // w^(+-i2 bitrev(s)); the inverse one also carries the prime's CRT scale.
-// Built once at start-up for the lengths that batches use (tables of a few
+// Built once per length, when a batch first has a class for it (tables of a few
 // MB that stay in L2 while a class's products go by).
 constexpr int kTabMinLog2 = 13;
 constexpr int kTabMaxLog2[2] = {18, 19};  // sets 0 and 2

@@ -46,6 +46,7 @@ struct Cls {
     int square = 0;               // every product of the class is a square
     Plan pl;                      // class-wide plan (k, set, k1, k2, rows, crt)
     std::vector<int> items;       // indices into the batch's products
+    const uint2* t4 = nullptr;    // four-step twiddle table (group_columns)
     size_t ws_per = 0;            // workspace bytes per product (four-step)
     int per_chunk = 0;            // products per chunk
     std::vector<Chunk> chunks;
@@ -168,7 +169,7 @@ static void batch_enqueue(prec_gpu_batch* b, cudaStream_t origin, bool branch) {
             args.crt = c.pl.crt;
             args.crt5 = c.pl.crt5;
             args.f = ctx_field(c.pl.set);
-            args.t4 = ctx_fourstep(c.pl.set, c.pl.k);
+            args.t4 = c.t4;
             for (const Chunk& ch : c.chunks) {
                 if (c.persistent) {
                     const size_t bytes = (kClassHdrWords + (size_t)kClassProdWords * ch.count) * sizeof(uint32_t);
@@ -228,9 +229,9 @@ static void group_columns(Cls& c) {
     if (d.k1 != c.pl.k1 || d.cg != c.pl.cg || d.cmr != c.pl.cmr) return;
     const int g = col_batch_group(c.pl.k1);
     // (instantiated: set 0 up to 2^18 points, set 2 up to 2^19)
-    if (g == c.pl.cg || c.pl.k > (set_wide(c.pl.set) ? 19 : 18) || !ctx_fourstep(c.pl.set, c.pl.k)) return;
+    if (g == c.pl.cg || c.pl.k > (set_wide(c.pl.set) ? 19 : 18)) return;
     const uint64_t ctas = (uint64_t)c.items.size() * c.pl.nprimes << c.pl.k2;
-    if (ctas / g >= (uint64_t)device_sm_count() / 2) c.pl.cg = g;
+    if (ctas / g >= (uint64_t)device_sm_count() / 2 && (c.t4 = ctx_fourstep_locked(c.pl.set, c.pl.k))) c.pl.cg = g;
 }
 
 // Plans a batch and uploads its descriptors.  `oneshot` (prec_gpu_mul_batch):

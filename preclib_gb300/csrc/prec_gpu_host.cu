@@ -310,14 +310,15 @@ struct Ctx {
     int* d_err = nullptr;
     int* h_err = nullptr;
     double2* fft_tw = nullptr;  // FP64 band twiddles
-    void* t4_mem = nullptr;     // four-step twiddle tables: sets 0 and 2, by log2 of the length
-    const uint2* t4[2][kMaxLog2 + 1] = {};
+    uint2* t4[2][kMaxLog2 + 1] = {};  // four-step twiddle tables in use: sets 0 and 2, by log2 of the length
     FieldArgs field[kSets] = {};
     cudaMemPool_t pool = nullptr;
     bool split_primes = true;  // PREC_GPU_PRIME_STREAMS=0 runs the primes in one launch per kernel
     std::vector<std::unique_ptr<Lane>> lanes;
     std::atomic<uint64_t> gen{0};  // bumped by shutdown: threads then take new lanes
 };
+
+static Ctx g_ctx;
 
 // 64-bit digits (set 2) for single products: on unless PREC_GPU_WIDE_DIGITS=0;
 // prec_gpu_set_wide_digits changes it at run time
@@ -333,8 +334,6 @@ bool wide_digits() {
     }
     return w != 0;
 }
-
-static Ctx g_ctx;
 
 static thread_local GraphRecorder* t_recorder = nullptr;
 GraphRecorder*& thread_recorder() { return t_recorder; }
@@ -487,31 +486,35 @@ static int build_tables(Ctx& c) {
     return 0;
 }
 
-// The four-step tables of every length in its default configuration (90 MB).
-static int build_fourstep_tables(Ctx& c) {
-    size_t total = 0;
-    for (int w = 0; w < 2; ++w)
-        for (int k = kTabMinLog2; k <= kTabMaxLog2[w]; ++k)
-            if (!w || k >= kWideMinLog2) total += fourstep_entries(kSetPrimes[w ? kWideSet : 0], k);
-    CK(cudaMalloc(&c.t4_mem, total * sizeof(uint2)));
-    uint2* p = static_cast<uint2*>(c.t4_mem);
-    for (int w = 0; w < 2; ++w)
-        for (int k = kTabMinLog2; k <= kTabMaxLog2[w]; ++k) {
-            if (w && k < kWideMinLog2) continue;
-            const int set = w ? kWideSet : 0, k1 = default_config(k).k1;
-            const CrtConst cc = w ? CrtConst{} : crt_for(0, k);
-            const Crt5Const c5 = w ? crt5_for(set, k) : Crt5Const{};
-            launch_fourstep_table(p, c.field[set], w ? c5.fold : cc.fold, kSetPrimes[set], k1, k - k1, nullptr);
-            c.t4[w][k] = p;
-            p += fourstep_entries(kSetPrimes[set], k);
-        }
-    CK(cudaGetLastError());
-    return 0;
-}
-
-const uint2* ctx_fourstep(int set, int k) {
-    if (set != 0 && set != kWideSet) return nullptr;
-    return g_ctx.t4[set == kWideSet][k];
+// A length's table is made when a batch first has a class for it, and kept (0.4
+// to 42 MB, up to 1 ms; all lengths 90 MB): most processes batch few lengths or
+// none.  From the library's pool: an allocation there waits for no device work.
+const uint2* ctx_fourstep_locked(int set, int k) {
+    Ctx& c = g_ctx;
+    const int w = set == kWideSet ? 1 : 0;
+    if ((set != 0 && set != kWideSet) || k < (w ? kWideMinLog2 : kTabMinLog2) || k > kTabMaxLog2[w]) return nullptr;
+    if (c.t4[w][k]) return c.t4[w][k];
+    const int k1 = default_config(k).k1;
+    const CrtConst cc = w ? CrtConst{} : crt_for(0, k);
+    const Crt5Const c5 = w ? crt5_for(set, k) : Crt5Const{};
+    cudaStream_t st = nullptr;
+    void* p = nullptr;
+    cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (!e) e = cudaMallocFromPoolAsync(&p, fourstep_entries(kSetPrimes[set], k) * sizeof(uint2), c.pool, st);
+    if (!e) {
+        launch_fourstep_table(static_cast<uint2*>(p), c.field[set], w ? c5.fold : cc.fold, kSetPrimes[set], k1, k - k1, st);
+        e = cudaGetLastError();
+        // (any stream may read it from here on)
+        const cudaError_t es = cudaStreamSynchronize(st);
+        if (!e) e = es;
+    }
+    if (e && p) cudaFreeAsync(p, st);
+    if (st) cudaStreamDestroy(st);
+    if (e) {  // the class runs without a table
+        cudaGetLastError();
+        return nullptr;
+    }
+    return c.t4[w][k] = static_cast<uint2*>(p);
 }
 
 static int init_locked(Ctx& c, int device) {
@@ -546,7 +549,6 @@ static int init_locked(Ctx& c, int device) {
     CK(cudaGetLastError());
     int r = build_tables(c);
     if (r) return r;
-    if ((r = build_fourstep_tables(c))) return r;
     CK(cudaDeviceSynchronize());
     c.ready.store(true, std::memory_order_release);
     // a saved tuning table (an invalid file leaves the defaults in place)
@@ -1158,9 +1160,11 @@ void prec_gpu_shutdown(void) {
     c.gen.fetch_add(1, std::memory_order_relaxed);  // every thread takes a new lane next time
     cudaFree(c.tables);
     cudaFree(c.fft_tw);
-    cudaFree(c.t4_mem);
-    c.t4_mem = nullptr;
-    std::memset(c.t4, 0, sizeof(c.t4));
+    for (auto& set : c.t4)
+        for (uint2*& t : set) {
+            cudaFree(t);
+            t = nullptr;
+        }
     cudaFree(c.d_err);
     cudaFreeHost(c.h_err);
     if (c.pool) cudaMemPoolDestroy(c.pool);

@@ -112,8 +112,9 @@ int ctx_ensure_ws_locked(size_t bytes);
 std::mutex& ctx_mutex();
 int ctx_init_locked(int device);
 const FieldArgs& ctx_field(int set);
-// the four-step twiddle table of sets 0 and 2 (nullptr: none for this length)
-const uint2* ctx_fourstep(int set, int k);
+// the four-step twiddle table of sets 0 and 2, made on first use (nullptr: none
+// for this length, or no memory for it); call with the context lock held
+const uint2* ctx_fourstep_locked(int set, int k);
 int* ctx_device_err();
 // reads and clears the device error bits (takes the library lock); 0 or a
 // PREC_GPU_E_* code
