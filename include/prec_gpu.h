@@ -115,11 +115,12 @@ typedef struct {
 } prec_gpu_tune_entry_t;
 
 /* Times the configurations of every length 2^kmin .. 2^kmax (clamped to
- * 13 .. 26) on the current device with balanced random operands of
- * 2^(k-2) limbs each, by coordinate descent from the default (per-prime
- * streams, rows per CTA, columns per CTA, radix caps, then the column/row
- * split).  A candidate counts only if its product equals the default
- * configuration's bit for bit; the fastest is installed.  Writes up to
+ * 13 .. 26) on the current device with balanced random operands that need 8,
+ * 7, 6 and 5 eighths of the length, by coordinate descent from the default
+ * (per-prime streams, rows per CTA, columns per CTA, radix caps, then the
+ * column/row split).  A candidate counts only if its products equal the default
+ * configuration's bit for bit; one is installed if it is faster on the whole
+ * length (2^(k-2) limbs each: the entry's ms) and on the four together.  Writes up to
  * `cap` entries to `out` (may be NULL) and the number of lengths to *count. */
 int prec_gpu_autotune(int kmin, int kmax, prec_gpu_tune_entry_t *out, size_t cap, size_t *count);
 

@@ -100,6 +100,23 @@ KernelConfig tuned_config(int k);
 // fills the four-step fields of a plan from a configuration
 void apply_config(Plan& pl, const KernelConfig& c);
 
+// The autotuner's rule.  Times (ms) of one length's products that need 8, 7, 6
+// and 5 eighths of the transform, each with the eighths kept that the
+// configuration has kernels for: a candidate replaces the best one so far if the
+// whole transform is 1% faster and the four together are too.  (Truncated
+// kernels exist for default configurations only: 1% on whole transforms would
+// be paid with up to a third on the others.)
+constexpr int kTuneShapes = 4;  // 8, 7, 6, 5 eighths
+inline bool tune_better(const float (&cand)[kTuneShapes], const float (&best)[kTuneShapes]) {
+    float c = 0.f, b = 0.f;
+    for (int i = 0; i < kTuneShapes; ++i) {
+        if (!(cand[i] > 0.f)) return false;  // failed, or another result
+        c += cand[i];
+        b += best[i];
+    }
+    return cand[0] < best[0] * 0.99f && c < b * 0.99f;
+}
+
 // Enqueues one NTT-band product with plan `pl` on device pointers (the
 // library workspace must hold pl.work_bytes: ctx_ensure_ws_locked).  Call
 // with the context lock held.

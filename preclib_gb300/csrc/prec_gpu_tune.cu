@@ -6,8 +6,9 @@
 // product runs each prime's kernels on its own stream.  plan_for reads the
 // table for every product (single, batch, serving loop), so a tuned length
 // changes every later product of that length.  The autotuner times the
-// candidates on the device with balanced random operands, keeps a
-// candidate only if its product equals the default configuration's bit for
+// candidates on the device with balanced random operands that need 8, 7, 6 and
+// 5 eighths of the length (tune_better), keeps a
+// candidate only if its products equal the default configuration's bit for
 // bit, and installs the fastest.  The reference has nothing to tune (one
 // CPU code path, src/mul_ntt.cpp); the table replaces the fixed choices a
 // GPU port would otherwise hard-code.
@@ -169,7 +170,9 @@ KernelConfig from_entry(const prec_gpu_tune_entry_t* e) {
 struct Tuner {
     cudaStream_t st = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
-    uint64_t *a = nullptr, *b = nullptr, *out = nullptr, *ref = nullptr;
+    uint64_t *a = nullptr, *b = nullptr, *out = nullptr;
+    uint64_t* ref = nullptr;  // the default configuration's product of ref_k, ref_e
+    int ref_k = 0, ref_e = 0;
     uint8_t* flush = nullptr;
     int* flag = nullptr;
     size_t flush_bytes = (size_t)256 << 20;  // twice the L2
@@ -201,29 +204,36 @@ struct Tuner {
         return cuda_code(e);
     }
 
-    // median product time of configuration c for length 2^k (la = lb =
-    // 2^(k-2) limbs); -1 if it fails or differs from the reference product
-    float time(int k, const Plan& base, const KernelConfig& c, bool make_ref) {
-        const uint64_t n = 1ull << (k - 2);
-        Plan pl = base;
+    // the product of length 2^k that needs e eighths of it (la = lb = e 2^(k-5)
+    // limbs) under configuration c
+    bool product(int k, int e, const KernelConfig& c, uint64_t* to) {
+        const uint64_t n = (uint64_t)e << (k - 5);
+        Plan pl;
+        if (plan_for(2 * n, 2 * n, 2 * n, pl, false, true) || pl.path != 1 || pl.k != k) return false;
         apply_config(pl, c);
-        if (ctx_enqueue_ntt_locked(a, n, b, n, out, pl, st)) return -1.f;
-        if (cudaStreamSynchronize(st) != cudaSuccess) return -1.f;
-        if (make_ref) {
-            if (cudaMemcpyAsync(ref, out, 2 * n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, st)) return -1.f;
-        } else {
-            int h = 0;
-            cudaMemsetAsync(flag, 0, sizeof(int), st);
-            k_tune_diff<<<8 * device_sm_count(), 256, 0, st>>>(out, ref, 2 * n, flag);
-            count_launches(1);
-            cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, st);
-            if (cudaStreamSynchronize(st) != cudaSuccess || h) return -1.f;
+        pl.keep = plan_keep(pl, 2 * n, 2 * n);
+        return ctx_enqueue_ntt_locked(a, n, b, n, to, pl, st) == 0;
+    }
+
+    // its median time; -1 if it fails or differs from the default configuration's
+    float time(int k, int e, const KernelConfig& c) {
+        if (ref_k != k || ref_e != e) {
+            if (!product(k, e, default_config(k), ref)) return -1.f;
+            ref_k = k;
+            ref_e = e;
         }
+        if (!product(k, e, c, out)) return -1.f;
+        int h = 0;
+        cudaMemsetAsync(flag, 0, sizeof(int), st);
+        k_tune_diff<<<8 * device_sm_count(), 256, 0, st>>>(out, ref, (size_t)e << (k - 4), flag);
+        count_launches(1);
+        cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, st);
+        if (cudaStreamSynchronize(st) != cudaSuccess || h) return -1.f;
         std::vector<float> ms;
         for (int r = 0; r < reps; ++r) {
             cudaMemsetAsync(flush, r & 0xFF, flush_bytes, st);
             cudaEventRecord(e0, st);
-            if (ctx_enqueue_ntt_locked(a, n, b, n, out, pl, st)) return -1.f;
+            if (!product(k, e, c, out)) return -1.f;
             cudaEventRecord(e1, st);
             if (cudaEventSynchronize(e1) != cudaSuccess) return -1.f;
             float t = 0.f;
@@ -238,23 +248,30 @@ struct Tuner {
 // Coordinate descent from the default configuration of length 2^k.
 int tune_one(Tuner& T, int k, KernelConfig& best, float& best_ms, float& default_ms) {
     const uint64_t n = 1ull << (k - 2);
-    Plan base;
-    int r = plan_for(2 * n, 2 * n, 2 * n, base);
-    if (r) return r;
-    if (base.path != 1 || base.k != k) return PREC_GPU_E_INTERNAL;
     k_tune_fill<<<8 * device_sm_count(), 256, 0, T.st>>>(T.a, n, 0x1234567ull + k);
     k_tune_fill<<<8 * device_sm_count(), 256, 0, T.st>>>(T.b, n, 0x7654321ull + k);
     count_launches(2);
     if (cudaGetLastError() != cudaSuccess) return PREC_GPU_E_CUDA;
     best = default_config(k);
-    best_ms = default_ms = T.time(k, base, best, true);
-    if (best_ms < 0) return PREC_GPU_E_INTERNAL;
+    // the best configuration's; those of the truncated lengths when a candidate
+    // first needs them
+    float times[kTuneShapes] = {T.time(k, 8, best)};
+    if (times[0] < 0) return PREC_GPU_E_INTERNAL;
+    best_ms = default_ms = times[0];
     auto consider = [&](const KernelConfig& c) {
         if (!config_valid(k, c) || same(c, best)) return;
-        const float t = T.time(k, base, c, false);
-        if (t > 0 && t < best_ms * 0.99f) {
+        float t[kTuneShapes];
+        t[0] = T.time(k, 8, c);
+        if (!(t[0] > 0 && t[0] < times[0] * 0.99f)) return;  // tune_better's first condition
+        for (int i = 1; i < kTuneShapes; ++i) {
+            if (times[i] == 0.f) times[i] = T.time(k, 8 - i, best);
+            if (times[i] < 0) return;
+            t[i] = T.time(k, 8 - i, c);
+        }
+        if (tune_better(t, times)) {
             best = c;
-            best_ms = t;
+            std::copy(t, t + kTuneShapes, times);
+            best_ms = t[0];
         }
     };
     auto tune_rows = [&]() {
