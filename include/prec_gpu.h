@@ -163,13 +163,17 @@ int prec_gpu_mul_device(const uint64_t *d_a, size_t an, const uint64_t *d_b, siz
  * before the first and after every kernel of the product, synchronises,
  * and writes each kernel's device time (ms) to stage_ms[0 .. *nstages)
  * (at most 8).  It always takes the NTT band's kernels, also where
- * prec_gpu_mul_device forms a short product directly.  Kernel names: prec_gpu_stage_name(path, i) with the path of
- * prec_gpu_stats_t.  Replaces: the wall-clock phase timers of the
+ * prec_gpu_mul_device forms a short product directly.  Kernel names:
+ * prec_gpu_stage_name(path, i) with the path of prec_gpu_stats_t; on path 1
+ * they name the passes, which a product of 2^13 .. 2^18 points runs with kernels
+ * of its own (k_fwd_cols_lat, k_rows_lat, k_inv_cols_lat and, up to 16384 limbs,
+ * k_crt_cluster).  Replaces: the wall-clock phase timers of the
  * reference's benches (test/bench_ntt.cpp:25-58, pi/pi_chudnovsky.cpp:183-188). */
 int prec_gpu_mul_device_profile(const uint64_t *d_a, size_t an, const uint64_t *d_b, size_t bn,
                                 uint64_t *d_out, void *stream, float *stage_ms, int *nstages);
 
-/* Kernel name of stage `stage` of path `path` ("" if out of range). */
+/* Kernel name of stage `stage` of path `path` (0 single CTA, 1 four-step,
+ * 2 FP64 FFT; "" if out of range). */
 const char *prec_gpu_stage_name(int path, int stage);
 
 /* The product of prec_gpu_mul_device for callers that cannot allocate device

@@ -112,13 +112,15 @@ PrimeC prime_constants(uint32_t p) {
 
 constexpr int kMaxStages = 8;
 
-// kernel names of each path, in launch order
+// kernel names of each path, in launch order (path 1: the throughput kernels; a
+// product of 2^13 .. 2^18 points runs the same passes as the kernels of
+// ntt_lat.cu, a chunked CRT launches its last one several times)
 static const char* const kStageNames[3][kMaxStages] = {
     {"k_small"},
     {"k_fwd_cols", "k_rows", "k_inv_cols", "k_crt_carry"},
-    {"k_fft_fwd_cols", "k_fft_rows", "k_fft_inv_cols", "k_fft_carry"},
+    {"k_fft_digits", "k_fft_fwd_cols", "k_fft_rows", "k_fft_inv_cols", "k_fft_carry"},
 };
-static const int kStageCount[3] = {1, 4, 4};
+static const int kStageCount[3] = {1, 4, 5};
 
 constexpr size_t kStatBytes = 16;       // device status block (error bits, FFT distance)
 constexpr size_t kFftBandMin = 192;     // src/mul_basic.cpp:4 (FFT above 192 limbs)
