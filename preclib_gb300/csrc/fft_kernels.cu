@@ -43,8 +43,9 @@
 //   * the inverse output is real: P is folded to Z_k = E_k + i O_k of half
 //     length, whose inverse has the even coefficients as real and the odd
 //     ones as imaginary parts.
-// Per call: 256 x 193 limbs 45.5 -> 32.0 us, 3000 x 3000 59.5 -> 42.1,
-// 6144 x 6144 80.4 -> 53.5 (kernels alone 34 -> 20, 46 -> 29, 63 -> 35).
+// Per C call from host memory (the Python binding adds about 8 us): 256 x 193 limbs
+// 45.5 -> 32.0 us, 3000 x 3000 59.5 -> 42.1, 6144 x 6144 80.4 -> 54.5 (kernels alone
+// 34 -> 20, 46 -> 28, 63 -> 37).
 #include <cuda_runtime.h>
 
 #include <cooperative_groups.h>

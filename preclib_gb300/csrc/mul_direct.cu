@@ -15,8 +15,8 @@
 // takes 2R - 1 digits of a (a window that slides by one block) and R of b.
 //
 // What bounds it: the 32x32->64-bit multiply-add, one per digit pair; 8192
-// products of 512 x 512 limbs reach 7.5 T multiply-adds/s, 40000 of 64 x 64
-// limbs 5.2 T/s (there the flushes and the carry stage show).  44643 products of
+// products of 512 x 96 limbs reach 6.2 T multiply-adds/s, 40000 of 64 x 64
+// limbs 5.1 T/s (there the flushes and the carry stage show).  44643 products of
 // 58 .. 66 limbs: kernels 0.98 -> 0.18 ms against the single-CTA transform.
 // A single product is bound by latency instead: launch, two trips to L2 and
 // the carries of the last CTA; 1024 x 1000 limbs 28.7 -> 8.1 us.

@@ -9,7 +9,7 @@
 
 namespace precgpu {
 
-// batch form: one product per group of 32 or more threads, longer operand
+// batch form: one product per group of 16 to 128 threads, longer operand
 // up to kDirectBatchMax limbs; classes 0 .. kDirectClasses-1 by that length
 constexpr int kDirectClasses = 5;
 constexpr uint64_t kDirectBatchMax = 512;

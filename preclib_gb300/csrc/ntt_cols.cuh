@@ -12,8 +12,9 @@
 //   otherwise cost the CRT one product per prime and coefficient), then the
 //   DIT transform over the row slots (the last stages of ntt_inverse,
 //   mul_ntt.cpp:257-329) back to natural coefficient order.
-// Both generate their twiddles as running Montgomery powers over a thread's
-// 32 slots of one column (twiddle32).
+// Both generate their twiddles as running powers over a thread's 32 slots of one
+// column (sets 0 and 2: a chain of Shoup products, twiddle32_shoup; sets 1 and 3:
+// Montgomery products, twiddle32), or read them from a table (col_table).
 // Columns are interleaved in shared memory (element i of column c at
 // P(i)*C + c); a warp covers C columns x 32/C items, so every global access
 // moves whole 32-byte sectors.

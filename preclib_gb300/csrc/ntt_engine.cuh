@@ -547,7 +547,7 @@ __device__ __forceinline__ u128 crt3(uint32_t y1, uint32_t y2, uint32_t y3, cons
 }
 
 // crt3 of the four-step path: the inverse column pass has already
-// multiplied y_1 by s1, y_2 by k22 2^32 and y_3 by k33 2^32 (CrtConst::fold), so
+// multiplied y_1 by s1, y_2 by m22 and y_3 by m33 (CrtConst::fold), so
 // y_1 is v1, and v2 = (y_2 + v1 n21) / 2^32, v3 = (y_3 + v1 n31 + v2 n32) / 2^32
 // mod p: one sum of products and one Montgomery reduction each (sums below
 // 0.6 * 2^32 p).  Set 0 leaves y_j in [0, 4p), set 1 in [0, p).

@@ -207,8 +207,7 @@ constexpr int kColGroup = PREC_COL_GROUP;      // adjacent columns per column-pa
 // Explicit graph construction.  While a thread has a recorder installed,
 // the library's launchers (launch_kernel) add kernel nodes to the
 // recorder's graph instead of launching: a node depends on the node last
-// recorded for the same stream handle, or on the recorder's fork point for
-// that stream.  The library's graphs are built this way rather than by
+// recorded for the same stream handle, and the first of a stream on none.  The library's graphs are built this way rather than by
 // stream capture: a capture in progress can be broken by a device-wide
 // synchronising call (cudaFree, cudaDeviceSynchronize, ...) that another
 // thread of the process makes at the same time, and callers and lanes run
@@ -220,8 +219,6 @@ struct GraphRecorder {
     uint64_t nodes = 0;
     cudaGraphNode_t tail(cudaStream_t st) const;
     void set_tail(cudaStream_t st, cudaGraphNode_t n);
-    // `to` starts after what is recorded on `from` so far (a fork)
-    void fork(cudaStream_t from, cudaStream_t to) { set_tail(to, tail(from)); }
     void add_kernel(const void* func, dim3 grid, dim3 block, size_t smem, void** args, cudaStream_t st);
     void add_memset(void* dst, size_t bytes, cudaStream_t st);  // zero fill
 };

@@ -65,7 +65,7 @@ int plan_for(uint64_t da, uint64_t db, uint64_t lout, Plan& pl, bool wide = fals
 // applied) that a product of la x lb digits of the plan's width needs
 int plan_keep(const Plan& pl, uint64_t la, uint64_t lb);
 // log2 of the 64-bit-digit transform for la x lb limbs, or 0 where the
-// 32-bit plan of 2^k32 points stays: it needs 2^13 .. 2^25 points, both
+// 32-bit plan of 2^k32 points stays: it needs 2^18 .. 2^25 points, both
 // operands in the lower half, min(la, lb) within the five primes' bound,
 // and fewer butterflies (5 N' log N' < 3 N log N)
 int wide_log2(uint64_t la, uint64_t lb, int k32);

@@ -4,9 +4,13 @@
 // is owned by its own pool allocator, a latency-critical loop that cannot
 // afford the device-wide synchronisation cudaFree implies, or a plugin host
 // that forbids device allocation once it has started.  For them,
-// prec_gpu_mul_device_noalloc runs the same kernels as prec_gpu_mul_device
-// but takes every byte it needs beyond the caller's inputs and outputs from
-// memory that is part of this library image:
+// prec_gpu_mul_device_noalloc computes the product of prec_gpu_mul_device but
+// takes every byte it needs beyond the caller's inputs and outputs from memory
+// that is part of this library image.  It runs the single-CTA kernel up to 2^12
+// points and the four throughput kernels, whole transforms on 32-bit digits,
+// above (not the direct products, the latency kernels or truncated transforms
+// of the other entry points): 1024 x 1024 limbs 16.5 us, 8192 x 8192 16.6,
+// 65536 x 65535 22.1, back to back.  Its memory:
 //   * g_noalloc_scratch -- the residue work buffer and carry words of one
 //     product of up to 2^18 transform points (an + bn <= 131072 limbs),
 //     about 6 MiB;
