@@ -701,21 +701,20 @@ static int grow(void** buf, size_t* cap, size_t bytes, bool slack) {
 // Work on `st` starts after the lane's previous product.  On the previous
 // product's own stream the stream's order says so already: no event wait.
 // Streams are told apart by their id, which, unlike the handle, no later
-// stream gets again; a stream being captured always gets the wait.
-static int lane_begin(Lane& L, cudaStream_t st) {
+// stream gets again.  A stream being captured has no id to ask for (the call
+// fails and ends the capture): it gets the wait, and so does what comes after it.
+static int lane_begin(Lane& L, cudaStream_t st, bool capturing = false) {
     unsigned long long id = 0;
-    CK(cudaStreamGetId(st, &id));
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    CK(cudaStreamIsCapturing(st, &cap));
-    if (!L.has_last || id != L.last_stream || cap != cudaStreamCaptureStatusNone)
-        CK(cudaStreamWaitEvent(st, L.last_done, 0));
+    if (!capturing) CK(cudaStreamGetId(st, &id));
+    if (capturing || !L.has_last || id != L.last_stream) CK(cudaStreamWaitEvent(st, L.last_done, 0));
     return 0;
 }
 
-static int lane_end(Lane& L, cudaStream_t st) {
-    CK(cudaStreamGetId(st, &L.last_stream));
+static int lane_end(Lane& L, cudaStream_t st, bool capturing = false) {
+    L.has_last = false;
+    if (!capturing) CK(cudaStreamGetId(st, &L.last_stream));
     CK(cudaEventRecord(L.last_done, st));
-    L.has_last = true;
+    L.has_last = !capturing;
     return 0;
 }
 
@@ -1217,25 +1216,27 @@ int prec_gpu_mul_device(const uint64_t* d_a, size_t an, const uint64_t* d_b, siz
     NvtxRange range("prec_gpu_mul_device %zux%zu", an, bn);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     Plan pl;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &status));
+    const bool capturing = status != cudaStreamCaptureStatusNone;
     const uint64_t B = block_limbs();
     if (an > B || bn > B) {
         if ((r = prepare_blocked(L, an, bn, B, pl))) return r;
-        if ((r = lane_begin(L, st))) return r;
+        if ((r = lane_begin(L, st, capturing))) return r;
         if ((r = enqueue_blocked(c, L, d_a, an, d_b, bn, d_out, st, B, c.d_err))) return r;
-        if ((r = lane_end(L, st))) return r;
+        if ((r = lane_end(L, st, capturing))) return r;
         return 0;
     }
-    // A product of up to 2^12 points that goes into a caller's graph runs as the
-    // one kernel that uses nothing of the lane: a replay is outside the lane's
+    // No direct product goes into a caller's graph: a replay is outside the lane's
     // order, and the direct kernel's column sums and counter are lane memory
-    // (allocated, too, which a capture refuses).
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    CK(cudaStreamIsCapturing(st, &cap));
-    if (cap != cudaStreamCaptureStatusNone && 2 * ((uint64_t)an + bn) - 1 <= 1ull << kSmallMaxLog2) {
+    // (allocated, too, which a capture refuses; a counter that two products shared
+    // would stay wrong).  Up to 2^12 points the one kernel that uses nothing of the
+    // lane takes it, above the four-step kernels.
+    if (capturing && 2 * ((uint64_t)an + bn) - 1 <= 1ull << kSmallMaxLog2) {
         if ((r = plan_for(2 * (uint64_t)an, 2 * (uint64_t)bn, an + bn, pl))) return r;
         return enqueue_ntt(c, L, d_a, an, d_b, bn, d_out, pl, st, c.d_err);
     }
-    if (direct_single(an, bn)) {
+    if (!capturing && direct_single(an, bn)) {
         if ((r = ensure_ws(L, direct_scratch_bytes(an, bn)))) return r;
         if ((r = lane_begin(L, st))) return r;
         launch_direct_single(d_a, an, d_b, bn, d_out, L.ws, L.direct_counter, c.d_err, st);
@@ -1245,9 +1246,9 @@ int prec_gpu_mul_device(const uint64_t* d_a, size_t an, const uint64_t* d_b, siz
     }
     if ((r = plan_for(2 * (uint64_t)an, 2 * (uint64_t)bn, an + bn, pl, wide_digits()))) return r;
     if ((r = ensure_ws(L, pl.work_bytes))) return r;
-    if ((r = lane_begin(L, st))) return r;
+    if ((r = lane_begin(L, st, capturing))) return r;
     if ((r = enqueue_ntt(c, L, d_a, an, d_b, bn, d_out, pl, st, c.d_err))) return r;
-    if ((r = lane_end(L, st))) return r;
+    if ((r = lane_end(L, st, capturing))) return r;
     return 0;
 }
 

@@ -2,6 +2,9 @@
 points uses no memory of the calling thread's lane, so it is accepted whatever
 the thread multiplied before, and its replays stay exact while the thread makes
 other products (which move the lane's workspace)."""
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -76,3 +79,34 @@ def test_noalloc_product_in_a_graph(gpu, an, bn):
             graph.replay()
         gpu.stream_check(s.cuda_stream)
         assert np.array_equal(out.cpu().numpy().view(np.uint64), _exact(a, b)), rep
+
+
+LONGER = """
+import numpy as np, torch
+from preclib_gb300 import native as N
+N.init(0)
+z = np.zeros(1, np.uint64)
+N.mul(z, z)  # the thread's lane, without a product on it
+rng = np.random.default_rng(1)
+a, b = (rng.integers(0, 1 << 64, n, dtype=np.uint64) for n in (1500, 1400))
+ta, tb = (torch.from_numpy(x.view(np.int64)).cuda() for x in (a, b))
+out = torch.zeros(2900, dtype=torch.int64, device="cuda")
+s, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+torch.cuda.synchronize()
+n0 = N.launch_count()
+with torch.cuda.graph(g, stream=s, capture_error_mode="relaxed"):
+    N.mul_device(ta.data_ptr(), 1500, tb.data_ptr(), 1400, out.data_ptr(), s.cuda_stream)
+print(N.launch_count() - n0)
+g.replay()
+torch.cuda.synchronize()
+x = int.from_bytes(a.tobytes(), "little") * int.from_bytes(b.tobytes(), "little")
+assert out.cpu().numpy().tobytes() == x.to_bytes(8 * 2900, "little")
+"""
+
+
+def test_longer_product_in_a_graph():
+    """Four-step kernels, not the direct one, whose counter is the lane's."""
+    pytest.importorskip("torch")
+    r = subprocess.run([sys.executable, "-c", LONGER], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert int(r.stdout) == 4
