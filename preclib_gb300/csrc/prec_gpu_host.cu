@@ -312,6 +312,7 @@ struct Ctx {
     int* d_err = nullptr;
     int* h_err = nullptr;
     double2* fft_tw = nullptr;  // FP64 band twiddles
+    cudaMemPool_t t4_pool = nullptr;  // the tables' own pool, made with the first
     uint2* t4[2][kMaxLog2 + 1] = {};  // four-step twiddle tables in use: sets 0 and 2, by log2 of the length
     FieldArgs field[kSets] = {};
     cudaMemPool_t pool = nullptr;
@@ -488,9 +489,18 @@ static int build_tables(Ctx& c) {
     return 0;
 }
 
+static cudaMemPoolProps device_pool_props(int device) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    return props;
+}
+
 // A length's table is made when a batch first has a class for it, and kept (0.4
 // to 42 MB, up to 1 ms; all lengths 90 MB): most processes batch few lengths or
-// none.  From the library's pool: an allocation there waits for no device work.
+// none.  From a pool of their own: an allocation there waits for no device work,
+// and no table stays in the middle of a block that the batches' pool hands out again.
 const uint2* ctx_fourstep_locked(int set, int k) {
     Ctx& c = g_ctx;
     const int w = set == kWideSet ? 1 : 0;
@@ -502,7 +512,11 @@ const uint2* ctx_fourstep_locked(int set, int k) {
     cudaStream_t st = nullptr;
     void* p = nullptr;
     cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-    if (!e) e = cudaMallocFromPoolAsync(&p, fourstep_entries(kSetPrimes[set], k) * sizeof(uint2), c.pool, st);
+    if (!e && !c.t4_pool) {
+        const cudaMemPoolProps props = device_pool_props(c.device);
+        e = cudaMemPoolCreate(&c.t4_pool, &props);
+    }
+    if (!e) e = cudaMallocFromPoolAsync(&p, fourstep_entries(kSetPrimes[set], k) * sizeof(uint2), c.t4_pool, st);
     if (!e) {
         launch_fourstep_table(static_cast<uint2*>(p), c.field[set], w ? c5.fold : cc.fold, kSetPrimes[set], k1, k - k1, st);
         e = cudaGetLastError();
@@ -529,10 +543,7 @@ static int init_locked(Ctx& c, int device) {
     CK(cudaSetDevice(device));
     c.device = device;
     {
-        cudaMemPoolProps props{};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = device;
+        const cudaMemPoolProps props = device_pool_props(device);
         CK(cudaMemPoolCreate(&c.pool, &props));
         uint64_t keep = ~0ull;
         CK(cudaMemPoolSetAttribute(c.pool, cudaMemPoolAttrReleaseThreshold, &keep));
@@ -1176,8 +1187,10 @@ void prec_gpu_shutdown(void) {
         }
     cudaFree(c.d_err);
     cudaFreeHost(c.h_err);
-    if (c.pool) cudaMemPoolDestroy(c.pool);
-    c.pool = nullptr;
+    for (cudaMemPool_t* p : {&c.t4_pool, &c.pool}) {
+        if (*p) cudaMemPoolDestroy(*p);
+        *p = nullptr;
+    }
     c.tables = nullptr;
     c.fft_tw = nullptr;
     c.d_err = c.h_err = nullptr;
