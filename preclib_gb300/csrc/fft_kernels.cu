@@ -480,6 +480,24 @@ static void launch_carry(const FftArgs& f, cudaStream_t st) {
 
 #define PREC_FFT_LOG2(X) X(3) X(4) X(5) X(6) X(7) X(8)
 
+// (limbs per thread, warps)
+#define PREC_FFT_CARRY(X) X(1, 16) X(1, 17) X(2, 16) X(2, 17) X(3, 16) X(3, 17)
+
+int configure_fft() {
+    cudaError_t e = load_kernel(k_fft_digits);
+#define X(M)                                        \
+    if (!e) e = load_kernel(k_fft_fwd_cols<M>);     \
+    if (!e) e = load_kernel(k_fft_rows<M>);         \
+    if (!e) e = load_kernel(k_fft_inv_cols<M>);
+    PREC_FFT_LOG2(X)
+#undef X
+#define X(L, W) \
+    if (!e) e = load_kernel(k_fft_carry<L, W>);
+    PREC_FFT_CARRY(X)
+#undef X
+    return (int)e;
+}
+
 int fft_launch(const FftArgs& f, cudaStream_t st) {
     const uint64_t nd = f.da > f.db ? f.da : f.db;
     launch_pdl(false, k_fft_digits, (unsigned)((nd + kDigitThreads - 1) / kDigitThreads), kDigitThreads, 0, st, f);
@@ -499,7 +517,7 @@ int fft_launch(const FftArgs& f, cudaStream_t st) {
     const int L = fft_carry_limbs(f.lout), NW = fft_carry_warps(f.lout);
 #define X(LL, W) \
     if (L == LL && NW == W) launch_carry<LL, W>(f, st);
-    X(1, 16) X(1, 17) X(2, 16) X(2, 17) X(3, 16) X(3, 17)
+    PREC_FFT_CARRY(X)
 #undef X
     count_launches(5);
     return (int)cudaGetLastError();

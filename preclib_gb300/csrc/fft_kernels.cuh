@@ -90,5 +90,6 @@ size_t fft_table_bytes();
 void fft_build_table(double2* tw, cudaStream_t st);
 // The product's 5 kernels on `st`.  Returns a cudaError_t.
 int fft_launch(const FftArgs& f, cudaStream_t st);
+int configure_fft();
 
 }  // namespace precgpu

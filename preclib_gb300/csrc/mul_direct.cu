@@ -467,7 +467,7 @@ void launch_direct_single(const uint64_t* a, uint64_t la, const uint64_t* b, uin
 }
 
 int configure_direct() {
-    cudaError_t e = cudaSuccess;
+    cudaError_t e = load_kernel(k_direct_lists);
 #define X(C, R, G) \
     if (!e) e = cudaFuncSetAttribute(k_direct<R, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DirectGeom<R, G>::SMEM);
     PREC_DIRECT(X)

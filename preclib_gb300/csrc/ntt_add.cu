@@ -108,4 +108,6 @@ void launch_add_into(uint64_t* out, uint64_t n, const uint64_t* t, uint64_t nt, 
     count_launches(1);
 }
 
+int configure_add() { return (int)load_kernel(k_add_into); }
+
 }  // namespace precgpu

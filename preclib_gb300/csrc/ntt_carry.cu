@@ -23,6 +23,14 @@ void launch_crt_carry(int set, const ProdArgs& a, cudaStream_t st, const ProdPtr
     count_launches(1);
 }
 
+int configure_carry() {
+    cudaError_t e = load_kernel(k_crt_carry<0>);
+    if (!e) e = load_kernel(k_crt_carry<1>);
+    if (!e) e = load_kernel(k_crt_carry<kWideSet>);
+    if (!e) e = load_kernel(k_crt_carry<kWideSetL>);
+    return (int)e;
+}
+
 void ntt_launch_4step_batch(int set, const ProdArgs& args, const ProdPtrs* batch, int count, int max_nblk,
                             cudaStream_t st) {
     launch_fwd_cols(set, args, st, batch, count);
@@ -111,6 +119,7 @@ int ntt_configure_kernels() {
     if (!e) e = configure_rows();
     if (!e) e = configure_small();
     if (!e) e = configure_class();
+    if (!e) e = configure_carry();
     return e;
 }
 

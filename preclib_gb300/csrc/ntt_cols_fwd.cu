@@ -76,7 +76,8 @@ bool cols_trunc_supported(int set, int k1, int k2, int cg, int mr, int keep) {
 }
 
 int configure_fwd_cols() {
-    cudaError_t e = (cudaError_t)configure_fwd_cols_k2();
+    cudaError_t e = load_kernel(k_fourstep_table);
+    if (!e) e = (cudaError_t)configure_fwd_cols_k2();
     if (!e) e = (cudaError_t)configure_fwd_cols_trunc5();
     if (!e) e = (cudaError_t)configure_fwd_cols_trunc6();
     if (!e) e = (cudaError_t)configure_fwd_cols_trunc7();

@@ -270,6 +270,18 @@ inline void launch_pdl(bool chain, void (*k)(P...), dim3 grid, dim3 block, size_
     cudaLaunchKernelEx(&cfg, k, static_cast<P>(std::forward<A>(args))...);
 }
 
+// Loads a kernel's code.  A kernel not loaded at start-up (here, or by setting its
+// shared-memory size) is loaded by its first launch, which then waits for what
+// the device is doing: beside a stream kept busy for 0.75 s the first FP64 product
+// took 0.75 s, and binary splitting of pi to 10^8 digits, beside the square root on
+// another thread, took 0.17 s instead of 0.095 in every other run.  (All of them: 0.5
+// ms of 27 at start-up.)
+template <class... P>
+inline cudaError_t load_kernel(void (*k)(P...)) {
+    cudaFuncAttributes attr;
+    return cudaFuncGetAttributes(&attr, reinterpret_cast<const void*>(k));
+}
+
 // Kernel launches issued by the library (process-wide, prec_gpu_launch_count);
 // every launcher adds its launches.  launches_this_thread() lets a graph
 // recording take back the launches it only recorded.
@@ -376,6 +388,9 @@ inline void col_config(int set, int m, int req_cg, int req_mr, int& cg, int& mr)
 int configure_rows();
 int configure_small();
 int configure_class();
+int configure_lat();
+int configure_carry();
+int configure_add();
 
 // The batch form's persistent kernel per length class (ntt_class.cu): its
 // scheduling words, zeroed before each launch, are kClassHdrWords (the next

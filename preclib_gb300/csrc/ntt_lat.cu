@@ -418,4 +418,21 @@ void ntt_launch_lat(int set, const ProdArgs& a, cudaStream_t st, cudaEvent_t* ev
     if (ev) cudaEventRecord(ev[4], st);
 }
 
+int configure_lat() {
+    cudaError_t e = cudaSuccess;
+#define X(S, A, B, E)                                      \
+    if (!e) e = load_kernel(k_fwd_cols_lat<S, A, B, E>);   \
+    if (!e && S == 0) e = load_kernel(k_inv_cols_lat<0, A, B, E>);
+    PREC_LAT(X)
+#undef X
+#define X(M)                                        \
+    if (!e) e = load_kernel(k_rows_lat<0, M, true>); \
+    if (!e) e = load_kernel(k_rows_lat<0, M, false>);
+    X(7) X(8) X(9)
+#undef X
+    if (!e) e = load_kernel(k_crt_cluster<1>);
+    if (!e) e = load_kernel(k_crt_cluster<2>);
+    return (int)e;
+}
+
 }  // namespace precgpu

@@ -557,6 +557,9 @@ static int init_locked(Ctx& c, int device) {
     CK(cudaMallocHost(&c.h_err, kStatBytes));
     CK((cudaError_t)ntt_configure_kernels());
     CK((cudaError_t)configure_direct());
+    CK((cudaError_t)configure_lat());
+    CK((cudaError_t)configure_fft());
+    CK((cudaError_t)configure_add());
     CK(cudaMalloc(&c.fft_tw, fft_table_bytes()));
     fft_build_table(c.fft_tw, nullptr);
     CK(cudaGetLastError());
